@@ -26,6 +26,7 @@ extern "C" {
 
 #define QG_MAX_GROUPS 8   /* coefficient groups (QobjEvo terms after merging) per operator */
 #define QG_MAX_EOPS 32    /* operators per expect launch */
+#define QG_EXPECT_TIMES 32 /* output times per qg_expect_dm_times launch */
 #define QG_MAX_COPS 64    /* collapse operators of one matrix-free Lindblad generator */
 
 typedef enum { QG_C128 = 0, QG_C64 = 1 } qg_dtype;
@@ -382,6 +383,17 @@ int qg_expect_dm(const qg_csr_groups* ops, int64_t d, const qg_state_view* rho, 
 /* out[2g..] = <psi|op_g|psi>, out[2G..] = <psi|psi>.  Replaces
  * _expect_csr_dense_ket (qutip/core/data/expect.pyx:133-144). */
 int qg_expect_ket(const qg_csr_groups* ops, const qg_state_view* psi, double* out, void* stream);
+
+/* qg_expect_dm at n_times output times inside one Vern7 step: rho(t) = base +
+ * sum_{j<16} f_j(tau) k_j with the 7th-order dense-output factors of
+ * Explicit_RungeKutta._interpolate_step (qutip/solver/integrator/explicit_rk.pyx:412-430),
+ * tau = (t - t_prev) / dt, formed on the device (rho->f and rho->n_k are not used; rho->k
+ * must hold all 16 stages).  out[(i (G+1) + g) 2 ..] is operator g at time i, operator G
+ * the trace.  tau is host memory; ops must be group-major; scratch and counter as in
+ * qg_rk_buffers (the counter is left zero). */
+int qg_expect_dm_times(const qg_csr_groups* ops, int64_t d, const qg_state_view* rho, int n_times,
+                       const double* tau, double dt, double* out, double* scratch,
+                       unsigned int* counter, void* stream);
 
 /* ---- batched, persistent solves ----------------------------------------- */
 /* One system of a batch.  Its generator is a row-major grouped CSR in the

@@ -15,6 +15,7 @@ LIB_PATH = Path(__file__).resolve().parent / "libqutip_gb300.so"
 QG_OK, QG_ERR_ARG, QG_ERR_CUDA, QG_ERR_UNSUPPORTED = 0, -1, -2, -3
 QG_C128, QG_C64 = 0, 1
 QG_MAX_GROUPS, QG_MAX_EOPS, QG_MAX_COPS = 8, 32, 64
+QG_EXPECT_TIMES = 32
 
 
 QG_LAYOUT_GROUP_MAJOR, QG_LAYOUT_ROW_MAJOR, QG_LAYOUT_SLICED, QG_LAYOUT_SLICED_DICT = 0, 1, 2, 3
@@ -118,6 +119,9 @@ _SIGS = {
     "qg_norm2": (C.c_int, [C.c_void_p, C.c_int, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p,
                            C.c_void_p]),
     "qg_expect_dm": (C.c_int, [_P(CsrGroups), C.c_int64, _P(StateView), C.c_void_p, C.c_void_p]),
+    "qg_expect_dm_times": (C.c_int, [_P(CsrGroups), C.c_int64, _P(StateView), C.c_int, C.c_void_p,
+                                     C.c_double, C.c_void_p, C.c_void_p, C.c_void_p,
+                                     C.c_void_p]),
     "qg_expect_ket": (C.c_int, [_P(CsrGroups), _P(StateView), C.c_void_p, C.c_void_p]),
     "qg_abi_sizes": (C.c_int, [C.c_void_p, C.c_int]),
     "qg_batch_slot_bytes": (C.c_int64, [C.c_int64, C.c_int]),
@@ -135,8 +139,9 @@ _lib = None
 # Entry points that launch exactly one kernel each; calls are counted so that a
 # benchmark can report how many of this library's kernels ran in a timed region.
 COMPUTE_ENTRY_POINTS = {
-    "qg_spmv_csr", "qg_spmm_csr", "qg_spmv_dia", "qg_vern7_stage", "qg_rk_combine", "qg_norm2",
-    "qg_expect_dm", "qg_expect_ket", "qg_batch_vern7", "qg_batch_vern7_noalloc",
+    "qg_spmv_csr", "qg_spmm_csr", "qg_spmv_dia", "qg_vern7_stage", "qg_vern7_range", "qg_rk_combine",
+    "qg_norm2",
+    "qg_expect_dm", "qg_expect_ket", "qg_expect_dm_times", "qg_batch_vern7", "qg_batch_vern7_noalloc",
     "qg_lindblad_apply", "qg_lindblad_stage", "qg_dense_lindblad_apply", "qg_dense_lindblad_stage",
     "qg_sde_platen", "qg_sde_euler",
 }

@@ -23,7 +23,7 @@ from .coefficients import Coefficient, coefficient
 from .lindblad import LindbladOperator
 from .operator import DeviceOperator, stream_ptr
 from .systems import OpenSystem, lindblad_dissipator, merge_terms, spost, spre
-from .vern7 import GpuVern7, PRECISIONS
+from .vern7 import GpuVern7, INTERPOLATED, PRECISIONS
 
 __all__ = ["MEResult", "mesolve", "solve_system", "liouvillian_terms", "ExpectOps"]
 
@@ -56,6 +56,18 @@ class ExpectOps:
     def expect_dm(self, d: int, view: _lib.StateView, out: torch.Tensor):
         _lib.call("qg_expect_dm", C.byref(self.dev.struct), d, C.byref(view), out.data_ptr(),
                   stream_ptr())
+
+    def expect_dm_step(self, d: int, ig: GpuVern7, times, out: torch.Tensor):
+        """Expectation values at output ``times`` that all lie inside ``ig``'s current step
+        (its dense output prepared), one row of ``out`` per time: one launch per
+        ``QG_EXPECT_TIMES`` times."""
+        tau = (np.asarray(times, dtype=np.float64) - ig.t_prev) / ig.dt_int
+        view = ig.step_view()
+        for i in range(0, len(tau), _lib.QG_EXPECT_TIMES):
+            t = np.ascontiguousarray(tau[i:i + _lib.QG_EXPECT_TIMES])
+            _lib.call("qg_expect_dm_times", C.byref(self.dev.struct), d, C.byref(view), len(t),
+                      t.ctypes.data, ig.dt_int, out[i].data_ptr(), ig.scratch.data_ptr(),
+                      ig.counter.data_ptr(), stream_ptr())
 
     def expect_ket(self, view: _lib.StateView, out: torch.Tensor):
         _lib.call("qg_expect_ket", C.byref(self.dev.struct), C.byref(view), out.data_ptr(),
@@ -126,10 +138,22 @@ def _evolve(ig: GpuVern7, tlist, ex: ExpectOps, d: int, store_states, store_fina
             states.append(ig.get_state().clone())
 
     record(0)
-    for i in range(1, nt):
+    i = 1
+    while i < nt:
         ig.integrate(float(tlist[i]))
         ig.check()
+        if kind == "me" and G and not store_states and ig.status == INTERPOLATED:
+            # every following output time inside this step is read from its dense output
+            j = i + 1
+            while j < nt and ig.t_prev <= tlist[j] < ig.t_front:
+                j += 1
+            ex.expect_dm_step(d, ig, tlist[i:j], raw[i:j])
+            if j > i + 1:
+                ig.integrate(float(tlist[j - 1]))
+            i = j
+            continue
         record(i)
+        i += 1
     final = ig.get_state().clone() if store_final else None
     r = raw.cpu().numpy()
     vals = r[:, 0:2 * G:2] + 1j * r[:, 1:2 * G:2]

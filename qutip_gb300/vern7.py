@@ -345,6 +345,10 @@ class GpuVern7:
             return self._view(self.y_front)
         return self._view(self.y_prev, self._out[1])
 
+    def step_view(self) -> _lib.StateView:
+        """The current step's dense output: ``y_prev`` and the 16 stages, no factors."""
+        return self._view(self.y_prev)
+
     def get_state(self) -> torch.Tensor:
         """Materialise the state at ``self.t`` into ``self.y_out`` (state dtype)."""
         if self._out[0] == "front":
