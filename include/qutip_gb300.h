@@ -290,6 +290,20 @@ int qg_spmv_dia(const qg_dia* A, const void* x, void* y, double alpha_re, double
 int qg_vern7_stage(const qg_csr_groups* A, const qg_rk_buffers* B, int stage, double t_prev,
                    double dt, double atol, double rtol, void* stream);
 
+/* The stages of a whole trial step (stage0 = 0, stage1 = 10: qg_vern7_stage 0..9) or the
+ * dense-output stages (10, 16: the input of stage 10 formed from k_0..k_9, then
+ * qg_vern7_stage 10..15; _prep_dense_out, explicit_rk.pyx:399-410) in one cooperative
+ * launch, for an operator whose rows all fit the GPU at once.  Returns 1 without a launch
+ * when they do not, or when the layout has no such kernel (group-major, sub-warps of 1, 16
+ * or 32, a complex128 dictionary that is not split): the caller then launches the stages
+ * one by one.  barrier: one word of device memory, zero before the first launch and owned
+ * by the caller's stream order; barrier_base: host word, zero at first, advanced by each
+ * call.  A bounded wait that gave up leaves *B->result = -1 and sets qg_device_fault(); zero both
+ * words before the next call. */
+int qg_vern7_range(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0, int stage1,
+                   double t_prev, double dt, double atol, double rtol, unsigned int* barrier,
+                   uint32_t* barrier_base, void* stream);
+
 /* y = alpha * L(t)[x] + beta * y for the matrix-free Lindblad generator; x and y
  * are vec(rho) of length d*d in L's dtype.  Replaces LindbladMatrixForm.matmul_data
  * (qutip/core/cy/lindblad_matrix_form.pyx:105-204). */

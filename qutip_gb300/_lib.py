@@ -100,6 +100,9 @@ _SIGS = {
                               C.c_double, C.c_double, C.c_void_p]),
     "qg_vern7_stage": (C.c_int, [_P(CsrGroups), _P(RkBuffers), C.c_int, C.c_double, C.c_double,
                                  C.c_double, C.c_double, C.c_void_p]),
+    "qg_vern7_range": (C.c_int, [_P(CsrGroups), _P(RkBuffers), C.c_int, C.c_int, C.c_double,
+                                 C.c_double, C.c_double, C.c_double, C.c_void_p,
+                                 _P(C.c_uint32), C.c_void_p]),
     "qg_lindblad_apply": (C.c_int, [_P(Lindblad), C.c_double, C.c_void_p, C.c_void_p,
                                     C.c_double, C.c_double, C.c_double, C.c_double,
                                     C.c_void_p]),

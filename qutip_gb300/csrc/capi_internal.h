@@ -11,7 +11,11 @@ int set_error(int code, const char* msg);
 int check_launch(const char* what);
 // Multiprocessor count of the current device (cached per device).
 int sm_count();
+// Validate a grouped operator (shape, layout and tables); QG_OK or an error code.
+int check_groups(const qg_csr_groups* A);
 }  // namespace qg
 
 // The dense kernel's fault flag, read and cleared (for qg_device_fault).
 int dense_fault_take();
+// The same for the fused step kernel's barrier waits.
+int step_fault_take();

@@ -24,6 +24,7 @@
 
 #include "capi_internal.h"
 #include "common.cuh"
+#include "rows.cuh"
 #include "stage.cuh"
 
 namespace qg {
@@ -33,30 +34,6 @@ constexpr int SPMV_BLOCK = 256;
 constexpr int SLICED_MIN_BLOCKS = 6;
 
 __device__ unsigned int g_fault = 0u;
-
-// Complex multiply-accumulate in the accumulation precision.
-__device__ __forceinline__ void cmac_any(double& ar, double& ai, double2 v, double2 x) {
-  ar = fma(v.x, x.x, ar);
-  ar = fma(-v.y, x.y, ar);
-  ai = fma(v.x, x.y, ai);
-  ai = fma(v.y, x.x, ai);
-}
-__device__ __forceinline__ void cmac_any(float& ar, float& ai, float2 v, float2 x) {
-  ar = fmaf(v.x, x.x, ar);
-  ar = fmaf(-v.y, x.y, ar);
-  ai = fmaf(v.x, x.y, ai);
-  ai = fmaf(v.y, x.x, ai);
-}
-
-template <int LANES, typename R>
-__device__ __forceinline__ cx<R> sub_reduce(R ar, R ai) {
-#pragma unroll
-  for (int o = LANES / 2; o > 0; o >>= 1) {
-    ar += __shfl_xor_sync(0xffffffffu, ar, o);
-    ai += __shfl_xor_sync(0xffffffffu, ai, o);
-  }
-  return cx<R>{ar, ai};
-}
 
 // Partial row dot product over entries [s, e) for one lane of a LANES-wide
 // sub-warp.  GLOBAL: val/col are global arrays; otherwise shared-memory
@@ -99,14 +76,9 @@ __device__ __forceinline__ void load_coefs(const qg_csr_groups& A, double t, cx<
   }
 }
 
-// Class of each group's coefficient, decided once per block: 0 = exactly one (the
-// group's sum goes straight into the row's), 1 = real, 2 = complex.
 template <typename CT>
 __device__ __forceinline__ void coef_classes(const qg_csr_groups& A, const cx<CT>* coef, int* cls) {
-  if (threadIdx.x < A.n_groups) {
-    const cx<CT> c = coef[threadIdx.x];
-    cls[threadIdx.x] = (c.re == (CT)1 && c.im == (CT)0) ? 0 : (c.im == (CT)0 ? 1 : 2);
-  }
+  if (threadIdx.x < A.n_groups) cls[threadIdx.x] = coef_class(coef[threadIdx.x]);
 }
 
 // ------------------------------------------------------------ direct kernel --
@@ -356,61 +328,6 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, UNR>::MIN_BLOCKS)
 // in the driven group, about 700 in the constant one), so the operator stream shrinks
 // from 12 bytes per entry (complex64 value, int32 column) to 1-2 bytes, and a stage is
 // bound by the shared-memory lookups and the L2 gathers of x instead of by HBM.
-template <int CB>
-struct Codes4;
-template <>
-struct Codes4<1> {
-  using T = unsigned int;
-  __device__ static int at(T c, int u) { return (int)((c >> (8 * u)) & 0xffu); }
-};
-template <>
-struct Codes4<2> {
-  using T = uint2;
-  __device__ static int at(T c, int u) {
-    const unsigned w = u < 2 ? c.x : c.y;
-    return (int)((w >> (16 * (u & 1))) & 0xffffu);
-  }
-};
-
-// One stored code: the table pair k applied to x[row + offset].  Whole complex values
-// (QG_LAYOUT_SLICED_DICT) cost four multiply-adds.  With the real/imaginary split
-// (QG_LAYOUT_SLICED_DICT_RI, complex128) a table entry is one real factor: toff holds
-// (offset << 1) | imag and tval the pair (c1, c2) = (a, a) for a real part or (-a, a) for
-// an imaginary part, applied as (c1 p, c2 q) with (p, q) = x, or x's parts exchanged for
-// an imaginary part -- two FP64 multiply-adds, GB300's scarce FP64 rate being the bound.
-template <bool RI, typename ST, typename R>
-__device__ __forceinline__ void dict_mac(const ST* __restrict__ tval, const int* __restrict__ toff,
-                                         const ST* __restrict__ x, int k, int row, int last_col,
-                                         R& ar, R& ai) {
-  if constexpr (RI) {
-    const int oc = toff[k];
-    const int col = min(max(row + (oc >> 1), 0), last_col);
-    const ST v = tval[k];
-    const ST xv = ld_gather(x + col);
-    const bool sw = (oc & 1) != 0;
-    ar = fma(v.x, sw ? xv.y : xv.x, ar);
-    ai = fma(v.y, sw ? xv.x : xv.y, ai);
-  } else {
-    const int col = min(max(row + toff[k], 0), last_col);
-    cmac_any(ar, ai, tval[k], ld_gather(x + col));
-  }
-}
-
-// acc += c * (ar, ai).  In FP64 a real coefficient (every group of a Liouvillian with a
-// real time dependence, and the constant group) takes two multiply-adds, not four; the
-// branch is uniform (one coefficient per group).  FP32 keeps the plain product.
-template <typename R>
-__device__ __forceinline__ void coef_mac(cx<R>& acc, cx<R> c, R ar, R ai) {
-  if constexpr (sizeof(R) == 8) {
-    if (c.im == (R)0) {
-      acc.re = fma(c.re, ar, acc.re);
-      acc.im = fma(c.re, ai, acc.im);
-      return;
-    }
-  }
-  acc = cx_add(acc, cx_mul(c, cx<R>{ar, ai}));
-}
-
 template <int DT, int YDT, int EPI, int CB, bool RI>
 __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, 4>::MIN_BLOCKS)
     spmv_dict_kernel(qg_csr_groups A, double t, const typename elem<DT>::T* __restrict__ x,
@@ -467,7 +384,7 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, 4>::MIN_BLOCKS)
             if (!__any_sync(0xffffffffu, k != 0)) continue;
           }
           k = t0 + (k < tn ? k : 0);  // a table index of this group whatever the code
-          dict_mac<RI>(tval, toff, x, k, row, last_col, ar, ai);
+          dict_mac<RI, true>(tval, toff, x, k, row, last_col, ar, ai);
         }
       }
       if (wr) {
@@ -480,7 +397,7 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, 4>::MIN_BLOCKS)
               if (!__any_sync(0xffffffffu, k != 0)) continue;
             }
             k = t0 + (k < tn ? k : 0);
-            dict_mac<RI>(tval, toff, x, k, row, last_col, ar, ai);
+            dict_mac<RI, true>(tval, toff, x, k, row, last_col, ar, ai);
           }
         }
       }
@@ -878,7 +795,7 @@ static int launch_lindblad(cudaStream_t st, const qg_lindblad& L, double t, cons
                      : launch_lindblad_form<DT, YDT, EPI, false>(st, L, t, x, ax, rk);
 }
 
-static int check_groups(const qg_csr_groups* A) {
+int check_groups(const qg_csr_groups* A) {
   if (!A || !A->row_ptr || !A->col || !A->val) return set_error(QG_ERR_ARG, "null operator");
   if (A->n_groups < 1 || A->n_groups > QG_MAX_GROUPS)
     return set_error(QG_ERR_ARG, "n_groups out of range");
@@ -965,7 +882,7 @@ extern "C" int qg_device_fault(void) {
   if (cudaMemcpyFromSymbol(&v, g_fault, sizeof(v)) != cudaSuccess)
     return set_error(QG_ERR_CUDA, "cannot read the device fault flag");
   if (v) cudaMemcpyToSymbol(g_fault, &zero, sizeof(zero));
-  return (int)(v | (unsigned)dense_fault_take());
+  return (int)(v | (unsigned)dense_fault_take() | (unsigned)step_fault_take());
 }
 
 extern "C" int qg_spmv_csr(const qg_csr_groups* A, double t, const void* x, void* y,

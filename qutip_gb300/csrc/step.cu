@@ -1,0 +1,507 @@
+// Several Vern7 stages of one system in one launch (qg_vern7_range): a trial step (stages
+// 0..9 with the error norm) or the dense-output stages (10..15) of a system whose rows all
+// fit the GPU at once, one row per sub-warp of LANES threads.
+//
+// What bounds it: latency.  A stage of a system of up to some 70,000 rows is a few
+// microseconds of dependent loads and FP64 work, so ten launches a step, each with its own
+// host call, launch gap and re-read of the row's data, cost more than the arithmetic:
+// 21.6 us per right-hand side at 65,536 rows, whose FP64 work takes 6.4 us.  Here the
+// stages follow one another behind a grid barrier; a row keeps its operator entries (or
+// codes), its k_j and its state in shared memory and registers for the whole launch, and
+// only the stage input crosses between SMs.  Measured, whole complex128 solves: the L = 8
+// Ising chain (65,536 rows) 39.1 -> 27.9 ms (12 us a stage), the d = 125 Bose-Hubbard trimer
+// (15,625 rows, odd) 9.8 -> 6.2 ms.  An operator with more rows than the GPU has resident
+// threads at 512 a block keeps one launch a stage: there a stage is 40 us and more, and the
+// launches no longer count.
+//
+// The launch is cooperative (all blocks resident), and every wait at the barrier is bounded:
+// a wait that gives up sets *result to -1 and every block leaves.  A row's sum and its
+// stage combination are formed by the operations of the per-stage kernels in their order.
+#include <mutex>
+
+#include "capi_internal.h"
+#include "common.cuh"
+#include "rows.cuh"
+#include "stage.cuh"
+
+namespace qg {
+
+// Layouts: row-major CSR with LANES threads per row, 32-row slices, dictionary codes.
+enum Kind { KIND_CSR = 0, KIND_SLICED = 1, KIND_DICT1 = 2, KIND_DICT2 = 3 };
+
+constexpr int STEP_THREADS = 512;   // most threads of a block (one block per SM)
+constexpr int STEP_MIN_WARPS = 4;   // fewer warps per block only spread the barrier wider
+// entries (CSR, sliced) or code words a thread keeps in shared memory; rows longer than
+// that read the rest from global memory at every stage
+constexpr int STEP_KEEP = 8;
+constexpr long long STEP_WAIT_CYCLES = 16 * WAIT_CYCLES;  // the GPU may be shared meanwhile
+
+struct StepArgs {
+  qg_csr_groups A;
+  RkArgs rk;           // buffers and tolerances (factors are formed on the device)
+  const void* x0;      // input of stage 0
+  void* ytmp;          // both stage-input buffers
+  double t_prev, dt;
+  int s0, s1;          // stages [s0, s1)
+  int keep;            // entries or code words kept per thread
+  unsigned int* bar;   // arrivals of every earlier launch and of this one
+  unsigned int bar_base;
+};
+
+__device__ unsigned int g_step_fault = 0u;
+
+// Shared memory of a block, in bytes from its start (every part 16-byte aligned).
+struct StepSmem {
+  int tval, toff, k, val, idx, rp, total;
+};
+template <typename ST>
+__host__ __device__ inline StepSmem step_smem(const qg_csr_groups& A, int kind, int threads,
+                                              int rows, int keep) {
+  const int D = kind >= KIND_DICT1 ? A.lanes : 0;
+  auto up = [](size_t b) { return (int)((b + 15) & ~(size_t)15); };
+  StepSmem L;
+  L.tval = 0;
+  L.toff = up((size_t)D * sizeof(ST));
+  L.k = L.toff + up((size_t)D * 4);
+  L.val = L.k + up((size_t)rows * RK_EXTRA_STEP * sizeof(ST));
+  const int vb = kind >= KIND_DICT1 ? 0 : (int)sizeof(ST);
+  const int ib = kind == KIND_DICT2 ? 8 : 4;
+  L.idx = L.val + up((size_t)threads * keep * vb);
+  L.rp = L.idx + up((size_t)threads * keep * ib);
+  L.total = L.rp + up((size_t)rows * (kind == KIND_CSR ? A.n_groups + 1 : 2 * A.n_groups) * 4);
+  return L;
+}
+
+// Grid barrier: block arrivals counted in one word that only grows; this launch's n-th
+// barrier completes at base + n * blocks.  False when the bounded wait gave up.
+__device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int target,
+                                             bool* ok_s) {
+  if (gridDim.x == 1) {
+    __syncthreads();
+    return true;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(bar, 1u);
+    const long long t0 = clock64();
+    unsigned int v;
+    bool ok;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      ok = (int)(v - target) >= 0;
+    } while (!ok && clock64() - t0 < STEP_WAIT_CYCLES);
+    __threadfence();
+    *ok_s = ok;
+  }
+  __syncthreads();
+  return *ok_s;
+}
+
+template <int DT, int YDT, int KIND, int LANES>
+__global__ void __launch_bounds__(STEP_THREADS, 1)
+    vern7_range_kernel(const __grid_constant__ StepArgs a) {
+  using ST = typename elem<DT>::T;
+  using YT = typename elem<YDT>::T;
+  using R = typename elem<DT>::R;
+  constexpr bool MIXED = DT != YDT;
+  constexpr bool RI = DT == QG_C128;
+  constexpr bool DICT = KIND >= KIND_DICT1;
+  constexpr int CB = KIND == KIND_DICT2 ? 2 : 1;
+  using C4 = typename Codes4<CB>::T;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ cx<R> coef[RK_EXTRA_STEP][QG_MAX_GROUPS];
+  __shared__ int ccls[RK_EXTRA_STEP][QG_MAX_GROUPS];
+  __shared__ R fac[RK_EXTRA_STEP][RK_EXTRA_STEP];  // dt a of the combination after stage s
+  __shared__ R fe_s[RK_STEP];
+  __shared__ float fel_s[RK_STEP];
+  __shared__ unsigned int nz_s[RK_EXTRA_STEP + 1];
+  __shared__ int tstart[QG_MAX_GROUPS + 1];
+  __shared__ double red[STEP_THREADS / 32];
+  __shared__ bool ok_s, last_s;
+  const qg_csr_groups& A = a.A;
+  const RkArgs& rk = a.rk;
+  const int G = A.n_groups, n = (int)A.n_rows;
+  const int tid = threadIdx.x, threads = blockDim.x;
+  const int rows = threads / LANES;
+  const int lrow = tid / LANES, lane = tid % LANES;
+  const int row = blockIdx.x * rows + lrow;
+  const bool valid = row < n;
+  const StepSmem L = step_smem<ST>(A, KIND, threads, rows, a.keep);
+  ST* tval = reinterpret_cast<ST*>(smem + L.tval);
+  int* toff = reinterpret_cast<int*>(smem + L.toff);
+  ST* ksm = reinterpret_cast<ST*>(smem + L.k) + lrow;  // k_j of this row at ksm[j * rows]
+  ST* vsm = reinterpret_cast<ST*>(smem + L.val) + tid;  // kept entry i at [i * threads]
+  int* csm = reinterpret_cast<int*>(smem + L.idx) + tid;
+  C4* wsm = reinterpret_cast<C4*>(smem + L.idx) + tid;
+  int* rpsm = reinterpret_cast<int*>(smem + L.rp) + lrow;  // row bounds, [g * rows]
+
+  // ---- once per launch: factors, coefficients, the row's operator data ----
+  for (int e = tid; e < (a.s1 - a.s0) * G; e += threads) {
+    const int s = a.s0 + e / G, g = e % G;
+    const cplx c = group_coef(A, g, a.t_prev + VERN7_C[s] * a.dt);
+    coef[s][g] = cx<R>{(R)c.re, (R)c.im};
+    ccls[s][g] = coef_class(coef[s][g]);
+  }
+  for (int e = tid; e < RK_EXTRA_STEP * RK_EXTRA_STEP; e += threads) {
+    const int s = e / RK_EXTRA_STEP, j = e % RK_EXTRA_STEP;
+    double v = 0.0;
+    if (s == RK_STEP - 1 && a.s0 == 0) v = j < RK_STEP ? a.dt * VERN7_B[j] : 0.0;
+    else if (s + 1 < RK_EXTRA_STEP && j <= s) v = a.dt * VERN7_A[s + 1][j];
+    fac[s][j] = (R)v;
+    const double w = s == 0 && j < RK_STEP ? a.dt * VERN7_E[j] : 0.0;
+    if (s == 0 && j < RK_STEP) {
+      fe_s[j] = (R)w;
+      fel_s[j] = (float)(w - (double)(float)w);
+    }
+    // the masks are of the double factors, as the per-stage kernels take them
+    const unsigned int nz = __ballot_sync(0xffffffffu, v != 0.0);
+    const unsigned int ne = __ballot_sync(0xffffffffu, w != 0.0);
+    if ((tid & 31) == 0) {  // a warp covers two rows of the table
+      nz_s[s] = nz & 0xffffu;
+      nz_s[s + 1 < RK_EXTRA_STEP ? s + 1 : s] = nz >> 16;
+      if (s == 0) nz_s[RK_EXTRA_STEP] = ne & 0xffffu;
+    }
+  }
+  if constexpr (DICT) {
+    for (int i = tid; i < A.lanes; i += threads) {
+      tval[i] = __ldg(static_cast<const ST*>(A.val) + i);
+      toff[i] = __ldg(A.dict_off + i);
+    }
+    if (tid <= G) tstart[tid] = __ldg(A.dict_start + tid);
+  }
+  const int sl = row >> 5;  // slice (sliced layouts: LANES == 1, a warp is a slice)
+  const int S = A.n_tiles;
+  const ST* __restrict__ gval = static_cast<const ST*>(A.val);
+  const int* __restrict__ gcol = A.col;
+  const unsigned char* __restrict__ codes = reinterpret_cast<const unsigned char*>(A.col);
+  if constexpr (KIND == KIND_CSR) {
+    int i = 0;
+    int s = valid ? __ldg(A.row_ptr + row * G) : 0;
+    if (lane == 0) rpsm[0] = s;
+    for (int g = 0; g < G; ++g) {
+      const int e = valid ? __ldg(A.row_ptr + row * G + g + 1) : 0;
+      if (lane == 0) rpsm[(g + 1) * rows] = e;
+      for (int p = s + lane; p < e; p += LANES, ++i)
+        if (i < a.keep) {
+          vsm[i * threads] = __ldg(gval + p);
+          csm[i * threads] = __ldg(gcol + p);
+        }
+      s = e;
+    }
+  } else if (sl < S) {
+    int i = 0;
+    int off = 0;
+    if constexpr (KIND == KIND_SLICED) off = __ldg(A.row_ptr + sl) + (tid & 31);
+    for (int g = 0; g < G; ++g) {
+      const int w = __ldg(A.tile_row + sl * G + g);
+      if constexpr (DICT) off = __ldg(A.row_ptr + g * (S + 1) + sl);
+      rpsm[(2 * g) * rows] = w;
+      rpsm[(2 * g + 1) * rows] = off;
+      if constexpr (DICT) {
+        const C4* cp = reinterpret_cast<const C4*>(codes + (size_t)CB * off) + (tid & 31);
+        for (int q = 0; q < (w + 3) / 4; ++q, ++i)
+          if (i < a.keep) wsm[i * threads] = __ldg(cp + 32 * q);
+      } else {
+        for (int j = 0; j < w; ++j, ++i)
+          if (i < a.keep) {
+            vsm[i * threads] = __ldg(gval + off + 32 * j);
+            csm[i * threads] = __ldg(gcol + off + 32 * j);
+          }
+        off += 32 * w;
+      }
+    }
+  }
+  const bool owner = valid && lane == 0;
+  const size_t n64 = (size_t)n;
+  ST* kg = static_cast<ST*>(rk.k) + row;
+  cx<R> base{0, 0};
+  if (owner) {
+    if constexpr (MIXED) base = ld_cx<R>(static_cast<const ST*>(rk.y_prev_s) + row);
+    else base = ld_cx<R>(static_cast<const YT*>(rk.y_prev) + row);
+    for (int j = 0; j < a.s0; ++j) ksm[j * rows] = kg[(size_t)j * n64];
+  }
+  __syncthreads();
+  ST* ytmp = static_cast<ST*>(a.ytmp);
+  unsigned int target = a.bar_base;
+  bool ok = true;
+  // out = base + sum_{j <= s} (dt a_{s+1,j}) k_j, in the reference's order
+  auto form_input = [&](int s) {
+    cx<R> v = base;
+    const unsigned int nz = nz_s[s];
+    for (int j = 0; j <= s; ++j)
+      if ((nz >> j) & 1u) cx_axpy(v, fac[s][j], ld_cx<R>(ksm + j * rows));
+    st_cx(ytmp + (size_t)((s + 1) & 1) * n64 + row, v);
+  };
+  if (a.s0 > 0) {  // the first stage's input (stages 10..15 follow an accepted step)
+    if (owner) form_input(a.s0 - 1);
+    target += gridDim.x;
+    ok = grid_barrier(a.bar, target, &ok_s);
+  }
+
+  // ---- stages ----
+  double err_acc = 0.0;
+  const int last_col = (int)A.n_cols - 1;
+  for (int s = a.s0; s < a.s1 && ok; ++s) {
+    const ST* x = s == 0 ? static_cast<const ST*>(a.x0) : ytmp + (size_t)(s & 1) * n64;
+    cx<R> acc{0, 0};
+    if constexpr (KIND == KIND_CSR) {
+      int i = 0;
+      int ps = rpsm[0];
+      for (int g = 0; g < G; ++g) {
+        const int pe = rpsm[(g + 1) * rows];
+        R ar = 0, ai = 0;
+        for (int p = ps + lane; p < pe; p += LANES, ++i) {
+          ST v;
+          int c;
+          if (i < a.keep) {
+            v = vsm[i * threads];
+            c = csm[i * threads];
+          } else {
+            v = __ldg(gval + p);
+            c = __ldg(gcol + p);
+          }
+          cmac_any(ar, ai, v, x[c]);
+        }
+        acc = cx_add(acc, cx_mul(coef[s][g], sub_reduce<LANES>(ar, ai)));
+        ps = pe;
+      }
+    } else if constexpr (KIND == KIND_SLICED) {
+      if (sl < S) {
+        int i = 0;
+        for (int g = 0; g < G; ++g) {
+          const int w = rpsm[(2 * g) * rows], off = rpsm[(2 * g + 1) * rows];
+          R ar = 0, ai = 0;
+          for (int j = 0; j < w; ++j, ++i) {
+            ST v;
+            int c;
+            if (i < a.keep) {
+              v = vsm[i * threads];
+              c = csm[i * threads];
+            } else {
+              v = __ldg(gval + off + 32 * j);
+              c = __ldg(gcol + off + 32 * j);
+            }
+            cmac_any(ar, ai, v, x[c]);
+          }
+          acc = cx_add(acc, cx_mul(coef[s][g], cx<R>{ar, ai}));
+        }
+      }
+    } else {
+      if (sl < S) {
+        int i = 0;
+        for (int g = 0; g < G; ++g) {
+          const int w = rpsm[(2 * g) * rows], off = rpsm[(2 * g + 1) * rows];
+          const int t0 = tstart[g], tn = tstart[g + 1] - t0;
+          const C4* cp = reinterpret_cast<const C4*>(codes + (size_t)CB * off) + (tid & 31);
+          const bool direct = sizeof(R) == 8 && ccls[s][g] == 0;
+          R ar = direct ? acc.re : (R)0, ai = direct ? acc.im : (R)0;
+          for (int q = 0; 4 * q < w; ++q, ++i) {
+            const C4 c4 = i < a.keep ? wsm[i * threads] : __ldg(cp + 32 * q);
+            const int m = min(4, w - 4 * q);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              if (u < m) {
+                int k = Codes4<CB>::at(c4, u);
+                if constexpr (RI) {  // FP64-bound: skip a position that is padding everywhere
+                  if (!__any_sync(0xffffffffu, k != 0)) continue;
+                }
+                k = t0 + (k < tn ? k : 0);  // a table index of this group whatever the code
+                dict_mac<RI, false>(tval, toff, x, k, row, last_col, ar, ai);
+              }
+            }
+          }
+          if (direct) acc = cx<R>{ar, ai};
+          else coef_mac(acc, coef[s][g], ar, ai);
+        }
+      }
+    }
+    if (owner) {
+      st_cx(ksm + s * rows, acc);
+      kg[(size_t)s * n64] = ksm[s * rows];
+      if (s == RK_STEP - 1) {
+        const unsigned int nz = nz_s[s], ne = nz_s[RK_EXTRA_STEP];
+        if constexpr (MIXED) {
+          cx<R> inc{0, 0};
+          float erh = 0.f, erl = 0.f, eih = 0.f, eil = 0.f;
+          for (int j = 0; j < RK_STEP; ++j) {
+            const cx<R> kj = ld_cx<R>(ksm + j * rows);
+            if ((nz >> j) & 1u) cx_axpy(inc, fac[s][j], kj);
+            if ((ne >> j) & 1u) {  // the error estimate in float-float
+              ff_acc(erh, erl, fe_s[j], fel_s[j], (float)kj.re);
+              ff_acc(eih, eil, fe_s[j], fel_s[j], (float)kj.im);
+            }
+          }
+          const double2 yp = static_cast<const double2*>(rk.y_prev)[row];
+          const double2 yf = make_double2(yp.x + (double)inc.re, yp.y + (double)inc.im);
+          static_cast<double2*>(rk.y_front)[row] = yf;
+          static_cast<float2*>(rk.y_front_s)[row] = make_float2((float)yf.x, (float)yf.y);
+          const double er = (double)erh + (double)erl, ei = (double)eih + (double)eil;
+          err_acc = wrms_term(er * er + ei * ei, yf.x * yf.x + yf.y * yf.y, rk.atol, rk.rtol);
+        } else {
+          cx<R> y = base, e{0, 0};
+          for (int j = 0; j < RK_STEP; ++j) {
+            const cx<R> kj = ld_cx<R>(ksm + j * rows);
+            if ((nz >> j) & 1u) cx_axpy(y, fac[s][j], kj);
+            if ((ne >> j) & 1u) cx_axpy(e, fe_s[j], kj);
+          }
+          YT yq;
+          st_cx(&yq, y);
+          static_cast<YT*>(rk.y_front)[row] = yq;
+          const cx<R> ys = ld_cx<R>(&yq);
+          const double mag2 = (double)ys.re * ys.re + (double)ys.im * ys.im;
+          const double sc = rk.atol + rk.rtol * sqrt(mag2);
+          err_acc = ((double)e.re * e.re + (double)e.im * e.im) / (sc * sc);
+        }
+      } else if (s + 1 < a.s1) {
+        form_input(s);
+      }
+    }
+    if (s + 1 < a.s1) {
+      target += gridDim.x;
+      ok = grid_barrier(a.bar, target, &ok_s);
+    }
+  }
+  if (!ok) {
+    if (tid == 0) {
+      atomicOr(&g_step_fault, 1u);
+      if (rk.result) *rk.result = -1.0;
+    }
+    return;
+  }
+  if (a.s1 != RK_STEP) return;
+  // WRMS error: block partials, summed in block order by the block that finishes last
+  __syncthreads();
+  double v = err_acc;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((tid & 31) == 0) red[tid >> 5] = v;
+  __syncthreads();
+  if (tid == 0) {
+    double t = 0.0;
+    for (int w = 0; w < threads / 32; ++w) t += red[w];
+    rk.scratch[blockIdx.x] = t;
+    __threadfence();
+    last_s = atomicAdd(rk.counter, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last_s || tid >= 32) return;
+  __threadfence();
+  double t = 0.0;
+  for (int i = tid; i < (int)gridDim.x; i += 32) t += __ldcg(rk.scratch + i);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  if (tid == 0) {
+    *rk.result = sqrt(t / (double)n);
+    *rk.counter = 0u;
+  }
+}
+
+constexpr int STEP_MAX_SMEM = 220 * 1024;
+
+// 1 when the launch does not fit (the caller then takes one launch per stage).
+template <int DT, int YDT, int KIND, int LANES>
+static int launch_range(StepArgs& a, uint32_t* bar_base, cudaStream_t st) {
+  using ST = typename elem<DT>::T;
+  const int64_t warps = (a.A.n_rows * LANES + 31) / 32;
+  const int64_t sms = sm_count();
+  int64_t per = (warps + sms - 1) / sms;  // warps of a block, one block per SM
+  if (per < STEP_MIN_WARPS) per = STEP_MIN_WARPS;
+  if (per * 32 > STEP_THREADS) return 1;
+  const int threads = (int)per * 32, rows = threads / LANES;
+  const int grid = (int)((warps + per - 1) / per);
+  a.keep = STEP_KEEP;
+  int smem = step_smem<ST>(a.A, KIND, threads, rows, a.keep).total;
+  if (smem > STEP_MAX_SMEM) {
+    a.keep = 2;
+    smem = step_smem<ST>(a.A, KIND, threads, rows, a.keep).total;
+    if (smem > STEP_MAX_SMEM) return 1;
+  }
+  auto kern = vern7_range_kernel<DT, YDT, KIND, LANES>;
+  static std::mutex mu;
+  static bool opted[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
+    return set_error(QG_ERR_CUDA, "no current CUDA device");
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (!opted[dev]) {
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               STEP_MAX_SMEM) != cudaSuccess)
+        return set_error(QG_ERR_CUDA, "fused step kernel: shared memory opt-in failed");
+      opted[dev] = true;
+    }
+  }
+  a.bar_base = *bar_base;
+  void* args[] = {&a};
+  if (cudaLaunchCooperativeKernel((const void*)kern, dim3((unsigned)grid), dim3((unsigned)threads),
+                                  args, (size_t)smem, st) != cudaSuccess)
+    return check_launch("vern7_range_kernel");
+  const int barriers = (a.s1 - a.s0 - 1) + (a.s0 > 0 ? 1 : 0);
+  if (grid > 1) *bar_base += (uint32_t)(barriers * grid);
+  return check_launch("vern7_range_kernel");
+}
+
+template <int DT, int YDT>
+static int launch_range_layout(StepArgs& a, uint32_t* bar_base, cudaStream_t st) {
+  const qg_csr_groups& A = a.A;
+  switch (A.layout) {
+    case QG_LAYOUT_ROW_MAJOR:
+      switch (A.lanes) {
+        case 2: return launch_range<DT, YDT, KIND_CSR, 2>(a, bar_base, st);
+        case 4: return launch_range<DT, YDT, KIND_CSR, 4>(a, bar_base, st);
+        case 8: return launch_range<DT, YDT, KIND_CSR, 8>(a, bar_base, st);
+        default: return 1;
+      }
+    case QG_LAYOUT_SLICED: return launch_range<DT, YDT, KIND_SLICED, 1>(a, bar_base, st);
+    case QG_LAYOUT_SLICED_DICT:
+      if (DT == QG_C128) return 1;  // complex128 dictionaries are split
+      return A.tile_nnz == 1 ? launch_range<DT, YDT, KIND_DICT1, 1>(a, bar_base, st)
+                             : launch_range<DT, YDT, KIND_DICT2, 1>(a, bar_base, st);
+    case QG_LAYOUT_SLICED_DICT_RI:
+      return A.tile_nnz == 1 ? launch_range<DT, YDT, KIND_DICT1, 1>(a, bar_base, st)
+                             : launch_range<DT, YDT, KIND_DICT2, 1>(a, bar_base, st);
+    default: return 1;
+  }
+}
+
+}  // namespace qg
+
+using namespace qg;
+
+int step_fault_take() {
+  unsigned int v = 0, zero = 0;
+  if (cudaMemcpyFromSymbol(&v, g_step_fault, sizeof(v)) != cudaSuccess) return 0;
+  if (v) cudaMemcpyToSymbol(g_step_fault, &zero, sizeof(zero));
+  return (int)v;
+}
+
+extern "C" int qg_vern7_range(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0,
+                              int stage1, double t_prev, double dt, double atol, double rtol,
+                              unsigned int* barrier, uint32_t* barrier_base, void* stream) {
+  int rc = check_groups(A);
+  if (rc) return rc;
+  if (!barrier || !barrier_base) return set_error(QG_ERR_ARG, "null barrier word");
+  if (A->n_rows != A->n_cols) return set_error(QG_ERR_ARG, "operator must be square with n rows");
+  if (!((stage0 == 0 && stage1 == RK_STEP) || (stage0 == RK_STEP && stage1 == RK_EXTRA_STEP)))
+    return set_error(QG_ERR_ARG, "stages must be a whole trial step or the dense-output stages");
+  StepArgs a{};
+  const void* x = nullptr;
+  rc = prepare_stage(B, A->dtype, A->n_rows, stage0 == 0 ? RK_STEP - 1 : stage0, dt, atol, rtol,
+                     a.rk, x);
+  if (rc) return rc;
+  if (B->n == 0) return 1;
+  a.A = *A;
+  a.x0 = B->state_dtype != B->stage_dtype ? B->y_prev_s : B->y_prev;
+  a.ytmp = B->ytmp;
+  a.t_prev = t_prev;
+  a.dt = dt;
+  a.s0 = stage0;
+  a.s1 = stage1;
+  a.bar = barrier;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (B->state_dtype == QG_C128 && B->stage_dtype == QG_C128)
+    return launch_range_layout<QG_C128, QG_C128>(a, barrier_base, st);
+  if (B->state_dtype == QG_C128) return launch_range_layout<QG_C64, QG_C128>(a, barrier_base, st);
+  return launch_range_layout<QG_C64, QG_C64>(a, barrier_base, st);
+}

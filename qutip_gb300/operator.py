@@ -677,6 +677,18 @@ class DeviceOperator:
         _lib.check(lib.qg_vern7_stage(C.byref(self.struct), C.byref(rk), stage, t_prev, dt,
                                       atol, rtol, stream), "qg_vern7_stage")
 
+    def vern7_range(self, rk, stage0: int, stage1: int, t_prev: float, dt: float, atol: float,
+                    rtol: float, barrier: int, base, stream: int) -> bool:
+        """A whole trial step (stages 0..9) or the dense-output stages (10..15) in one
+        launch (``qg_vern7_range``); False, without a launch, when the operator does not
+        fit that kernel."""
+        rc = _lib.load().qg_vern7_range(C.byref(self.struct), C.byref(rk), stage0, stage1, t_prev,
+                                        dt, atol, rtol, barrier, C.byref(base), stream)
+        if rc == 1:
+            return False
+        _lib.check(rc, "qg_vern7_range")
+        return True
+
     def matmat(self, t: float, X: torch.Tensor, Y: torch.Tensor, alpha=1.0, beta=0.0):
         """``Y = alpha A(t) X + beta Y`` for F-ordered column blocks stored as ``[n_vec, n]``."""
         if X.dtype != _TORCH[self.dtype] or Y.dtype != _TORCH[self.dtype]:

@@ -4,9 +4,11 @@ The control flow mirrors ``Explicit_RungeKutta`` (qutip/solver/integrator/explic
 step for step -- first-step estimate, ``integrate`` with ``step=True`` for
 Monte-Carlo stepping, ``_step_in_err`` retries, interpolation past the target
 with the 7th-order dense output -- so that the step sequence, and therefore the
-result, is the reference's.  The vector work runs in three kinds of launches:
+result, is the reference's.  The vector work runs in these kinds of launches:
 
-* ``qg_vern7_stage`` -- one per stage: the matvec ``k_s = A(t_s) x_s`` fused
+* ``qg_vern7_range`` -- all ten stages of a trial step, or the six dense-output stages, in
+  one launch, for operators whose rows all fit the GPU at once;
+* ``qg_vern7_stage`` -- otherwise one per stage: the matvec ``k_s = A(t_s) x_s`` fused
   with the next stage's input combination; the tenth fuses ``y_front`` and the
   FP64 WRMS error reduction (``wrmn_error_dense``, qutip/core/data/ode.pyx:27-52);
 * ``qg_rk_combine`` -- dense-output stage input and materialised outputs;
@@ -91,7 +93,9 @@ class GpuVern7:
         self.ytmp = torch.zeros(2 * n, dtype=kdt, device=dev)
         self.scratch = torch.zeros(int(_lib.load().qg_scratch_doubles()), dtype=torch.float64,
                                    device=dev)
+        # word 0: reductions (left zero); word 1: arrivals at the fused step kernel's barrier
         self.counter = torch.zeros(4, dtype=torch.int32, device=dev)
+        self._barrier_base = C.c_uint32(0)
         self.result = torch.zeros(4, dtype=torch.float64, device=dev)
         self._host = torch.zeros(4, dtype=torch.float64).pin_memory()
         self.y_prev, self.y_front = self._ya, self._yb
@@ -276,21 +280,37 @@ class GpuVern7:
         # explicit_rk.pyx:358-397: ten fused stages; the last returns the error
         rk = self._rk()
         s = stream_ptr()
-        for i in range(T.RK_STEP):
-            self.op.vern7_stage(rk, i, self.t_prev, dt, self.atol, self.rtol, s)
+        fused = self._range(rk, 0, T.RK_STEP, dt, s)
+        if not fused:
+            for i in range(T.RK_STEP):
+                self.op.vern7_stage(rk, i, self.t_prev, dt, self.atol, self.rtol, s)
         self.stats["rhs"] += T.RK_STEP
         self.t_front = self.t_prev + dt
-        return self._read_result()
+        error = self._read_result()
+        if fused and error < 0:
+            self.counter.zero_()
+            self._barrier_base.value = 0
+            raise IntegratorError("a device wait of the fused step kernel gave up; the GPU may "
+                                  "be unhealthy")
+        return error
+
+    def _range(self, rk, stage0, stage1, dt, s) -> bool:
+        """The stages in one launch where the operator's rows all fit the GPU at once."""
+        run = getattr(self.op, "vern7_range", None)
+        return run is not None and run(rk, stage0, stage1, self.t_prev, dt, self.atol, self.rtol,
+                                       self.counter.data_ptr() + 4, self._barrier_base, s)
 
     def _prep_dense_out(self):
         # explicit_rk.pyx:399-410
         dt = self.dt_int
         rk = self._rk()
-        self._combine(self._stage_base(), [dt * self.a[T.RK_STEP, j] for j in range(T.RK_STEP)],
-                      self._ytmp(T.RK_STEP & 1))
         s = stream_ptr()
-        for i in range(T.RK_STEP, T.RK_EXTRA_STEP):
-            self.op.vern7_stage(rk, i, self.t_prev, dt, self.atol, self.rtol, s)
+        if not self._range(rk, T.RK_STEP, T.RK_EXTRA_STEP, dt, s):
+            self._combine(self._stage_base(),
+                          [dt * self.a[T.RK_STEP, j] for j in range(T.RK_STEP)],
+                          self._ytmp(T.RK_STEP & 1))
+            for i in range(T.RK_STEP, T.RK_EXTRA_STEP):
+                self.op.vern7_stage(rk, i, self.t_prev, dt, self.atol, self.rtol, s)
         self.stats["rhs"] += T.RK_EXTRA_STEP - T.RK_STEP
 
     def dense_factors(self, t):
