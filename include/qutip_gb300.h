@@ -304,6 +304,22 @@ int qg_vern7_range(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0, i
                    double t_prev, double dt, double atol, double rtol, unsigned int* barrier,
                    uint32_t* barrier_base, void* stream);
 
+/* *flag = 1 (left alone otherwise) unless the dictionary-coded superoperator A maps
+ * Hermitian d x d matrices to Hermitian ones, group by group (every entry of row (r, c) has
+ * its conjugate at the mirrored place of row (c, r), to rounding), and rho (state dtype,
+ * vec order) is Hermitian to rounding.  With real coefficients the stages may then go
+ * through qg_vern7_stage_herm.  The reference's counterpart is the test before
+ * assume_hermitian_state (qutip/solver/mesolve.py:270-277).  d a multiple of 32, the
+ * layout QG_LAYOUT_SLICED_DICT_RI (complex128) or QG_LAYOUT_SLICED_DICT (complex64). */
+int qg_hermitian_check(const qg_csr_groups* A, int64_t d, const void* rho, int rho_dtype,
+                       int* flag, void* stream);
+
+/* qg_vern7_stage for an operator and a state that passed qg_hermitian_check and real
+ * coefficients: the elements (r, c) on and below the diagonal blocks are evaluated and the
+ * others written as their conjugates. */
+int qg_vern7_stage_herm(const qg_csr_groups* A, int64_t d, const qg_rk_buffers* B, int stage,
+                        double t_prev, double dt, double atol, double rtol, void* stream);
+
 /* y = alpha * L(t)[x] + beta * y for the matrix-free Lindblad generator; x and y
  * are vec(rho) of length d*d in L's dtype.  Replaces LindbladMatrixForm.matmul_data
  * (qutip/core/cy/lindblad_matrix_form.pyx:105-204). */

@@ -103,6 +103,11 @@ _SIGS = {
     "qg_vern7_range": (C.c_int, [_P(CsrGroups), _P(RkBuffers), C.c_int, C.c_int, C.c_double,
                                  C.c_double, C.c_double, C.c_double, C.c_void_p,
                                  _P(C.c_uint32), C.c_void_p]),
+    "qg_hermitian_check": (C.c_int, [_P(CsrGroups), C.c_int64, C.c_void_p, C.c_int, C.c_void_p,
+                                     C.c_void_p]),
+    "qg_vern7_stage_herm": (C.c_int, [_P(CsrGroups), C.c_int64, _P(RkBuffers), C.c_int,
+                                      C.c_double, C.c_double, C.c_double, C.c_double,
+                                      C.c_void_p]),
     "qg_lindblad_apply": (C.c_int, [_P(Lindblad), C.c_double, C.c_void_p, C.c_void_p,
                                     C.c_double, C.c_double, C.c_double, C.c_double,
                                     C.c_void_p]),
@@ -142,8 +147,8 @@ _lib = None
 # Entry points that launch exactly one kernel each; calls are counted so that a
 # benchmark can report how many of this library's kernels ran in a timed region.
 COMPUTE_ENTRY_POINTS = {
-    "qg_spmv_csr", "qg_spmm_csr", "qg_spmv_dia", "qg_vern7_stage", "qg_vern7_range", "qg_rk_combine",
-    "qg_norm2",
+    "qg_spmv_csr", "qg_spmm_csr", "qg_spmv_dia", "qg_vern7_stage", "qg_vern7_stage_herm", "qg_vern7_range",
+    "qg_hermitian_check", "qg_rk_combine", "qg_norm2",
     "qg_expect_dm", "qg_expect_ket", "qg_expect_dm_times", "qg_batch_vern7", "qg_batch_vern7_noalloc",
     "qg_lindblad_apply", "qg_lindblad_stage", "qg_dense_lindblad_apply", "qg_dense_lindblad_stage",
     "qg_sde_platen", "qg_sde_euler",

@@ -11,6 +11,7 @@ reference's CSR (qutip/core/data/csr.pxd:17-30, 32-bit ``idxint``).
 from __future__ import annotations
 
 import ctypes as C
+import math
 
 import numpy as np
 import scipy.sparse as sp
@@ -676,6 +677,39 @@ class DeviceOperator:
         lib = _lib.load()
         _lib.check(lib.qg_vern7_stage(C.byref(self.struct), C.byref(rk), stage, t_prev, dt,
                                       atol, rtol, stream), "qg_vern7_stage")
+
+    # -- Hermitian half form ------------------------------------------------
+    def hermitian_dim(self) -> int:
+        """The Hilbert dimension d when this operator can act on a Hermitian d x d state by
+        half (dictionary-coded d*d x d*d storage, d a multiple of 32, and enough rows that
+        the stages go out one by one: more than 512 per SM), else 0."""
+        split = getattr(self, "dict_split", False)
+        if self.fmt != "dict" or self.n_rows != self.n_cols or split != (self.dtype == "c128"):
+            return 0
+        sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+        d = math.isqrt(self.n_rows)
+        return d if d * d == self.n_rows and d % 32 == 0 and self.n_rows > 512 * sms else 0
+
+    def real_coefficients(self) -> bool:
+        """Whether every group's coefficient is real at every t."""
+        return all(c is None or c.is_real() for c in self.coeffs)
+
+    def check_hermitian(self, rho: torch.Tensor) -> bool:
+        """Whether the generator keeps Hermitian matrices Hermitian and ``rho`` is one
+        (``qg_hermitian_check``; reads the answer back)."""
+        flag = torch.zeros(1, dtype=torch.int32, device=self.device)
+        _lib.call("qg_hermitian_check", C.byref(self.struct), self.hermitian_dim(),
+                  rho.data_ptr(), _lib.QG_C128 if rho.dtype == torch.complex128 else _lib.QG_C64,
+                  flag.data_ptr(), stream_ptr())
+        return int(flag.item()) == 0
+
+    def vern7_stage_herm(self, rk, stage: int, t_prev: float, dt: float, atol: float, rtol: float,
+                         stream: int):
+        """:meth:`vern7_stage` on a Hermitian state (``qg_vern7_stage_herm``)."""
+        lib = _lib.load()
+        _lib.check(lib.qg_vern7_stage_herm(C.byref(self.struct), math.isqrt(self.n_rows),
+                                           C.byref(rk), stage, t_prev, dt, atol, rtol, stream),
+                   "qg_vern7_stage_herm")
 
     def vern7_range(self, rk, stage0: int, stage1: int, t_prev: float, dt: float, atol: float,
                     rtol: float, barrier: int, base, stream: int) -> bool:

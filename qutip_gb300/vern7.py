@@ -107,6 +107,7 @@ class GpuVern7:
         else:
             self.y_prev_s = self.y_front_s = None
         self._set = False
+        self._hermitian = False   # decided for each initial value
         self.status = NOT_INITIATED
         self.stats = {"steps": 0, "rejected": 0, "rhs": 0}
         self._out = ("front", None)  # how the state at self.t is obtained
@@ -173,6 +174,9 @@ class GpuVern7:
         self._out = ("front", None)
         self.status = NORMAL
         self._set = True
+        dim = getattr(self.op, "hermitian_dim", None)
+        self._hermitian = (dim is not None and dim() > 0 and self.op.real_coefficients()
+                           and self.op.check_hermitian(self.y_prev))
         self.dt_safe = self._estimate_first_step(self.t, self.y_prev) if not self.first_step \
             else self.first_step
 
@@ -282,8 +286,9 @@ class GpuVern7:
         s = stream_ptr()
         fused = self._range(rk, 0, T.RK_STEP, dt, s)
         if not fused:
+            stage = self._stage()
             for i in range(T.RK_STEP):
-                self.op.vern7_stage(rk, i, self.t_prev, dt, self.atol, self.rtol, s)
+                stage(rk, i, self.t_prev, dt, self.atol, self.rtol, s)
         self.stats["rhs"] += T.RK_STEP
         self.t_front = self.t_prev + dt
         error = self._read_result()
@@ -293,6 +298,14 @@ class GpuVern7:
             raise IntegratorError("a device wait of the fused step kernel gave up; the GPU may "
                                   "be unhealthy")
         return error
+
+    def _stage(self):
+        """The operator's stage launch: by half when the state is a Hermitian density matrix
+        that the generator keeps Hermitian (the coefficients may have been replaced since
+        the state was set, so their part is looked at again)."""
+        if self._hermitian and self.op.real_coefficients():
+            return self.op.vern7_stage_herm
+        return self.op.vern7_stage
 
     def _range(self, rk, stage0, stage1, dt, s) -> bool:
         """The stages in one launch where the operator's rows all fit the GPU at once."""
@@ -309,8 +322,9 @@ class GpuVern7:
             self._combine(self._stage_base(),
                           [dt * self.a[T.RK_STEP, j] for j in range(T.RK_STEP)],
                           self._ytmp(T.RK_STEP & 1))
+            stage = self._stage()
             for i in range(T.RK_STEP, T.RK_EXTRA_STEP):
-                self.op.vern7_stage(rk, i, self.t_prev, dt, self.atol, self.rtol, s)
+                stage(rk, i, self.t_prev, dt, self.atol, self.rtol, s)
         self.stats["rhs"] += T.RK_EXTRA_STEP - T.RK_STEP
 
     def dense_factors(self, t):
