@@ -10,9 +10,18 @@
 // full non-Hermitian branch) with dense operators.  Per collapse operator two products:
 // T = X C^dag, then C T.
 //
-// Work split: CTA j owns the 16 output columns [16 j, 16 j + 16) of every product; column n
-// of A X, X A^dag, T = X C^dag and C T needs only column n of X, of A^dag, of C^dag and of
-// T, so the CTAs never exchange data and T's block stays in the CTA's shared memory.
+// Work split: a cluster of CTAs owns the 16 output columns [16 j, 16 j + 16); column n of
+// A X, X A^dag, T = X C^dag and C T needs only column n of X, of A^dag, of C^dag and of T.
+// The terms of the sum are independent, so each goes to a CTA of its own: rank 0 takes A X
+// and X A^dag (two ranks without collapse operators), rank 1 + i the pair of products of
+// C_i, whose T stays in its shared memory; more than seven collapse operators go round the
+// ranks.  The partial sums meet through distributed shared memory, added in rank order by
+// the CTA that runs the epilogue of those elements.  Every product is a chain of K chunks
+// whose staging is latency, not tensor work (the MMAs of a chunk take 0.55 us of its 3 us),
+// so the chain's length is the time: six products in a row on one CTA per 16 columns took
+// 77 us at d = 128 with two collapse operators.  Measured with the split, and with the
+// operator's groups merged per coefficient: the whole d = 128 solve (156 right-hand sides)
+// 14.7 -> 7.9 ms.
 // One CTA of 512 threads computes Y = Aop Bop^T (M = 128 rows, N = 16 columns) in K chunks
 // of 32: every thread writes its share of the chunk's operand planes (real / imaginary x
 // TF32 hi / lo) into one of two shared-memory buffers, one thread issues the 6 MMAs per
@@ -24,6 +33,7 @@
 // level (a chain over all of K loses up to 5x more, growing with d).  The accumulated
 // generator goes through the same fused Vern7 epilogue as the sparse kernels (stage.cuh).
 // The stage vectors are complex64: this is the mixed form's generator.
+#include <cooperative_groups.h>
 #include <mutex>
 
 #include "capi_internal.h"
@@ -115,6 +125,7 @@ __device__ __forceinline__ void load_chunk(const DenseCtx& c, int src, int row0,
       if (in[i]) ch.v[i] = base[off[i]];
     return;
   }
+#pragma unroll 2
   for (int g = 0; g < L.n_groups; ++g) {  // A(t) = sum_g a_g(t) A_g
     const float2 a = c.ca[g];
     const float2* bg = base + (size_t)g * d * d;
@@ -211,7 +222,10 @@ __global__ void __launch_bounds__(DN_THREADS, 1)
   __shared__ double red[DN_THREADS / 32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int d = L.d;
-  const int n0 = blockIdx.x * DN_NB;
+  namespace cgrp = cooperative_groups;
+  cgrp::cluster_group cl = cgrp::this_cluster();
+  const int ranks = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int n0 = (int)(blockIdx.x / (unsigned)ranks) * DN_NB;
   unsigned char* a_planes = dn_smem;                      // 2 buffers
   unsigned char* b_planes = dn_smem + 2 * DN_BUF_A;       // 2 buffers
   float2* t_blk = reinterpret_cast<float2*>(dn_smem + 2 * DN_BUF_A + 2 * DN_BUF_B);
@@ -251,6 +265,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1)
   float prod[DN_CW], gen[DN_CW];
 #pragma unroll
   for (int j = 0; j < DN_CW; ++j) gen[j] = 0.f;
+  // (a rank without a product leaves its partial sum zero)
 
   auto wait_buf = [&](int b) {
     const bool r = __syncthreads_and(mbar_poll(&bar[b], par[b]) ? 1 : 0) != 0;
@@ -317,14 +332,18 @@ __global__ void __launch_bounds__(DN_THREADS, 1)
     for (int j = 0; j < DN_CW; ++j) gen[j] = fmaf(w, prod[j], gen[j]);
   };
 
-  gemm(SRC_OPA, SRC_XB, false);  // A X
-#pragma unroll
-  for (int j = 0; j < DN_CW; ++j) gen[j] = prod[j];
-  gemm(SRC_XA, SRC_OPA, true);   // X A^dag
-  accumulate(1.f);
+  if (rank == 0) {
+    gemm(SRC_OPA, SRC_XB, false);  // A X
+    accumulate(1.f);
+  }
+  if (rank == (L.n_cops == 0 ? 1 : 0)) {
+    gemm(SRC_XA, SRC_OPA, true);   // X A^dag
+    accumulate(1.f);
+  }
   for (int i = 0; i < L.n_cops && ok; ++i) {
+    if ((1 + i) % ranks != rank) continue;
     c.cop = i;
-    gemm(SRC_XA, SRC_OPC, true);  // T = X C^dag, this CTA's columns
+    gemm(SRC_XA, SRC_OPC, true);  // T = X C^dag, this cluster's columns
     float* tp = reinterpret_cast<float*>(t_blk) + part;
 #pragma unroll
     for (int j = 0; j < DN_CW; ++j) tp[2 * ((cw0 + j) * DN_TS + m)] = prod[j];
@@ -334,17 +353,26 @@ __global__ void __launch_bounds__(DN_THREADS, 1)
   }
 
   double err_acc = 0.0;
+  // real and imaginary parts meet in shared memory (the A planes are free once every chunk's
+  // MMAs are done; after a wait that gave up they may not be, and nothing is written)
   if (ok) {
-    // real and imaginary parts meet in shared memory (the A planes are free now)
     float* ex = reinterpret_cast<float*>(a_planes) + part;
 #pragma unroll
     for (int j = 0; j < DN_CW; ++j) ex[2 * ((cw0 + j) * 128 + m)] = gen[j];
-    __syncthreads();
-    const float2* exv = reinterpret_cast<const float2*>(a_planes);
+  }
+  cl.sync();  // every rank's partial sum is in its shared memory
+  if (ok) {
+    // the ranks share the elements of the column block; partial sums in rank order
     const int ncols = min(DN_NB, d - n0);
-    for (int e = tid; e < ncols * d; e += DN_THREADS) {
+    for (int e = tid + rank * DN_THREADS; e < ncols * d; e += ranks * DN_THREADS) {
       const int jl = e / d, mm = e - jl * d;
-      const float2 v = exv[jl * 128 + mm];
+      float2 v = make_float2(0.f, 0.f);
+      for (int q = 0; q < ranks; ++q) {
+        const float2 p =
+            cl.map_shared_rank(reinterpret_cast<float2*>(a_planes), q)[jl * 128 + mm];
+        v.x += p.x;
+        v.y += p.y;
+      }
       epilogue<QG_C64, YDT, EPI>((n0 + jl) * d + mm, cx<float>{v.x, v.y}, ax, rk,
                                  err_acc);
     }
@@ -354,6 +382,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1)
     for (int b = 0; b < 2; ++b)
       if (pend[b]) (void)mbar_poll(&bar[b], par[b]);
   }
+  cl.sync();  // no CTA leaves while another may still read its partial sum
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
@@ -364,6 +393,10 @@ __global__ void __launch_bounds__(DN_THREADS, 1)
 }
 
 static size_t dense_smem(int) { return DN_SMEM; }
+
+// CTAs of a cluster: A X and X A^dag, and a rank for each collapse operator up to seven
+// (eight CTAs is the portable cluster size); two without collapse operators.
+static int dense_ranks(int n_cops) { return n_cops == 0 ? 2 : (n_cops < 7 ? n_cops + 1 : 8); }
 
 template <int YDT, int EPI>
 static int launch_dense(cudaStream_t st, const qg_dense_lindblad& L, double t, const void* x,
@@ -384,8 +417,21 @@ static int launch_dense(cudaStream_t st, const qg_dense_lindblad& L, double t, c
       set_bytes[dev] = smem;
     }
   }
-  const int grid = (L.d + DN_NB - 1) / DN_NB;
-  kern<<<grid, DN_THREADS, smem, st>>>(L, t, static_cast<const float2*>(x), ax, rk);
+  const int ranks = dense_ranks(L.n_cops);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ranks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(ranks * ((L.d + DN_NB - 1) / DN_NB)));
+  cfg.blockDim = dim3(DN_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, L, t, static_cast<const float2*>(x), ax, rk) != cudaSuccess)
+    return check_launch("dense_lindblad_kernel");
   return check_launch("dense_lindblad_kernel");
 }
 

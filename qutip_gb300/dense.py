@@ -6,12 +6,11 @@ qutip/core/cy/lindblad_matrix_form.pyx:105-204) applies ``A rho + rho A^dag +
 sum_i C_i rho C_i^dag`` with ``A = -i H_nh`` through sparse or dense matmuls.  For a
 system of Hilbert dimension ``d <= 128`` whose operators are dense, those products are
 small dense GEMMs: :class:`DenseLindbladOperator` keeps ``A_g`` and ``C_i`` as complex64
-``d x d`` matrices and applies the generator in one CTA with ``tcgen05`` tensor-core
-MMAs (TF32 inputs split hi + lo, FP32 accumulation in tensor memory; ``qg_dense_lindblad_*``
-in ``csrc/dense.cu``; one CTA per 16 output columns; each K chunk of 32 in fresh
-accumulators, the large hi*hi part and the small hi*lo + lo*hi corrections apart, summed
-on the CUDA cores with round-to-nearest).  The stages are
-complex64, so it serves the mixed form
+``d x d`` matrices and applies the generator with ``tcgen05`` tensor-core MMAs (TF32
+inputs split hi + lo, FP32 accumulation in tensor memory; ``qg_dense_lindblad_*`` in
+``csrc/dense.cu``; a cluster of CTAs per 16 output columns, one CTA per term; each K chunk
+of 32 in fresh accumulators, the large hi*hi part and the small hi*lo + lo*hi corrections
+apart, summed on the CUDA cores with round-to-nearest).  The stages are complex64, so it serves the mixed form
 (``precision="mixed"``: FP64 state, step control and expectation values).
 
 Sparse operators (a Jaynes-Cummings system has three entries per row) keep the sparse
@@ -75,17 +74,26 @@ class DenseLindbladOperator:
             a = m.toarray() if sp.issparse(m) else np.asarray(m)
             if a.shape != (d, d):
                 raise ValueError("all operators must be d x d")
-            return a.astype(np.complex64)
-        self.a_coeffs = [c for _, c in a_terms]
+            return a.astype(np.complex128)
+        # terms that share a coefficient are one group (QobjEvo.compress): every group is
+        # read and scaled again at each application
+        groups: dict = {}
+        for m, c in a_terms:
+            key = None if c is None else c.key()
+            groups[key] = (groups[key][0] + dense(m), c) if key in groups else (dense(m), c)
+        self.a_coeffs = [c for _, c in groups.values()]
         self.c_coeffs = [c for _, c in c_terms]
-        self.a = torch.from_numpy(np.stack([dense(m) for m, _ in a_terms])).to(self.device)
-        self.c = (torch.from_numpy(np.stack([dense(m) for m, _ in c_terms])).to(self.device)
+
+        def single(mats):
+            return torch.from_numpy(np.stack(mats).astype(np.complex64)).to(self.device)
+        self.a = single([m for m, _ in groups.values()])
+        self.c = (single([dense(m) for m, _ in c_terms])
                   if c_terms else None)
         self._a_prog = self._programs(self.a_coeffs)
         self._c_prog = self._programs(self.c_coeffs)
         self.coeffs = self.a_coeffs + self.c_coeffs
         st = _lib.DenseLindblad()
-        st.d, st.n_groups, st.n_cops, st.reserved = d, len(a_terms), len(c_terms), 0
+        st.d, st.n_groups, st.n_cops, st.reserved = d, len(groups), len(c_terms), 0
         st.a, st.c = _ptr(self.a), _ptr(self.c)
         st.a_coef_code, st.a_coef_start, st.a_coef_consts = (_ptr(v) for v in self._a_prog)
         st.c_coef_code, st.c_coef_start, st.c_coef_consts = (_ptr(v) for v in self._c_prog)
@@ -142,8 +150,10 @@ class DenseLindbladOperator:
 
     @property
     def n_ctas(self) -> int:
-        """CTAs (one per SM) of one application: one per 16 output columns."""
-        return (self.d + 15) // 16
+        """CTAs (one per SM) of one application: a cluster per 16 output columns, of one CTA
+        for A X + X A^dag and one per collapse operator (two without any, eight at most)."""
+        ranks = 2 if self.n_cops == 0 else min(self.n_cops + 1, 8)
+        return ranks * ((self.d + 15) // 16)
 
     def gemm_flops(self) -> int:
         """Real multiply-adds x 2 of one application as issued: per complex product of two
