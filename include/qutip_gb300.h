@@ -44,8 +44,9 @@ typedef enum {
   QG_NORM_SEARCH_FAILED = -5, /* jump-time search exhausted (qutip/solver/mcsolve.py:363-367) */
   QG_TIMEOUT = -6,            /* cancelled through the host-visible cancel flag */
   QG_JUMP_OVERFLOW = -7,      /* more jumps than the batch's max_jumps */
-  QG_BAD_ITEM = -8            /* item not run: bad system index, state longer than max_n,
+  QG_BAD_ITEM = -8,           /* item not run: bad system index, state longer than max_n,
                                  or a group count outside 1..QG_MAX_GROUPS */
+  QG_DEVICE_WAIT = -9         /* a bounded device wait gave up (qg_vern7_integrate) */
 } qg_status;
 
 /* A sum of CSR matrices with time-dependent coefficients,
@@ -240,6 +241,33 @@ typedef struct qg_state_view {
   double f[16];
 } qg_state_view;
 
+/* The generator an integration drives, and the integrator's scalar state: the fields of
+ * Explicit_RungeKutta (qutip/solver/integrator/explicit_rk.pyx:47-203).  Host memory. */
+#define QG_GEN_CSR 0      /* op: qg_csr_groups */
+#define QG_GEN_LINDBLAD 1 /* op: qg_lindblad */
+#define QG_GEN_DENSE 2    /* op: qg_dense_lindblad */
+typedef struct qg_generator {
+  int32_t kind;
+  int32_t pad_;
+  const void* op;
+  int64_t hermitian_d; /* > 0: stages through qg_vern7_stage_herm (QG_GEN_CSR) */
+} qg_generator;
+typedef struct qg_vern7_ctl {
+  double t, t_prev, t_front, dt_safe, dt_int;
+  double atol, rtol, min_step, max_step;
+  int64_t max_numsteps;
+  int64_t steps, rejected, rhs; /* counts, added to */
+  int64_t launches;             /* kernels launched, added to */
+  int32_t status;               /* qg_status */
+  int32_t interpolate;
+  int32_t interp; /* 1: the state at t is the dense output of the current step */
+  int32_t swaps;  /* toggled when y_prev and y_front changed places */
+  uint32_t barrier_base;   /* of qg_vern7_range */
+  int32_t pad_;
+  unsigned int* barrier;   /* of qg_vern7_range (device) */
+  double* host_result;     /* one double of pinned host memory */
+} qg_vern7_ctl;
+
 /* ---- library ---------------------------------------------------------- */
 int qg_version(void);
 const char* qg_last_error(void);
@@ -391,6 +419,21 @@ int qg_sde_euler(const qg_sde* S, int32_t n_traj, void* states, const double* dW
 /* Non-zero when a kernel of this library gave up a bounded wait on the current
  * device (the result of that launch is invalid); reading clears the flag. */
 int qg_device_fault(void);
+
+/* Explicit_RungeKutta.integrate (explicit_rk.pyx:278-331) from c->t to t: trial steps until
+ * t is reached, then the dense output when it was passed; step != 0: one step at most.  The
+ * buffers' y_prev / y_front pointers change places as steps are accepted (c->swaps).  Failures
+ * of the integration are in c->status; waits for the error norm of each trial step. */
+int qg_vern7_integrate(const qg_generator* gen, qg_rk_buffers* B, qg_vern7_ctl* c, double t,
+                       int step, void* stream);
+
+/* The outputs of a master equation: integrate to each of n_times (host memory) and record
+ * the expectation values as qg_expect_dm does, one row of 2 (G + 1) doubles (device) per time,
+ * the times inside one step together (qg_expect_dm_times; ops group-major).  Stops at the
+ * first time the integration fails (c->status < 0). */
+int qg_vern7_run_dm(const qg_generator* gen, qg_rk_buffers* B, qg_vern7_ctl* c,
+                    const double* tlist, int n_times, const qg_csr_groups* ops, int64_t d,
+                    double* out, void* stream);
 
 /* out = base + sum_{j<n_k} f_j k_j (out in out_dtype).  Replaces _accumulate
  * and _interpolate_step (qutip/solver/integrator/explicit_rk.pyx:412-437). */

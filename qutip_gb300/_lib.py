@@ -84,6 +84,24 @@ class StateView(C.Structure):
                 ("f", C.c_double * 16)]
 
 
+class Generator(C.Structure):
+    _fields_ = [("kind", C.c_int32), ("pad_", C.c_int32), ("op", C.c_void_p),
+                ("hermitian_d", C.c_int64)]
+
+
+class Vern7Ctl(C.Structure):
+    _fields_ = [(n, C.c_double) for n in ("t", "t_prev", "t_front", "dt_safe", "dt_int", "atol",
+                                          "rtol", "min_step", "max_step")] + [
+        ("max_numsteps", C.c_int64), ("steps", C.c_int64), ("rejected", C.c_int64),
+        ("rhs", C.c_int64), ("launches", C.c_int64), ("status", C.c_int32),
+        ("interpolate", C.c_int32), ("interp", C.c_int32), ("swaps", C.c_int32),
+        ("barrier_base", C.c_uint32), ("pad_", C.c_int32), ("barrier", C.c_void_p),
+        ("host_result", C.c_void_p)]
+
+
+QG_GEN_CSR, QG_GEN_LINDBLAD, QG_GEN_DENSE = 0, 1, 2
+QG_DEVICE_WAIT = -9
+
 _P = C.POINTER
 _SIGS = {
     "qg_version": (C.c_int, []),
@@ -108,6 +126,10 @@ _SIGS = {
     "qg_vern7_stage_herm": (C.c_int, [_P(CsrGroups), C.c_int64, _P(RkBuffers), C.c_int,
                                       C.c_double, C.c_double, C.c_double, C.c_double,
                                       C.c_void_p]),
+    "qg_vern7_integrate": (C.c_int, [_P(Generator), _P(RkBuffers), _P(Vern7Ctl), C.c_double,
+                                     C.c_int, C.c_void_p]),
+    "qg_vern7_run_dm": (C.c_int, [_P(Generator), _P(RkBuffers), _P(Vern7Ctl), C.c_void_p, C.c_int,
+                                  _P(CsrGroups), C.c_int64, C.c_void_p, C.c_void_p]),
     "qg_lindblad_apply": (C.c_int, [_P(Lindblad), C.c_double, C.c_void_p, C.c_void_p,
                                     C.c_double, C.c_double, C.c_double, C.c_double,
                                     C.c_void_p]),
@@ -144,7 +166,7 @@ _SIGS = {
 
 _lib = None
 
-# Entry points that launch exactly one kernel each; calls are counted so that a
+# Entry points that launch exactly one kernel each (the drivers count their own); calls are counted so that a
 # benchmark can report how many of this library's kernels ran in a timed region.
 COMPUTE_ENTRY_POINTS = {
     "qg_spmv_csr", "qg_spmm_csr", "qg_spmv_dia", "qg_vern7_stage", "qg_vern7_stage_herm", "qg_vern7_range",

@@ -139,6 +139,10 @@ def _evolve(ig: GpuVern7, tlist, ex: ExpectOps, d: int, store_states, store_fina
 
     record(0)
     i = 1
+    if kind == "me" and G and not store_states and nt > 1 and \
+            ig.run_dm(tlist[1:], ex.dev, d, raw[1:]):
+        ig.check()
+        i = nt
     while i < nt:
         ig.integrate(float(tlist[i]))
         ig.check()

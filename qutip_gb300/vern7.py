@@ -19,7 +19,9 @@ Precision forms: ``"double"`` (complex128 operator, stages and state),
 state ``y``, the stage combinations and the error control in FP64) and
 ``"single"`` (complex64 state as well; error control still FP64).  The scalar
 step-size recurrences run on the host in IEEE double; the only per-step
-device-to-host transfer is the 8-byte error norm.
+device-to-host transfer is the 8-byte error norm.  For the library's own operators that
+host loop is the library's (``qg_vern7_integrate``); the methods below are the same loop for
+any other operator with ``matvec`` and ``vern7_stage``.
 """
 from __future__ import annotations
 
@@ -225,6 +227,10 @@ class GpuVern7:
         if not self._set:
             self.status = NOT_INITIATED
             return
+        gen = self._generator()
+        if gen is not None:
+            self._drive("qg_vern7_integrate", gen, t, int(step))
+            return
         if t == self.t:
             return
         if t < self.t_prev:
@@ -258,6 +264,59 @@ class GpuVern7:
             self.status = AT_FRONT
             self.t = self.t_front
             self._out = ("front", None)
+
+    # -- the same loop in the library ---------------------------------------
+    def _generator(self):
+        """The operator as the library's driver takes it (``qg_vern7_integrate``); None for
+        an operator that is not one of the library's own, which the loops here then drive."""
+        from .dense import DenseLindbladOperator
+        from .lindblad import LindbladOperator
+        kind = {DeviceOperator: _lib.QG_GEN_CSR, LindbladOperator: _lib.QG_GEN_LINDBLAD,
+                DenseLindbladOperator: _lib.QG_GEN_DENSE}.get(type(self.op))
+        if kind is None:
+            return None
+        half = self._hermitian and self.op.real_coefficients()
+        return _lib.Generator(kind, 0, C.addressof(self.op.struct),
+                              math.isqrt(self.n) if half else 0)
+
+    def _drive(self, name, gen, *args):
+        """Call a driver of the library on this integrator's buffers and scalar state."""
+        rk = self._rk()
+        c = _lib.Vern7Ctl(self.t, self.t_prev, self.t_front, self.dt_safe, self.dt_int, self.atol,
+                          self.rtol, self.min_step, self.max_step, self.max_numsteps,
+                          self.stats["steps"], self.stats["rejected"], self.stats["rhs"], 0,
+                          self.status, int(self.interpolate), int(self._out[0] == "interp"), 0,
+                          self._barrier_base.value, 0, self.counter.data_ptr() + 4,
+                          self._host.data_ptr())
+        rc = getattr(_lib.load(), name)(C.byref(gen), C.byref(rk), C.byref(c), *args, stream_ptr())
+        _lib.LAUNCHES[0] += c.launches
+        if c.swaps:
+            self._swap()
+        self.t, self.t_prev, self.t_front = c.t, c.t_prev, c.t_front
+        self.dt_safe, self.dt_int, self.status = c.dt_safe, c.dt_int, c.status
+        self.stats.update(steps=c.steps, rejected=c.rejected, rhs=c.rhs)
+        self._barrier_base.value = c.barrier_base
+        if rc != _lib.QG_OK and c.status == _lib.QG_DEVICE_WAIT:
+            self.counter.zero_()
+            self._barrier_base.value = 0
+            raise IntegratorError(_lib.load().qg_last_error().decode())
+        _lib.check(rc, name)
+        if c.status >= 0:
+            if c.interp:
+                self._set_interp(self.t)
+            else:
+                self._out = ("front", None)
+
+    def run_dm(self, tlist, ops, d: int, out: torch.Tensor) -> bool:
+        """Integrate to each of ``tlist`` and record ``ops``' expectation values, one row of
+        ``out`` per time, up to the first failure; False when the loops here must do it."""
+        gen = self._generator()
+        if gen is None or not self._set:
+            return False
+        tl = np.ascontiguousarray(tlist, dtype=np.float64)
+        self._drive("qg_vern7_run_dm", gen, tl.ctypes.data, len(tl), C.byref(ops.struct), d,
+                    out.data_ptr())
+        return True
 
     def _step_in_err(self, t, max_step):
         # explicit_rk.pyx:333-356
