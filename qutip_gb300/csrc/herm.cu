@@ -24,6 +24,7 @@
 
 #include "capi_internal.h"
 #include "common.cuh"
+#include "herm.cuh"
 #include "rows.cuh"
 #include "stage.cuh"
 
@@ -123,11 +124,6 @@ template <int DT>
 struct HermBounds {
   static constexpr int MIN_BLOCKS = DT == QG_C64 ? 5 : 4;
 };
-// Row stride of the shared-memory tiles: 16-byte elements 33, 8-byte elements 34, so that
-// the transposed reads meet no bank twice.
-template <typename T>
-constexpr int HERM_PAD = sizeof(T) == 16 ? 33 : 34;
-
 template <int DT, int YDT, int CB, bool RI>
 __global__ void __launch_bounds__(HERM_BLOCK, HermBounds<DT>::MIN_BLOCKS)
     vern7_herm_kernel(qg_csr_groups A, int d, double t, const typename elem<DT>::T* __restrict__ x,
@@ -136,7 +132,6 @@ __global__ void __launch_bounds__(HERM_BLOCK, HermBounds<DT>::MIN_BLOCKS)
   using YT = typename elem<YDT>::T;
   using CT = typename elem<DT>::R;
   using C4 = typename Codes4<CB>::T;
-  constexpr bool MIXED = DT != YDT;
   extern __shared__ __align__(16) unsigned char dict_smem[];
   __shared__ cx<CT> coef[QG_MAX_GROUPS];
   __shared__ int ccls[QG_MAX_GROUPS];
@@ -167,7 +162,7 @@ __global__ void __launch_bounds__(HERM_BLOCK, HermBounds<DT>::MIN_BLOCKS)
   const int units = 2 * nt * (nt + 1);  // four per 32 x 32 block on or below the diagonal
   const int last_col = d * d - 1;
   const int s = rk.stage;
-  const bool last = s == RK_STEP - 1, forms = !last && s != RK_EXTRA_STEP - 1;
+  const bool last = herm_last(rk), forms = herm_forms(rk);
   const size_t n64 = (size_t)rk.n;
   ST* kbuf = static_cast<ST*>(rk.k);
   const unsigned char* __restrict__ codes = reinterpret_cast<const unsigned char*>(A.col);
@@ -226,34 +221,15 @@ __global__ void __launch_bounds__(HERM_BLOCK, HermBounds<DT>::MIN_BLOCKS)
       if (direct) acc = cx<CT>{ar, ai};
       else coef_mac(acc, coef[g], ar, ai);
     }
-    // the fused epilogue (stage.cuh), its values also conjugated into the tiles
-    ST kv;
-    st_cx(&kv, acc);
-    kbuf[(size_t)s * n64 + row] = kv;
+    const HermValues<DT, YDT> o = herm_epilogue<DT, YDT>(row, acc, rk);
     const int at = w8 * PAD + lane;
     const int mc = threadIdx.x & (HERM_COLS - 1), mr = threadIdx.x / HERM_COLS;
     const size_t mrow = (size_t)(c0 + mc) + (size_t)(ti * 32 + mr) * d;
     if (!last) {
       ST* tk = tiles + buf * 2 * TILE;
       ST* tv = tk + TILE;
-      if (forms) {
-        cx<CT> v;
-        if constexpr (MIXED) v = ld_cx<CT>(static_cast<const ST*>(rk.y_prev_s) + row);
-        else v = ld_cx<CT>(static_cast<const YT*>(rk.y_prev) + row);
-#pragma unroll
-        for (int j = 0; j < RK_EXTRA_STEP - 1; ++j) {
-          if (j > s) break;
-          if ((rk.nz_a >> j) & 1u)
-            cx_axpy(v, fa<CT>(rk, j), j == s ? acc : ld_cx<CT>(kbuf + (size_t)j * n64 + row));
-        }
-        ST vv;
-        st_cx(&vv, v);
-        static_cast<ST*>(rk.ytmp_out)[row] = vv;
-        vv.y = -vv.y;
-        tv[at] = vv;
-      }
-      kv.y = -kv.y;
-      tk[at] = kv;
+      tk[at] = ST{o.k.x, -o.k.y};
+      if (forms) tv[at] = ST{o.v.x, -o.v.y};
       __syncthreads();
       if (mirrored) {
         kbuf[(size_t)s * n64 + mrow] = tk[mc * PAD + mr];
@@ -262,56 +238,13 @@ __global__ void __launch_bounds__(HERM_BLOCK, HermBounds<DT>::MIN_BLOCKS)
     } else {
       ST* tk = tiles;
       YT* ty = reinterpret_cast<YT*>(tiles + TILE);
-      YT yv;
-      double term;
-      if constexpr (MIXED) {
-        cx<CT> inc{0, 0};
-        float erh = 0.f, erl = 0.f, eih = 0.f, eil = 0.f;
-#pragma unroll
-        for (int j = 0; j < RK_STEP; ++j) {
-          const bool ub = (rk.nz_a >> j) & 1u, uq = (rk.nz_e >> j) & 1u;
-          if (!ub && !uq) continue;
-          const cx<CT> kj = (j == s) ? acc : ld_cx<CT>(kbuf + (size_t)j * n64 + row);
-          if (ub) cx_axpy(inc, fa<CT>(rk, j), kj);
-          if (uq) {  // the error estimate in float-float
-            ff_acc(erh, erl, fe<CT>(rk, j), rk.fe_l[j], (float)kj.re);
-            ff_acc(eih, eil, fe<CT>(rk, j), rk.fe_l[j], (float)kj.im);
-          }
-        }
-        const double2 yp = static_cast<const double2*>(rk.y_prev)[row];
-        yv = make_double2(yp.x + (double)inc.re, yp.y + (double)inc.im);
-        static_cast<float2*>(rk.y_front_s)[row] = make_float2((float)yv.x, (float)yv.y);
-        const double er = (double)erh + (double)erl, ei = (double)eih + (double)eil;
-        term = wrms_term(er * er + ei * ei, yv.x * yv.x + yv.y * yv.y, rk.atol, rk.rtol);
-      } else {
-        cx<CT> y = ld_cx<CT>(static_cast<const YT*>(rk.y_prev) + row), e{0, 0};
-#pragma unroll
-        for (int j = 0; j < RK_STEP; ++j) {
-          const bool ub = (rk.nz_a >> j) & 1u, uq = (rk.nz_e >> j) & 1u;
-          if (!ub && !uq) continue;
-          const cx<CT> kj = (j == s) ? acc : ld_cx<CT>(kbuf + (size_t)j * n64 + row);
-          if (ub) cx_axpy(y, fa<CT>(rk, j), kj);
-          if (uq) cx_axpy(e, fe<CT>(rk, j), kj);
-        }
-        st_cx(&yv, y);
-        const cx<CT> ys = ld_cx<CT>(&yv);
-        const double mag2 = (double)ys.re * ys.re + (double)ys.im * ys.im;
-        const double sc = rk.atol + rk.rtol * sqrt(mag2);
-        term = ((double)e.re * e.re + (double)e.im * e.im) / (sc * sc);
-      }
-      static_cast<YT*>(rk.y_front)[row] = yv;
-      err_acc += mirrored ? 2.0 * term : term;  // the mirrored element has the same term
-      kv.y = -kv.y;
-      yv.y = -yv.y;
-      tk[at] = kv;
-      ty[w8 * YPAD + lane] = yv;
+      err_acc += mirrored ? 2.0 * o.term : o.term;  // the mirrored element has the same term
+      tk[at] = ST{o.k.x, -o.k.y};
+      ty[w8 * YPAD + lane] = YT{o.y.x, -o.y.y};
       __syncthreads();
       if (mirrored) {
         kbuf[(size_t)s * n64 + mrow] = tk[mc * PAD + mr];
-        const YT y = ty[mc * YPAD + mr];
-        static_cast<YT*>(rk.y_front)[mrow] = y;
-        if constexpr (MIXED)
-          static_cast<float2*>(rk.y_front_s)[mrow] = make_float2((float)y.x, (float)y.y);
+        herm_mirror_front<DT, YDT>(mrow, ty[mc * YPAD + mr], rk);
       }
       __syncthreads();  // one set of tiles: read before the next unit writes them
     }

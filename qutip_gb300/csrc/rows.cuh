@@ -22,6 +22,26 @@ __device__ __forceinline__ void cmac_any(float& ar, float& ai, float2 v, float2 
   ai = fmaf(v.y, x.x, ai);
 }
 
+// acc += conj(v) * x
+__device__ __forceinline__ void cmac_conj(double& ar, double& ai, double2 v, double2 x) {
+  ar = fma(v.x, x.x, ar);
+  ar = fma(v.y, x.y, ar);
+  ai = fma(v.x, x.y, ai);
+  ai = fma(-v.y, x.x, ai);
+}
+__device__ __forceinline__ void cmac_conj(float& ar, float& ai, float2 v, float2 x) {
+  ar = fmaf(v.x, x.x, ar);
+  ar = fmaf(v.y, x.y, ar);
+  ai = fmaf(v.x, x.y, ai);
+  ai = fmaf(-v.y, x.x, ai);
+}
+
+__device__ __forceinline__ cplx prog_coef(const int* code, const int* start, const double* consts,
+                                          int g, double t) {
+  if (code == nullptr) return cplx{1.0, 0.0};
+  return eval_coef(code + start[g], consts, t);
+}
+
 template <int LANES, typename R>
 __device__ __forceinline__ cx<R> sub_reduce(R ar, R ai) {
 #pragma unroll

@@ -24,6 +24,7 @@
 
 #include "capi_internal.h"
 #include "common.cuh"
+#include "lindblad_herm.cuh"
 #include "rows.cuh"
 #include "stage.cuh"
 
@@ -426,32 +427,11 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, 4>::MIN_BLOCKS)
 // rho.  The d x d operators stay in L1/L2 and the state (d^2 entries) in L2: the HBM
 // traffic of a stage is its vectors only.  Diagonal parts (the diagonal of A and the
 // all-diagonal collapse operators, e.g. dephasing) fold into one factor on x[r + c d].
-// With L.hermitian (rho Hermitian, the reference's A + A^dag branch) only the elements
-// r >= c are evaluated; each also goes through the epilogue at its mirror c + r d as its
-// conjugate, and the diagonal is taken real.
+// With L.hermitian (rho Hermitian, the reference's A + A^dag branch) the kernel of
+// lindblad_herm.cu evaluates the elements r >= c only.
 constexpr int LB_BLOCK = 256;
 
-// acc += conj(v) * x
-__device__ __forceinline__ void cmac_conj(double& ar, double& ai, double2 v, double2 x) {
-  ar = fma(v.x, x.x, ar);
-  ar = fma(v.y, x.y, ar);
-  ai = fma(v.x, x.y, ai);
-  ai = fma(-v.y, x.x, ai);
-}
-__device__ __forceinline__ void cmac_conj(float& ar, float& ai, float2 v, float2 x) {
-  ar = fmaf(v.x, x.x, ar);
-  ar = fmaf(v.y, x.y, ar);
-  ai = fmaf(v.x, x.y, ai);
-  ai = fmaf(-v.y, x.x, ai);
-}
-
-__device__ __forceinline__ cplx prog_coef(const int* code, const int* start, const double* consts,
-                                          int g, double t) {
-  if (code == nullptr) return cplx{1.0, 0.0};
-  return eval_coef(code + start[g], consts, t);
-}
-
-template <int DT, int YDT, int EPI, bool HERM>
+template <int DT, int YDT, int EPI>
 __global__ void __launch_bounds__(LB_BLOCK)
     lindblad_kernel(qg_lindblad L, double t, const typename elem<DT>::T* __restrict__ x,
                     AxpbyArgs ax, RkArgs rk) {
@@ -577,62 +557,19 @@ __global__ void __launch_bounds__(LB_BLOCK)
     }
     return acc;
   };
-  if constexpr (!HERM) {
-    // (r, c) of idx, advanced by the grid stride without a division per element
-    const int stride = gridDim.x * LB_BLOCK;
-    const int sc = stride / d, sr = stride - (stride / d) * d;
-    int idx = blockIdx.x * LB_BLOCK + threadIdx.x;
-    int c = idx / d;
-    int r = idx - c * d;
-    for (; idx < n; idx += stride) {
-      epilogue<DT, YDT, EPI>(idx, element(r, c), ax, rk, err_acc);
-      c += sc;
-      r += sr;
-      if (r >= d) {
-        r -= d;
-        ++c;
-      }
-    }
-  } else {
-    // Hermitian rho: 32 x 32 tiles on or below the diagonal; warp w evaluates 32
-    // consecutive r of the columns w, w + 8, w + 16, w + 24 (elements r >= c), then the
-    // block writes the conjugates to the mirrors (c, r) through shared memory, a warp
-    // covering 32 consecutive c of one row r.
-    __shared__ cx<R> tile[32][33];  // [c - c0][r - r0]
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    // only the n_t (n_t + 1) / 2 tiles on or below the diagonal are enumerated, column
-    // block j holding row blocks j .. n_t - 1, so the blocks share the work evenly
-    const int n_t = (d + 31) / 32;
-    const int n_tiles = n_t * (n_t + 1) / 2;
-    int tj = 0, tbase = 0;  // column block of tau and the index of its first tile
-    for (int tau = blockIdx.x; tau < n_tiles; tau += gridDim.x) {
-      while (tau >= tbase + (n_t - tj)) {
-        tbase += n_t - tj;
-        ++tj;
-      }
-      const int r0 = (tj + (tau - tbase)) * 32, c0 = tj * 32;
-#pragma unroll 1
-      for (int q = 0; q < 4; ++q) {
-        const int cl = w + 8 * q, r = r0 + lane, c = c0 + cl;
-        cx<R> acc{0, 0};
-        if (r < d && c < d && r >= c) {
-          acc = element(r, c);
-          if (r == c) acc.im = 0;  // A + A^dag: real diagonal
-          epilogue<DT, YDT, EPI>(r + c * d, acc, ax, rk, err_acc);
-        }
-        tile[cl][lane] = acc;
-      }
-      __syncthreads();
-#pragma unroll 1
-      for (int q = 0; q < 4; ++q) {
-        const int rl = w + 8 * q;
-        const int mr = r0 + rl, mc = c0 + lane;  // the mirror of (mr, mc)
-        if (mr < d && mc < d && mr > mc) {
-          const cx<R> v = tile[lane][rl];
-          epilogue<DT, YDT, EPI>(mc + mr * d, cx<R>{v.re, -v.im}, ax, rk, err_acc);
-        }
-      }
-      __syncthreads();
+  // (r, c) of idx, advanced by the grid stride without a division per element
+  const int stride = gridDim.x * LB_BLOCK;
+  const int sc = stride / d, sr = stride - (stride / d) * d;
+  int idx = blockIdx.x * LB_BLOCK + threadIdx.x;
+  int c = idx / d;
+  int r = idx - c * d;
+  for (; idx < n; idx += stride) {
+    epilogue<DT, YDT, EPI>(idx, element(r, c), ax, rk, err_acc);
+    c += sc;
+    r += sr;
+    if (r >= d) {
+      r -= d;
+      ++c;
     }
   }
   if constexpr (EPI == EPI_RK) {
@@ -768,31 +705,22 @@ static int launch_any(cudaStream_t st, const qg_csr_groups& A, double t, const v
   return check_launch("spmv_direct_kernel");
 }
 
-// The full form and the Hermitian branch are separate instantiations: sharing one kernel
-// body, the full form's code generation degraded (dense d = 128 operators: 3x slower).
-template <int DT, int YDT, int EPI, bool HERM>
-static int launch_lindblad_form(cudaStream_t st, const qg_lindblad& L, double t, const void* x,
-                                const AxpbyArgs& ax, const RkArgs& rk) {
+template <int DT, int YDT, int EPI>
+static int launch_lindblad(cudaStream_t st, const qg_lindblad& L, double t, const void* x,
+                           const AxpbyArgs& ax, const RkArgs& rk) {
   using ST = typename elem<DT>::T;
-  auto kern = lindblad_kernel<DT, YDT, EPI, HERM>;
+  if (L.hermitian) return launch_lindblad_herm<DT, YDT, EPI>(st, L, t, x, ax, rk);
+  auto kern = lindblad_kernel<DT, YDT, EPI>;
   static OccCache cache;  // one per instantiation
   const int per_sm = staged_occupancy(kern, LB_BLOCK, 0, cache);
   if (per_sm <= 0) return set_error(QG_ERR_CUDA, "occupancy query failed");
   const int64_t n = L.d * L.d;
-  const int64_t n_t = (L.d + 31) / 32;
-  const int64_t blocks = HERM ? n_t * (n_t + 1) / 2 : (n + LB_BLOCK - 1) / LB_BLOCK;
+  const int64_t blocks = (n + LB_BLOCK - 1) / LB_BLOCK;
   int64_t cap = (int64_t)sm_count() * per_sm;
   if (cap > qg_scratch_doubles()) cap = qg_scratch_doubles();
   const int grid = (int)(blocks < 1 ? 1 : (blocks < cap ? blocks : cap));
   kern<<<grid, LB_BLOCK, 0, st>>>(L, t, (const ST*)x, ax, rk);
   return check_launch("lindblad_kernel");
-}
-
-template <int DT, int YDT, int EPI>
-static int launch_lindblad(cudaStream_t st, const qg_lindblad& L, double t, const void* x,
-                           const AxpbyArgs& ax, const RkArgs& rk) {
-  return L.hermitian ? launch_lindblad_form<DT, YDT, EPI, true>(st, L, t, x, ax, rk)
-                     : launch_lindblad_form<DT, YDT, EPI, false>(st, L, t, x, ax, rk);
 }
 
 int check_groups(const qg_csr_groups* A) {

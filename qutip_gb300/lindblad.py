@@ -227,14 +227,15 @@ class LindbladOperator:
 
     def hermitian_pays(self) -> bool:
         """Whether the Hermitian branch is the faster form for this size.  It halves the
-        generator's arithmetic and writes the mirrored half through 32 x 32 shared-memory
-        tiles, one CTA per tile on or below the diagonal: measured on the Ising chain
-        (mixed form), 58 -> 43 us per stage at L = 10 (528 tiles) and 4.8 -> 2.6 ms at
-        L = 13.  With fewer tiles than two per SM the GPU idles (dense random d = 128,
-        10 tiles: 534 -> 2133 ms per solve), so the full form stays there."""
+        generator's arithmetic, but its units (32 rows x 16 columns) leave the GPU idle at
+        small dimensions.  Measured per stage, full form against this one: complex64 L = 10
+        Ising (528 blocks of 32 x 32 on or below the diagonal) 51 and 31 us, L = 9 (136) 19
+        and 23, d = 512 Bose-Hubbard 13 and 17; complex128, bound by FP64, L = 9 105 and 80,
+        d = 512 70 and 47, d = 343 (66 blocks) 39 and 33, d = 216 (28) 23 and 31.  So it is
+        taken from two blocks per SM in complex64, two for five SMs in complex128."""
         n_t = (self.d + 31) // 32
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
-        return n_t * (n_t + 1) // 2 >= 2 * sms
+        return n_t * (n_t + 1) // 2 >= (2 * sms if self.dtype == "c64" else 0.4 * sms)
 
     @property
     def n_groups(self) -> int:
