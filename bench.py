@@ -843,12 +843,12 @@ def run_sde(args):
 
 
 def run_dense(args):
-    """The dense small-dimension bucket (tensor-core Lindblad generator, mixed form) against
+    """The dense small-dimension bucket (dense Lindblad generator, mixed form) against
     the sparse paths, one request at a time: Jaynes-Cummings mesolve (N = 5..60, d = 2N,
     tlist linspace(0, 20, 101)) and dense random systems (d = 32, 64, 128, t in [0, 2]).
     Sparse paths: the matrix-free kernel (one system, whole GPU) and the batched kernel's
     sparse row loop (the served path, one request in one launch).  Also the generator
-    application alone, with the tensor-core rate of the MMAs it issues."""
+    application alone, with the FP32 rate of the multiply-adds it issues."""
     import scipy.sparse as sp
     import torch
     from qutip_gb300 import systems as S
@@ -872,7 +872,7 @@ def run_dense(args):
 
     peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json"))) \
         if os.path.exists(os.path.join(ROOT, "MEASURED_PEAKS.json")) else {}
-    tf32_peak = 0.5 * float(peaks.get("bf16_tflops", 1900.0))
+    fp32_sm = 2 * 128 * 1e6 * float(peaks.get("sm_max_mhz", 2070.0)) / 1e12
     out = {"jc": [], "dense_random": []}
     tl = np.linspace(0.0, 20.0, 101)
     for N in (5, 10, 20, 30, 45, 60):
@@ -892,7 +892,7 @@ def run_dense(args):
         ms_b = timed(batched)
         out["jc"].append({"N": N, "d": 2 * N, "dense_bucket_ms": ms_dense,
                           "matrix_free_sparse_ms": ms_mf, "batched_sparse_row_loop_ms": ms_b})
-        log(f"dense: JC N={N}: tensor cores {ms_dense:.1f} ms, matrix-free {ms_mf:.1f} ms, "
+        log(f"dense: JC N={N}: dense kernel {ms_dense:.1f} ms, matrix-free {ms_mf:.1f} ms, "
             f"batched row loop {ms_b:.1f} ms")
     rng = np.random.default_rng(11)
     for d in (32, 64, 128):
@@ -928,12 +928,12 @@ def run_dense(args):
         tflops = dop.gemm_flops() / (us * 1e-6) / 1e12
         n_sm = dop.n_ctas
         out["dense_random"].append({"d": d, "dense_bucket_ms": ms_dense, "matrix_free_sparse_ms": ms_mf,
-                                    "apply_us": us, "issued_tf32_tflops": tflops, "sms": n_sm,
-                                    "frac_of_sms_tf32": tflops / (tf32_peak * n_sm / 152.0)})
-        log(f"dense: random d={d}: tensor cores {ms_dense:.1f} ms, matrix-free {ms_mf:.1f} ms, "
-            f"apply {us:.1f} us = {tflops:.2f} TFLOP/s issued TF32 on {n_sm} SMs")
-    out["note"] = ("one CTA (one SM) per 16 output columns per application; TF32 rate per SM "
-                   "taken as half the measured bf16 GEMM rate / 152 SMs")
+                                    "apply_us": us, "issued_tflops": tflops, "sms": n_sm,
+                                    "frac_of_sms_fp32": tflops / (fp32_sm * min(n_sm, 152))})
+        log(f"dense: random d={d}: dense kernel {ms_dense:.1f} ms, matrix-free {ms_mf:.1f} ms, "
+            f"apply {us:.1f} us = {tflops:.2f} TFLOP/s on {n_sm} CTAs")
+    out["note"] = ("a CTA per 16 x 8 tile of the result per application; FP32 rate per SM taken as "
+                   "128 multiply-adds per clock at the maximum SM clock")
     return out
 
 
@@ -1245,7 +1245,7 @@ def run_profile_matrix(args):
 
 
 def run_profile_dense(args):
-    """ncu case for the dense tensor-core Lindblad kernel: a dense random system of
+    """ncu case for the dense Lindblad kernel: a dense random system of
     dimension ``--profile-sites`` (default 10 is raised to 128 here: d = 128), ten
     applications of the generator."""
     import scipy.sparse as sp

@@ -186,11 +186,10 @@ typedef struct qg_lindblad {
 
 /* Dense small-dimension bucket (d <= QG_DENSE_MAX_D): the Lindblad generator with
  * dense operators, L(t)[X] = A X + X A^dag + sum_i |f_i(t)|^2 C_i X C_i^dag with
- * A = sum_g a_g(t) A_g = -i H_nh, applied as GEMMs on the tensor cores (TF32 split into
- * hi + lo parts, FP32 accumulation).  Operators are complex64, row-major:
+ * A = sum_g a_g(t) A_g = -i H_nh, applied as FP32 GEMMs.  Operators are complex64, row-major:
  * A_g[m][k] at a + (g*d + m)*d + k, C_i[m][k] at c + (i*d + m)*d + k.  Coefficient
- * programs as in qg_lindblad (NULL code: all 1).  One CTA per 16 columns of the
- * result; no workspace. */
+ * programs as in qg_lindblad (NULL code: all 1).  A cluster of CTAs (16
+ * rows each) per 8 columns of the result; no workspace. */
 #define QG_DENSE_MAX_D 128
 typedef struct qg_dense_lindblad {
   int32_t d;
@@ -362,8 +361,7 @@ int qg_lindblad_stage(const qg_lindblad* L, const qg_rk_buffers* B, int stage, d
 
 /* y = alpha * L(t)[x] + beta * y for the dense generator; x, y complex64 vec(rho) of
  * length d*d.  Replaces LindbladMatrixForm.matmul_data
- * (qutip/core/cy/lindblad_matrix_form.pyx:105-204, full branch) for small dense systems;
- * one CTA per application, tcgen05 tensor-core GEMMs. */
+ * (qutip/core/cy/lindblad_matrix_form.pyx:105-204, full branch) for small dense systems. */
 int qg_dense_lindblad_apply(const qg_dense_lindblad* L, double t, const void* x, void* y,
                             double alpha_re, double alpha_im, double beta_re, double beta_im,
                             void* stream);

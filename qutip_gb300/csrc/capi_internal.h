@@ -15,7 +15,6 @@ int sm_count();
 int check_groups(const qg_csr_groups* A);
 }  // namespace qg
 
-// The dense kernel's fault flag, read and cleared (for qg_device_fault).
-int dense_fault_take();
-// The same for the fused step kernel's barrier waits.
+// The fault flag of the fused step kernel's barrier waits, read and cleared (for
+// qg_device_fault).
 int step_fault_take();

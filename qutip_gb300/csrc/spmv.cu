@@ -810,7 +810,7 @@ extern "C" int qg_device_fault(void) {
   if (cudaMemcpyFromSymbol(&v, g_fault, sizeof(v)) != cudaSuccess)
     return set_error(QG_ERR_CUDA, "cannot read the device fault flag");
   if (v) cudaMemcpyToSymbol(g_fault, &zero, sizeof(zero));
-  return (int)(v | (unsigned)dense_fault_take() | (unsigned)step_fault_take());
+  return (int)(v | (unsigned)step_fault_take());
 }
 
 extern "C" int qg_spmv_csr(const qg_csr_groups* A, double t, const void* x, void* y,

@@ -1,16 +1,17 @@
 """Dense small-dimension bucket: the Lindblad generator of a small system with dense
-operators, applied as GEMMs on the tensor cores.
+operators, applied as FP32 GEMMs over the whole GPU.
 
 The reference's matrix form (``LindbladMatrixForm``,
 qutip/core/cy/lindblad_matrix_form.pyx:105-204) applies ``A rho + rho A^dag +
 sum_i C_i rho C_i^dag`` with ``A = -i H_nh`` through sparse or dense matmuls.  For a
 system of Hilbert dimension ``d <= 128`` whose operators are dense, those products are
 small dense GEMMs: :class:`DenseLindbladOperator` keeps ``A_g`` and ``C_i`` as complex64
-``d x d`` matrices and applies the generator with ``tcgen05`` tensor-core MMAs (TF32
-inputs split hi + lo, FP32 accumulation in tensor memory; ``qg_dense_lindblad_*`` in
-``csrc/dense.cu``; a cluster of CTAs per 16 output columns, one CTA per term; each K chunk
-of 32 in fresh accumulators, the large hi*hi part and the small hi*lo + lo*hi corrections
-apart, summed on the CUDA cores with round-to-nearest).  The stages are complex64, so it serves the mixed form
+``d x d`` matrices and applies the generator in one launch (``qg_dense_lindblad_*`` in
+``csrc/dense.cu``): a cluster of CTAs per 8 output columns, one CTA per 16 rows, with FP32
+multiply-adds.  The products are too small for the tensor cores: 1.3 us of the GPU's FP32
+units at d = 128, while splitting and staging TF32 operands took longer and lost accuracy
+to an accumulation that does not round to nearest.  The stages are complex64,
+so it serves the mixed form
 (``precision="mixed"``: FP64 state, step control and expectation values).
 
 Sparse operators (a Jaynes-Cummings system has three entries per row) keep the sparse
@@ -135,8 +136,8 @@ class DenseLindbladOperator:
         return ("dense", 0, 1)
 
     def launch_desc(self) -> str:
-        return (f"dense tensor-core Lindblad (d={self.d}, {self.n_groups} A groups, "
-                f"{self.n_cops} collapse operators, tcgen05 TF32x3)")
+        return (f"dense Lindblad (d={self.d}, {self.n_groups} A groups, "
+                f"{self.n_cops} collapse operators, FP32 tiles of 16 x 8)")
 
     def tune(self, *args, **kwargs):
         return self.launch
@@ -150,20 +151,15 @@ class DenseLindbladOperator:
 
     @property
     def n_ctas(self) -> int:
-        """CTAs (one per SM) of one application: a cluster per 16 output columns, of one CTA
-        for A X + X A^dag and one per collapse operator (two without any, eight at most)."""
-        ranks = 2 if self.n_cops == 0 else min(self.n_cops + 1, 8)
-        return ranks * ((self.d + 15) // 16)
+        """CTAs of one application: a cluster per 8 output columns, a CTA per 16 rows."""
+        return ((self.d + 15) // 16) * ((self.d + 7) // 8)
 
     def gemm_flops(self) -> int:
-        """Real multiply-adds x 2 of one application as issued: per complex product of two
-        d x d matrices (padded to 128 rows, 16-column blocks, 8-wide K steps) four real
-        products in three TF32 terms."""
+        """Real multiply-adds x 2 of one application as issued: a complex product of two d x d
+        matrices (K padded to 16, rows to 16, columns to 8) is four real ones."""
         d = self.d
-        np_ = (d + 15) // 16 * 16
-        k = (d + 7) // 8 * 8
-        products = 2 + 2 * self.n_cops
-        return 2 * 128 * np_ * k * 12 * products
+        k = (d + 15) // 16 * 16
+        return 8 * k * k * ((d + 7) // 8 * 8) * (2 + 2 * self.n_cops)
 
     def matvec(self, t: float, x: torch.Tensor, y: torch.Tensor, alpha=1.0, beta=0.0):
         """``y = alpha * L(t)[x] + beta * y`` (complex64 vec(rho))."""

@@ -705,7 +705,7 @@ def lindblad_operator(rhs, dtype="c128", dense="auto"):
     (lindblad_matrix_form.pyx:88-96) and one term per collapse operator.
 
     The dense small-dimension bucket (:class:`~qutip_gb300.dense.DenseLindbladOperator`,
-    tensor-core GEMMs) takes the mixed form (complex64 stages) of a system with
+    dense FP32 GEMMs) takes the mixed form (complex64 stages) of a system with
     ``d <= 128`` whose operators are at least ``DENSE_FILL`` filled, or whenever
     ``dense=True``; sparse systems keep the matrix-free sparse kernel."""
     from .dense import DENSE_FILL, DenseLindbladOperator, dense_fill
@@ -889,7 +889,7 @@ class IntegratorGpuVern7(Integrator):
         """atol, rtol, nsteps, first_step, max_step, min_step, interpolate: as the
         reference ``vern7``; precision: ``"double"`` or ``"mixed"``; dense (matrix form
         only): ``"auto"`` sends small systems with dense operators in the mixed form to
-        the tensor-core bucket, ``True`` forces it, ``False`` keeps the sparse kernel;
+        the dense bucket, ``True`` forces it, ``False`` keeps the sparse kernel;
         hermitian_branch (matrix form only): with a Hermitian rho0, ``"auto"`` evaluates
         half the elements where that is faster (at least two 32 x 32 tiles per SM),
         ``True`` always, ``False``
