@@ -49,6 +49,7 @@ def generate_tableau() -> Path:
     lo = lambda v: [f32(x - f32(x)) for x in v]  # noqa: E731
     fa1 = lambda v: "{" + ", ".join(float(x).hex() + "f" if x else "0.0f" for x in v) + "}"  # noqa: E731
     fa2 = lambda m: "{" + ", ".join(fa1(r) for r in m) + "}"  # noqa: E731
+    bits = lambda v: hex(sum(1 << j for j, x in enumerate(v) if x)) + "u"  # noqa: E731
     src = f"""// Generated from qutip_gb300/vern7_tableau.py by qutip_gb300/build.py.  Do not edit.
 #pragma once
 namespace qg {{
@@ -67,6 +68,10 @@ static __constant__ float VERN7_BH[10] = {fa1(hi(T.B))};
 static __constant__ float VERN7_BL[10] = {fa1(lo(T.B))};
 static __constant__ float VERN7_EF[10] = {fa1(hi(T.E))};
 static __constant__ float VERN7_EL[10] = {fa1(lo(T.E))};
+// bit j set where the j-th coefficient of the row is nonzero
+constexpr unsigned VERN7_NZ_A[16] = {{{", ".join(bits(r) for r in a)}}};
+constexpr unsigned VERN7_NZ_B = {bits(T.B)};
+constexpr unsigned VERN7_NZ_E = {bits(T.E)};
 static const double VERN7_A_HOST[16][16] = {arr2(a)};
 static const double VERN7_B_HOST[10] = {arr1(T.B)};
 static const double VERN7_C_HOST[16] = {arr1(T.C)};

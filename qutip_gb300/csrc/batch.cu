@@ -165,28 +165,48 @@ struct WarpGroup {
     return make_double2(a, b);
   }
   __device__ __forceinline__ int bcast(int v) const { return __shfl_sync(0xffffffffu, v, 0); }
+  // f(sum(v)), a pair
+  template <class F>
+  __device__ __forceinline__ double2 sum_map(double v, F f) const {
+    return f(sum(v));
+  }
+  // whether this warp forms the values its block shares, and their block-wide order
+  __device__ __forceinline__ bool forms_shared() const { return true; }
+  __device__ __forceinline__ void block_sync() const { __syncwarp(); }
 };
+
+// Warp sums of 16 values at once, each in the order of the XOR butterfly: at every level a lane
+// keeps half of its values and adds the partner's, so a level of the butterfly costs half of
+// the last one's adds (16 in all, where 16 butterflies take 80; an FP64 add occupies its SM for
+// 16 clocks).  Value i ends in the lanes 2 i and 2 i + 1.
+__device__ __forceinline__ double warp_sums16(double (&v)[16]) {
+  const unsigned lane = threadIdx.x & 31u;
+#pragma unroll
+  for (int h = 8; h > 0; h >>= 1) {
+    const bool up = lane & (2u * h);
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const double keep = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * h);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
 
 template <int BB>
 struct CtaGroup {
   static constexpr int SIZE = BB;
-  static constexpr bool DEFER = true;  // record sums: put2 / sync / take2
+  static constexpr bool DEFER = true;  // record sums: put_all / sync / take2
   int rank;
   int64_t slot;
   double* red;  // shared [2 * BB/32]
   int* ibuf;    // shared [1]
   double* rec;  // shared [REC_SLOTS * 2 * BB/32]: warp partials of deferred sums
-  // warp partial of deferred sum pair k; the totals are read by take2 after a sync()
-  __device__ __forceinline__ void put2(int k, double a, double b) const {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_xor_sync(0xffffffffu, a, o);
-      b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
-    if ((rank & 31) == 0) {
-      rec[(2 * k) * (BB / 32) + (rank >> 5)] = a;
-      rec[(2 * k + 1) * (BB / 32) + (rank >> 5)] = b;
-    }
+  // warp partials of REC_SLOTS deferred sum pairs (value 2 k, 2 k + 1 for pair k); the totals
+  // are read by take2 after a sync()
+  __device__ __forceinline__ void put_all(double (&v)[2 * REC_SLOTS]) const {
+    const double t = warp_sums16(v);
+    if ((rank & 1) == 0) rec[((rank & 31) >> 1) * (BB / 32) + (rank >> 5)] = t;
   }
   // sum pair k, each component in the order of sum()
   __device__ __forceinline__ double2 take2(int k) const {
@@ -203,38 +223,35 @@ struct CtaGroup {
   }
   __device__ __forceinline__ int take_flag() const { return *ibuf; }
   __device__ __forceinline__ void sync() const { __syncthreads(); }
-  __device__ __forceinline__ double sum(double v) const {
+  // f(sum), a pair: the warp partials are added, in order, and f evaluated by warp 0 alone,
+  // which shares the result (every warp adding them for itself and taking the square root,
+  // division and power of the step control kept the FP64 pipe busy eight times over).  A
+  // total is read by everyone before the next sum's first barrier, after which it is
+  // overwritten; the partials are read before the second barrier.
+  template <class F>
+  __device__ __forceinline__ double2 sum_map(double v, F f) const {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();  // earlier readers of red are done
     if ((rank & 31) == 0) red[rank >> 5] = v;
     __syncthreads();
-    double t = 0.0;
+    if (rank < 32) {
+      double t = 0.0;
 #pragma unroll
-    for (int i = 0; i < BB / 32; ++i) t += red[i];
-    return t;
-  }
-  // two sums behind one pair of barriers, each component in the order of sum()
-  __device__ __forceinline__ double2 sum2(double a, double b) const {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_xor_sync(0xffffffffu, a, o);
-      b += __shfl_xor_sync(0xffffffffu, b, o);
+      for (int i = 0; i < BB / 32; ++i) t += red[i];
+      const double2 r = f(t);
+      if (rank == 0) {
+        red[BB / 32] = r.x;
+        red[BB / 32 + 1] = r.y;
+      }
     }
     __syncthreads();
-    if ((rank & 31) == 0) {
-      red[rank >> 5] = a;
-      red[BB / 32 + (rank >> 5)] = b;
-    }
-    __syncthreads();
-    double ta = 0.0, tb = 0.0;
-#pragma unroll
-    for (int i = 0; i < BB / 32; ++i) {
-      ta += red[i];
-      tb += red[BB / 32 + i];
-    }
-    return make_double2(ta, tb);
+    return make_double2(red[BB / 32], red[BB / 32 + 1]);
   }
+  __device__ __forceinline__ double sum(double v) const {
+    return sum_map(v, [](double t) { return make_double2(t, 0.0); }).x;
+  }
+  __device__ __forceinline__ bool forms_shared() const { return rank < 32; }
+  __device__ __forceinline__ void block_sync() const { __syncthreads(); }
   __device__ __forceinline__ int bcast(int v) const {
     __syncthreads();
     if (rank == 0) *ibuf = v;
@@ -251,22 +268,18 @@ struct CtaGroup {
 template <int BB, int CS>
 struct ClusterGroup {
   static constexpr int SIZE = BB * CS;
-  static constexpr bool DEFER = true;  // record sums: put2 / sync / take2
+  static constexpr bool DEFER = true;  // record sums: put_all / sync / take2
   int rank;
   int64_t slot;
-  double* red;  // shared [2 * BB/32] of this CTA
+  double* red;  // shared [2 * BB/32 + 2] of this CTA
   int* ibuf;    // shared [1] of this CTA
   double* rec;  // shared [REC_SLOTS * 2 * BB/32] of this CTA: warp partials
-  __device__ __forceinline__ void put2(int k, double a, double b) const {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_xor_sync(0xffffffffu, a, o);
-      b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      rec[(2 * k) * (BB / 32) + (threadIdx.x >> 5)] = a;
-      rec[(2 * k + 1) * (BB / 32) + (threadIdx.x >> 5)] = b;
-    }
+  mutable int parity;  // half of red the next sum uses
+  // as CtaGroup::put_all, into this CTA's rec
+  __device__ __forceinline__ void put_all(double (&v)[2 * REC_SLOTS]) const {
+    const double t = warp_sums16(v);
+    if ((threadIdx.x & 1) == 0)
+      rec[((threadIdx.x & 31) >> 1) * (BB / 32) + (threadIdx.x >> 5)] = t;
   }
   // every CTA's partials through distributed shared memory, in the order of sum()
   __device__ __forceinline__ double2 take2(int k) const {
@@ -289,46 +302,44 @@ struct ClusterGroup {
     return *cgrp::this_cluster().map_shared_rank(ibuf, 0);
   }
   __device__ __forceinline__ void sync() const { cgrp::this_cluster().sync(); }
-  __device__ __forceinline__ double sum(double v) const {
+  // f(sum), a pair: warp 0 of every CTA adds all CTAs' partials in rank order, evaluates f and
+  // shares it with its CTA.  Partials alternate between two halves of red, so one cluster
+  // barrier is enough: a half is written again only after the next sum's barrier, which
+  // every reader of it has passed.
+  template <class F>
+  __device__ __forceinline__ double2 sum_map(double v, F f) const {
     cgrp::cluster_group cl = cgrp::this_cluster();
+    constexpr int W = BB / 32;
+    static_assert(CS * W == 64, "two partials per lane");
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    cl.sync();  // earlier readers of every CTA's red are done
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    double* half = red + parity * W;
+    parity ^= 1;
+    if ((threadIdx.x & 31) == 0) half[threadIdx.x >> 5] = v;
     cl.sync();
-    double t = 0.0;
-    for (int c = 0; c < CS; ++c) {
-      const double* rr = cl.map_shared_rank(red, c);
-#pragma unroll
-      for (int i = 0; i < BB / 32; ++i) t += rr[i];
-    }
-    return t;
-  }
-  // two sums behind one pair of cluster barriers, each component in the order of sum()
-  __device__ __forceinline__ double2 sum2(double a, double b) const {
-    cgrp::cluster_group cl = cgrp::this_cluster();
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_xor_sync(0xffffffffu, a, o);
-      b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
-    cl.sync();
-    if ((threadIdx.x & 31) == 0) {
-      red[threadIdx.x >> 5] = a;
-      red[BB / 32 + (threadIdx.x >> 5)] = b;
-    }
-    cl.sync();
-    double ta = 0.0, tb = 0.0;
-    for (int c = 0; c < CS; ++c) {
-      const double* rr = cl.map_shared_rank(red, c);
-#pragma unroll
-      for (int i = 0; i < BB / 32; ++i) {
-        ta += rr[i];
-        tb += rr[BB / 32 + i];
+    if (threadIdx.x < 32) {
+      const int l = threadIdx.x;
+      const double a = cl.map_shared_rank(half, l / W)[l % W];
+      const double b = cl.map_shared_rank(half, 32 / W + l / W)[l % W];
+      double t = 0.0;
+#pragma unroll 8
+      for (int i = 0; i < 32; ++i) t += __shfl_sync(0xffffffffu, a, i);
+#pragma unroll 8
+      for (int i = 0; i < 32; ++i) t += __shfl_sync(0xffffffffu, b, i);
+      const double2 r = f(t);
+      if (l == 0) {
+        red[2 * W] = r.x;
+        red[2 * W + 1] = r.y;
       }
     }
-    return make_double2(ta, tb);
+    __syncthreads();
+    return make_double2(red[2 * W], red[2 * W + 1]);
   }
+  __device__ __forceinline__ double sum(double v) const {
+    return sum_map(v, [](double t) { return make_double2(t, 0.0); }).x;
+  }
+  __device__ __forceinline__ bool forms_shared() const { return threadIdx.x < 32; }
+  __device__ __forceinline__ void block_sync() const { __syncthreads(); }
   __device__ __forceinline__ int bcast(int v) const {
     cgrp::cluster_group cl = cgrp::this_cluster();
     cl.sync();
@@ -347,23 +358,47 @@ struct Ctl {
   int status, cur, interp_ready, out_front, steps, rhs;
 };
 
-// Per-warp factor slice in shared memory (WF_FLOATS floats, 512 B): the stage factors
-// (mixed: dt a_j, its low part, dt e_j, its low part as float[16] each; double:
-// dt a_j, dt e_j as double[16]) and the combination / dense-output factors bf (double[16],
-// dt-scaled) with their float pairs bfh, bfl (mixed form).  Lanes 0-15 of the warp write
-// factor j = lane between two __syncwarp(); every lane reads them as broadcasts.  Held
-// per thread, the arrays were indexed at run time and lived in local memory (1.6 KB of
-// stack per thread, ~1.1e9 local-load sectors in one 4096-trajectory launch).
-// The group coefficients at the current stage time follow (double2[8], float2[8]).
-constexpr int WF_FLOATS = 128 + 4 * QG_MAX_GROUPS + 2 * QG_MAX_GROUPS;
-__device__ __forceinline__ double* wf_bf(float* wf) { return reinterpret_cast<double*>(wf + 64); }
-__device__ __forceinline__ float* wf_bfh(float* wf) { return wf + 96; }
-__device__ __forceinline__ float* wf_bfl(float* wf) { return wf + 112; }
+// Per-warp factor slice in shared memory.  Lanes 0-15 of the warp write factor j = lane
+// between two __syncwarp(); every lane reads them as broadcasts.  Held per thread, the arrays
+// were indexed at run time and lived in local memory (1.6 KB of stack per thread, ~1.1e9
+// local-load sectors in one 4096-trajectory launch).  In floats:
+//   0    stage factors dt a_j: mixed float4[16] (hi, hi, lo, lo), pairs for the packed
+//        two-component arithmetic; double form double[16]
+//   64   error factors dt e_j, in the same form (double form: at 32)
+//   128  group coefficients at the current stage time: double2[8], then float2[8]
+//   176  combination factors (double[16], dt-scaled)
+// and, of the slice of the warp that forms them for its block (wf0: the first warp of a CTA,
+// every warp in warp mode), the dense-output factors: double[16] at 176, float4[16] at 208.
+constexpr int WF_FLOATS = 272;
+__device__ __forceinline__ float4* wf_fa(float* wf) { return reinterpret_cast<float4*>(wf); }
+__device__ __forceinline__ float4* wf_fe(float* wf) { return reinterpret_cast<float4*>(wf + 64); }
 __device__ __forceinline__ double2* wf_coef(float* wf) {
   return reinterpret_cast<double2*>(wf + 128);
 }
 __device__ __forceinline__ float2* wf_coef_f(float* wf) {
-  return reinterpret_cast<float2*>(wf + 128 + 4 * QG_MAX_GROUPS);
+  return reinterpret_cast<float2*>(wf + 160);
+}
+__device__ __forceinline__ double* wf_bf(float* wf) { return reinterpret_cast<double*>(wf + 176); }
+__device__ __forceinline__ float4* wf_bf4(float* wf) { return reinterpret_cast<float4*>(wf + 208); }
+
+// hi + lo += (f.x + f.z) k for both components at once (f = (fh, fh, fl, fl)): ff_acc of
+// common.cuh, operation by operation, on packed pairs -- one instruction per two FP32
+// operations, the row loop being bound by instruction issue.
+__device__ __forceinline__ void ff_acc2(float2& hi, float2& lo, float4 f, float2 k) {
+  const float2 fh = make_float2(f.x, f.y), fl = make_float2(f.z, f.w);
+  const float2 np = __fmul2_rn(fh, make_float2(-k.x, -k.y));  // -(fh k)
+  const float2 p = make_float2(-np.x, -np.y);
+  float2 pe = __ffma2_rn(fh, k, np);
+  pe = __ffma2_rn(fl, k, pe);
+  const float2 sum = __fadd2_rn(hi, p);
+  const float2 nhi = make_float2(-hi.x, -hi.y);
+  const float2 bp = __fadd2_rn(sum, nhi);                                  // sum - hi
+  const float2 nbp = make_float2(-bp.x, -bp.y);
+  const float2 back = __fadd2_rn(sum, nbp);                                // sum - bp
+  const float2 nback = make_float2(-back.x, -back.y);
+  const float2 e = __fadd2_rn(__fadd2_rn(hi, nback), __fadd2_rn(p, nbp));
+  hi = sum;
+  lo = __fadd2_rn(lo, __fadd2_rn(e, pe));
 }
 
 template <int DT>
@@ -381,7 +416,8 @@ struct Ctx {
   const ST* opval;        // generator entries: global pool, or the staged copy
   const int* op_col;
   const int* op_rp;
-  float* wf;  // this warp's factor and coefficient slice (shared memory)
+  float* wf;   // this warp's factor and coefficient slice (shared memory)
+  float* wf0;  // the slice that holds the block's dense-output factors
 };
 
 template <typename T>
@@ -420,32 +456,53 @@ __device__ __forceinline__ void load_coef(Ctx<DT>& X, double t) {
   __syncwarp();
 }
 
+// The generator's operands in registers: read from the context struct inside the row loop,
+// they were loaded again for every row and entry (a store through any of its pointers might
+// change it).
+template <int DT>
+struct RowOperands {
+  const typename elem<DT>::T* val;
+  const int* col;
+  const int* rp;
+  float* wf;
+  int G;
+  __device__ __forceinline__ explicit RowOperands(const Ctx<DT>& X)
+      : val(X.opval), col(X.op_col), rp(X.op_rp + X.S->rp_off), wf(X.wf), G(X.G) {}
+};
+
+__device__ __forceinline__ bool part_nonzero(double a) {
+  return ((__double2hiint(a) << 1) | __double2loint(a)) != 0;
+}
+
 // row r of A(t) x in the compute type
 template <int DT, typename XT>
-__device__ __forceinline__ void row_matvec(const Ctx<DT>& X, int r, const XT* x,
+__device__ __forceinline__ void row_matvec(const RowOperands<DT>& O, int r, const XT* x,
                                            typename elem<DT>::R& ar, typename elem<DT>::R& ai) {
   using CT = typename elem<DT>::R;
   ar = 0;
   ai = 0;
-  const int* rp = X.op_rp + X.S->rp_off + (int64_t)r * X.G;
-  for (int g = 0; g < X.G; ++g) {
-    const int s = rp[g], e = rp[g + 1];
+  const int* rp = O.rp + (int64_t)r * O.G;
+  int s = rp[0];
+  for (int g = 0; g < O.G; ++g) {
+    const int e = rp[g + 1];
     CT gr = 0, gi = 0;
+#pragma unroll 4
     for (int p = s; p < e; ++p) {
-      const auto v = X.opval[p];
-      const auto xv = x[X.op_col[p]];
+      const auto v = O.val[p];
+      const auto xv = x[O.col[p]];
       gr = fma((CT)v.x, (CT)xv.x, gr);
       gr = fma(-(CT)v.y, (CT)xv.y, gr);
       gi = fma((CT)v.x, (CT)xv.y, gi);
       gi = fma((CT)v.y, (CT)xv.x, gi);
     }
+    s = e;
     CT cr, ci;
     if constexpr (DT == QG_C64) {
-      const float2 k = wf_coef_f(X.wf)[g];
+      const float2 k = wf_coef_f(O.wf)[g];
       cr = k.x;
       ci = k.y;
     } else {
-      const double2 k = wf_coef(X.wf)[g];
+      const double2 k = wf_coef(O.wf)[g];
       cr = k.x;
       ci = k.y;
     }
@@ -460,39 +517,167 @@ __device__ void matvec_to_k(const GT& g, Ctx<DT>& X, Ctl& c, double t,
                             const typename elem<DT>::T* x, int j) {
   using CT = typename elem<DT>::R;
   load_coef(X, t);
-  for (int r = g.rank; r < X.n; r += GT::SIZE) {
+  const RowOperands<DT> O(X);
+  const int n = X.n;
+  auto* k = X.k + (int64_t)j * n;
+  for (int r = g.rank; r < n; r += GT::SIZE) {
     CT ar, ai;
-    row_matvec(X, r, x, ar, ai);
-    st2(X.k + (int64_t)j * X.n + r, (double)ar, (double)ai);
+    row_matvec(O, r, x, ar, ai);
+    st2(k + r, (double)ar, (double)ai);
   }
   c.rhs += 1;
   g.sync();
 }
 
-// One fused stage: k_s = A(t_prev + c_s dt) x_s and the next stage input, or at
-// s == 9 y_front and the WRMS error (returned).  In the mixed form the stage
-// input x_{s+1} = y_prev + sum_j dt a_{s+1,j} k_j is accumulated in float-float
-// from the complex128 y_prev and rounded once to complex64; the step increment
-// is accumulated the same way and added to y_prev in FP64.
-template <int DT, class GT>
-__device__ __noinline__ double stage(const GT& g, Ctx<DT>& X, Ctl& c, int s, double dt) {
+// The rows of stage S: k_S = A x_S and the next stage input, or at S == 9 y_front, and this
+// thread's part of the WRMS error (returned).  In the mixed form the stage input
+// x_{S+1} = y_prev + sum_j dt a_{S+1,j} k_j is accumulated in float-float from the complex128
+// y_prev and rounded once to complex64; the step increment is accumulated the same way and
+// added to y_prev in FP64.
+//
+// Bound: instruction issue and load latency.  A row took 900 instructions, most of them around
+// the arithmetic: operands loaded again per row, tests of the factors, one load of a k_j
+// waited for after another.  With S a template argument the k_j that have a factor are known
+// to the compiler and loaded together before the row's matvec, and the pair sums run on
+// packed components.  Measured, clocks per stage of a trajectory's CTA (512 rows, two CTAs per
+// SM) 15.5k -> 7.5k, of a 3600-row item's 71k -> 35k; with the shared sums and step control
+// above, 608 Bose-Hubbard trajectories 47 -> 33 ms and 96 Jaynes-Cummings requests 39 -> 25 ms
+// per call (13 to 17 ms of either are host work).
+template <int DT, int S>
+__device__ __noinline__ double stage_rows(const Ctx<DT>& X, int rank, int size, int cur) {
   using ST = typename elem<DT>::T;
   using CT = typename elem<DT>::R;
+  constexpr bool MIXED = (DT == QG_C64);
+  constexpr bool LAST = S == RK_STEP - 1, FORMS = !LAST && S != RK_EXTRA_STEP - 1;
+  constexpr unsigned NA = LAST ? VERN7_NZ_B : (FORMS ? VERN7_NZ_A[S + 1 < 16 ? S + 1 : 15] : 0u);
+  constexpr unsigned NE = LAST ? VERN7_NZ_E : 0u;
+  constexpr unsigned USED = NA | NE;
+  const RowOperands<DT> O(X);
+  const int n = X.n;
+  const int64_t n64 = n;
+  const ST* const kr = X.k;
+  ST* const kw = X.k + S * n64;
+  const double2* const yc = X.y[cur];
+  double2* const yf = X.y[cur ^ 1];
+  const ST *const ysc = X.ys[cur], *const ylc = X.yl[cur];
+  ST *const ysf = X.ys[cur ^ 1], *const ylf = X.yl[cur ^ 1];
+  const float4* const fa4 = wf_fa(X.wf);
+  const float4* const fe4 = wf_fe(X.wf);
+  const double* const fad = reinterpret_cast<const double*>(X.wf);
+  const double* const fed = fad + 16;
+  const double atol = X.S->atol, rtol = X.S->rtol;
+  const ST* x;
+  if constexpr (S == 0) {
+    if constexpr (MIXED) x = ysc;
+    else x = reinterpret_cast<const ST*>(yc);
+  } else {
+    x = X.ytmp + (S & 1) * n64;
+  }
+  ST* const out = X.ytmp + ((S + 1) & 1) * n64;
+  double err_acc = 0.0;
+  for (int r = rank; r < n; r += size) {
+    ST kj[S + 1];
+#pragma unroll
+    for (int j = 0; j < S; ++j)
+      if ((USED >> j) & 1u) kj[j] = kr[j * n64 + r];
+    [[maybe_unused]] float2 bh, bl;
+    [[maybe_unused]] double2 yb;
+    if constexpr (MIXED && FORMS) {
+      bh = ysc[r];
+      bl = ylc[r];
+    } else if constexpr (LAST || !MIXED) {
+      yb = yc[r];
+    }
+    CT ar, ai;
+    row_matvec(O, r, x, ar, ai);
+    st2(kw + r, (double)ar, (double)ai);
+    kj[S].x = ar;  // the stored k_S entry, without reading it back
+    kj[S].y = ai;
+    if constexpr (FORMS) {
+      if constexpr (MIXED) {
+        float2 hi = make_float2(0.f, 0.f), lo = hi;
+#pragma unroll
+        for (int j = 0; j <= S; ++j)
+          if ((NA >> j) & 1u) ff_acc2(hi, lo, fa4[j], kj[j]);
+        out[r] = make_float2(ff_round4(bh.x, bl.x, hi.x, lo.x), ff_round4(bh.y, bl.y, hi.y, lo.y));
+      } else {
+        CT vr = yb.x, vi = yb.y;
+#pragma unroll
+        for (int j = 0; j <= S; ++j) {
+          if ((NA >> j) & 1u) {
+            const CT f = fad[j];
+            vr = fma(f, (CT)kj[j].x, vr);
+            vi = fma(f, (CT)kj[j].y, vi);
+          }
+        }
+        st2(out + r, (double)vr, (double)vi);
+      }
+    } else if constexpr (LAST) {
+      if constexpr (MIXED) {
+        float2 hi = make_float2(0.f, 0.f), lo = hi, eh = hi, el = hi;
+#pragma unroll
+        for (int j = 0; j <= S; ++j) {
+          if (!((USED >> j) & 1u)) continue;
+          ff_acc2(hi, lo, fa4[j], kj[j]);
+          ff_acc2(eh, el, fe4[j], kj[j]);  // error estimate in float-float
+        }
+        // the once-per-step FP64 state update, then its float-pair shadow
+        const double yr = yb.x + ((double)hi.x + (double)lo.x);
+        const double yi = yb.y + ((double)hi.y + (double)lo.y);
+        yf[r] = make_double2(yr, yi);
+        float shr, slr, shi, sli;
+        split_f(yr, shr, slr);
+        split_f(yi, shi, sli);
+        ysf[r] = make_float2(shr, shi);
+        ylf[r] = make_float2(slr, sli);
+        // WRMS error term in FP64 against the FP64 state (wrmn_error_dense,
+        // qutip/core/data/ode.pyx:27-52), written as |e|^2 / (atol + rtol |y|)^2
+        const double er = (double)eh.x + (double)el.x, ei = (double)eh.y + (double)el.y;
+        // (roundings spelt out: the last bit of the sum reaches the step size, and through it
+        // every later rounding of a complex64 stage)
+        err_acc = __fma_rn(__fma_rn(er, er, __dmul_rn(ei, ei)),
+                           wrms_inv2(__fma_rn(yr, yr, __dmul_rn(yi, yi)), atol, rtol), err_acc);
+      } else {
+        CT er = 0, ei = 0;
+        double yr = yb.x, yi = yb.y;
+#pragma unroll
+        for (int j = 0; j <= S; ++j) {
+          if ((NA >> j) & 1u) {
+            yr = fma(fad[j], (double)kj[j].x, yr);
+            yi = fma(fad[j], (double)kj[j].y, yi);
+          }
+          if ((NE >> j) & 1u) {
+            er = fma((CT)fed[j], (CT)kj[j].x, er);
+            ei = fma((CT)fed[j], (CT)kj[j].y, ei);
+          }
+        }
+        yf[r] = make_double2(yr, yi);
+        // IEEE square roots and division: the complex128 form takes the reference's steps
+        // (a 1e-13 change of the error norm moved one of 4096 BH trajectories' jumps)
+        const double w = sqrt((double)er * er + (double)ei * ei) /
+                         (atol + rtol * sqrt(yr * yr + yi * yi));
+        err_acc += w * w;
+      }
+    }
+  }
+  return err_acc;
+}
+
+// One fused stage s: its factors and coefficients, then its rows.  At s == 9 the error norm
+// and the step-size factor of _recompute_safe_step (explicit_rk.pyx:451-467, FP64 in both
+// forms) are returned.
+template <int DT, class GT>
+__device__ __noinline__ double2 stage(const GT& g, Ctx<DT>& X, Ctl& c, int s, double dt) {
   constexpr bool MIXED = (DT == QG_C64);
   const bool last = (s == RK_STEP - 1);
   const bool forms_input = !last && s != RK_EXTRA_STEP - 1;
   const int nk = last ? RK_STEP : s + 1;  // k_j that enter the combination
   // factors: FP64 for the double form; float pairs from the hi/lo tableau for the
   // mixed form (no FP64 work per stage); lane j of each warp forms factor j
-  const CT* fa;
-  const CT* fe;
-  const float* fl;
-  const float* fel;
   {
     const int j = lane_id();
     __syncwarp();  // the warp's earlier readers of the slice are done
     if constexpr (MIXED) {
-      float* w = X.wf;
       if (j < 16) {
         float dh, dl;
         split_f(dt, dh, dl);
@@ -508,13 +693,14 @@ __device__ __noinline__ double stage(const GT& g, Ctx<DT>& X, Ctl& c, int s, dou
             al = VERN7_AL[s + 1][j];
           }
         }
-        ff_factor(dh, dl, ah, al, w[j], w[16 + j]);
-        ff_factor(dh, dl, eh, el, w[32 + j], w[48 + j]);
+        float fh, fl;
+        ff_factor(dh, dl, ah, al, fh, fl);
+        wf_fa(X.wf)[j] = make_float4(fh, fh, fl, fl);
+        if (last) {
+          ff_factor(dh, dl, eh, el, fh, fl);
+          wf_fe(X.wf)[j] = make_float4(fh, fh, fl, fl);
+        }
       }
-      fa = reinterpret_cast<const CT*>(w);
-      fl = w + 16;
-      fe = reinterpret_cast<const CT*>(w + 32);
-      fel = w + 48;
     } else {
       double* w = reinterpret_cast<double*>(X.wf);
       if (j < 16) {
@@ -530,142 +716,77 @@ __device__ __noinline__ double stage(const GT& g, Ctx<DT>& X, Ctl& c, int s, dou
         w[j] = a;
         w[16 + j] = e;
       }
-      fa = reinterpret_cast<const CT*>(w);
-      fe = reinterpret_cast<const CT*>(w + 16);
-      fl = fel = nullptr;  // not used by the double form
     }
     __syncwarp();
   }
   load_coef(X, c.t_prev + VERN7_C[s] * dt);
-  const int cur = c.cur;
-  const ST* x;
-  if (s == 0) {
-    if constexpr (MIXED) x = X.ys[cur];
-    else x = reinterpret_cast<const ST*>(X.y[cur]);
-  } else {
-    x = X.ytmp + (int64_t)(s & 1) * X.n;
-  }
-  ST* out = X.ytmp + (int64_t)((s + 1) & 1) * X.n;
-  const int64_t n = X.n;
-  double err_acc = 0.0;
-  for (int r = g.rank; r < X.n; r += GT::SIZE) {
-    CT ar, ai;
-    row_matvec(X, r, x, ar, ai);
-    st2(X.k + s * n + r, (double)ar, (double)ai);
-    ST ks;  // the stored k_s entry, without reading it back
-    ks.x = ar;
-    ks.y = ai;
-    if (forms_input) {
-      if constexpr (MIXED) {
-        float hr = 0.f, lr = 0.f, hi = 0.f, li = 0.f;
-        for (int j = 0; j <= s; ++j) {
-          if (fa[j] != 0.f || fl[j] != 0.f) {
-            const ST kj = (j == s) ? ks : X.k[j * n + r];
-            ff_acc(hr, lr, fa[j], fl[j], kj.x);
-            ff_acc(hi, li, fa[j], fl[j], kj.y);
-          }
-        }
-        const float2 bh = X.ys[cur][r], bl = X.yl[cur][r];
-        out[r] = make_float2(ff_round4(bh.x, bl.x, hr, lr), ff_round4(bh.y, bl.y, hi, li));
-      } else {
-        CT vr = X.y[cur][r].x, vi = X.y[cur][r].y;
-        for (int j = 0; j <= s; ++j) {
-          const CT f = fa[j];
-          if (f != (CT)0) {
-            const ST kj = (j == s) ? ks : X.k[j * n + r];
-            vr = fma(f, (CT)kj.x, vr);
-            vi = fma(f, (CT)kj.y, vi);
-          }
-        }
-        st2(out + r, (double)vr, (double)vi);
-      }
-    } else if (last) {
-      if constexpr (MIXED) {
-        float hr = 0.f, lr = 0.f, hi = 0.f, li = 0.f;
-        float erh = 0.f, erl = 0.f, eih = 0.f, eil = 0.f;
-        for (int j = 0; j < RK_STEP; ++j) {
-          if (fa[j] == 0.f && fl[j] == 0.f && fe[j] == 0.f && fel[j] == 0.f) continue;
-          const ST kj = (j == s) ? ks : X.k[j * n + r];
-          ff_acc(hr, lr, fa[j], fl[j], kj.x);
-          ff_acc(hi, li, fa[j], fl[j], kj.y);
-          ff_acc(erh, erl, fe[j], fel[j], kj.x);   // error estimate in float-float
-          ff_acc(eih, eil, fe[j], fel[j], kj.y);
-        }
-        // the once-per-step FP64 state update, then its float-pair shadow
-        const double yr = X.y[cur][r].x + ((double)hr + (double)lr);
-        const double yi = X.y[cur][r].y + ((double)hi + (double)li);
-        X.y[cur ^ 1][r] = make_double2(yr, yi);
-        float shr, slr, shi, sli;
-        split_f(yr, shr, slr);
-        split_f(yi, shi, sli);
-        X.ys[cur ^ 1][r] = make_float2(shr, shi);
-        X.yl[cur ^ 1][r] = make_float2(slr, sli);
-        // WRMS error term in FP64 against the FP64 state (wrmn_error_dense,
-        // qutip/core/data/ode.pyx:27-52), written as |e|^2 / (atol + rtol |y|)^2
-        const double er = (double)erh + (double)erl, ei = (double)eih + (double)eil;
-        err_acc += wrms_term(er * er + ei * ei, yr * yr + yi * yi, X.S->atol, X.S->rtol);
-      } else {
-        CT er = 0, ei = 0;
-        double yr = X.y[cur][r].x, yi = X.y[cur][r].y;
-        for (int j = 0; j < RK_STEP; ++j) {
-          const double fb = (double)fa[j], fq = (double)fe[j];
-          if (fb == 0.0 && fq == 0.0) continue;
-          const ST kj = (j == s) ? ks : X.k[j * n + r];
-          if (fb != 0.0) {
-            yr = fma(fb, (double)kj.x, yr);
-            yi = fma(fb, (double)kj.y, yi);
-          }
-          if (fq != 0.0) {
-            er = fma((CT)fq, (CT)kj.x, er);
-            ei = fma((CT)fq, (CT)kj.y, ei);
-          }
-        }
-        X.y[cur ^ 1][r] = make_double2(yr, yi);
-        // IEEE square roots and division: the complex128 form takes the reference's steps
-        // (a 1e-13 change of the error norm moved one of 4096 BH trajectories' jumps)
-        const double w = sqrt((double)er * er + (double)ei * ei) /
-                         (X.S->atol + X.S->rtol * sqrt(yr * yr + yi * yi));
-        err_acc += w * w;
-      }
-    }
+  double err = 0.0;
+  switch (s) {
+#define QG_ROWS(S)                                    \
+  case S:                                             \
+    err = stage_rows<DT, S>(X, g.rank, GT::SIZE, c.cur); \
+    break;
+    QG_ROWS(0) QG_ROWS(1) QG_ROWS(2) QG_ROWS(3) QG_ROWS(4) QG_ROWS(5) QG_ROWS(6) QG_ROWS(7)
+    QG_ROWS(8) QG_ROWS(9) QG_ROWS(10) QG_ROWS(11) QG_ROWS(12) QG_ROWS(13) QG_ROWS(14) QG_ROWS(15)
+#undef QG_ROWS
   }
   c.rhs += 1;
-  double err = 0.0;
-  if (last) err = sqrt(g.sum(err_acc) / (double)X.n);
-  g.sync();
-  return err;
+  double2 res = make_double2(0.0, 0.0);
+  if (last) {
+    const double n = (double)X.n;
+    res = g.sum_map(err, [n](double t) {
+      const double e = sqrt(t / n);
+      // one thread's pow: the FP64 pipe would see one per lane
+      double f = 10.0;
+      if (e != 0.0) {
+        f = 0.0;
+        if (lane_id() == 0) f = fmax(0.2, fmin(10.0, 0.9 * pow(e, -1.0 / (RK_ORDER + 1))));
+        f = shfl_d(f, 0);
+      }
+      return make_double2(e, f);
+    });
+    g.block_sync();  // (the sum's barrier ordered the rows' vectors)
+  } else {
+    g.sync();
+  }
+  return res;
 }
 
 // Mixed form: out = fl32(y_prev + sum_{j<nk} dt a_{row,j} k_j) in float pairs from
-// the (ys, yl) base -- the stage input of the first dense-output stage.
+// the (ys, yl) base -- the stage input of the first dense-output stage (row = nk = RK_STEP).
 template <int DT, class GT>
 __device__ void form_input_mixed(const GT& g, Ctx<DT>& X, const Ctl& c, typename elem<DT>::T* out,
-                                 int row, int nk, double dt) {
+                                 double dt) {
+  constexpr int row = RK_STEP, nk = RK_STEP;
   using ST = typename elem<DT>::T;
-  float* fa = X.wf;
-  float* fl = X.wf + 16;
+  float4* const fa = wf_fa(X.wf);
   __syncwarp();
   if (lane_id() < 16) {
     const int j = lane_id();
     float dh, dl;
     split_f(dt, dh, dl);
     const float ah = j < nk ? VERN7_AH[row][j] : 0.f, al = j < nk ? VERN7_AL[row][j] : 0.f;
-    ff_factor(dh, dl, ah, al, fa[j], fl[j]);
+    float fh, fl;
+    ff_factor(dh, dl, ah, al, fh, fl);
+    fa[j] = make_float4(fh, fh, fl, fl);
   }
   __syncwarp();
-  const int cur = c.cur;
-  const int64_t n = X.n;
-  for (int r = g.rank; r < X.n; r += GT::SIZE) {
-    float hr = 0.f, lr = 0.f, hi = 0.f, li = 0.f;
-    for (int j = 0; j < nk; ++j) {
-      if (fa[j] != 0.f || fl[j] != 0.f) {
-        const ST kj = X.k[j * n + r];
-        ff_acc(hr, lr, fa[j], fl[j], kj.x);
-        ff_acc(hi, li, fa[j], fl[j], kj.y);
-      }
-    }
-    const float2 bh = X.ys[cur][r], bl = X.yl[cur][r];
-    out[r] = make_float2(ff_round4(bh.x, bl.x, hr, lr), ff_round4(bh.y, bl.y, hi, li));
+  constexpr unsigned NA = VERN7_NZ_A[RK_STEP];
+  const int n = X.n;
+  const int64_t n64 = n;
+  const ST* const kr = X.k;
+  const ST *const ysc = X.ys[c.cur], *const ylc = X.yl[c.cur];
+  for (int r = g.rank; r < n; r += GT::SIZE) {
+    ST kj[RK_STEP];
+#pragma unroll
+    for (int j = 0; j < RK_STEP; ++j)
+      if ((NA >> j) & 1u) kj[j] = kr[j * n64 + r];
+    float2 hi = make_float2(0.f, 0.f), lo = hi;
+#pragma unroll
+    for (int j = 0; j < RK_STEP; ++j)
+      if ((NA >> j) & 1u) ff_acc2(hi, lo, fa[j], kj[j]);
+    const float2 bh = ysc[r], bl = ylc[r];
+    out[r] = make_float2(ff_round4(bh.x, bl.x, hi.x, lo.x), ff_round4(bh.y, bl.y, hi.y, lo.y));
   }
   g.sync();
 }
@@ -674,13 +795,17 @@ __device__ void form_input_mixed(const GT& g, Ctx<DT>& X, const Ctl& c, typename
 template <int DT, class GT, typename OT, typename BT>
 __device__ void combine(const GT& g, Ctx<DT>& X, const Ctl& c, OT* out, const BT* base, int nk) {
   const double* bf = wf_bf(X.wf);
-  for (int r = g.rank; r < X.n; r += GT::SIZE) {
+  const int n = X.n;
+  const auto* const k = X.k;
+  for (int r = g.rank; r < n; r += GT::SIZE) {
     double vr = (double)base[r].x, vi = (double)base[r].y;
+#pragma unroll 4
     for (int j = 0; j < nk; ++j) {
       const double f = bf[j];
-      if (f != 0.0) {
-        vr = fma(f, (double)X.k[(int64_t)j * X.n + r].x, vr);
-        vi = fma(f, (double)X.k[(int64_t)j * X.n + r].y, vi);
+      if (part_nonzero(f)) {
+        const auto kv = k[(int64_t)j * n + r];
+        vr = fma(f, (double)kv.x, vr);
+        vi = fma(f, (double)kv.y, vi);
       }
     }
     st2(out + r, vr, vi);
@@ -688,44 +813,82 @@ __device__ void combine(const GT& g, Ctx<DT>& X, const Ctl& c, OT* out, const BT
   g.sync();
 }
 
-// entry i of the current state: y_front, or y_prev + sum_j bf_j k_j (the mixed
-// form sums the increment in float pairs and adds it to y_prev in FP64)
+// Entries of the current state: y_front, or y_prev + sum_j bf_j k_j (the mixed form sums the
+// increment in float pairs and adds it to y_prev in FP64).  Built by whole warps; the
+// pointers and the set of nonzero factors stay in registers, and an entry's k_j are loaded
+// together.
 template <int DT>
-__device__ __forceinline__ double2 state_at(const Ctx<DT>& X, const Ctl& c, int i) {
-  if (c.out_front) return X.y[c.cur ^ 1][i];
-  if constexpr (DT == QG_C64) {
-    const float* bfh = wf_bfh(X.wf);
-    const float* bfl = wf_bfl(X.wf);
-    float hr = 0.f, lr = 0.f, hi = 0.f, li = 0.f;
-    for (int j = 0; j < RK_EXTRA_STEP; ++j) {
-      if (bfh[j] != 0.f || bfl[j] != 0.f) {
-        const float2 kj = X.k[(int64_t)j * X.n + i];
-        ff_acc(hr, lr, bfh[j], bfl[j], kj.x);
-        ff_acc(hi, li, bfh[j], bfl[j], kj.y);
+struct StateReader {
+  using ST = typename elem<DT>::T;
+  const double2* y;
+  const ST* k;
+  float* wf0;
+  int64_t n;
+  unsigned int use;  // 0 for y_front
+  __device__ __forceinline__ StateReader(const Ctx<DT>& X, const Ctl& c)
+      : y(X.y[c.out_front ? c.cur ^ 1 : c.cur]), k(X.k), wf0(X.wf0), n(X.n) {
+    bool u = false;
+    if (!c.out_front && lane_id() < RK_EXTRA_STEP) {
+      if constexpr (DT == QG_C64) {
+        const float4 f = wf_bf4(wf0)[lane_id()];
+        u = f.x != 0.f || f.z != 0.f;
+      } else {
+        u = wf_bf(wf0)[lane_id()] != 0.0;
       }
     }
-    return make_double2(X.y[c.cur][i].x + ((double)hr + (double)lr),
-                        X.y[c.cur][i].y + ((double)hi + (double)li));
-  } else {
-    const double* bf = wf_bf(X.wf);
-    double vr = X.y[c.cur][i].x, vi = X.y[c.cur][i].y;
-    for (int j = 0; j < RK_EXTRA_STEP; ++j) {
-      const double f = bf[j];
-      if (f != 0.0) {
-        vr = fma(f, (double)X.k[(int64_t)j * X.n + i].x, vr);
-        vi = fma(f, (double)X.k[(int64_t)j * X.n + i].y, vi);
-      }
-    }
-    return make_double2(vr, vi);
+    use = __ballot_sync(0xffffffffu, u);
   }
-}
+  __device__ __forceinline__ double2 at(int i) const {
+    const double2 b = y[i];
+    if (use == 0u) return b;
+    if constexpr (DT == QG_C64) {
+      const float4* const f = wf_bf4(wf0);
+      ST kj[RK_EXTRA_STEP];
+#pragma unroll
+      for (int j = 0; j < RK_EXTRA_STEP; ++j)
+        if ((use >> j) & 1u) kj[j] = k[j * n + i];
+      float2 hi = make_float2(0.f, 0.f), lo = hi;
+#pragma unroll
+      for (int j = 0; j < RK_EXTRA_STEP; ++j)
+        if ((use >> j) & 1u) ff_acc2(hi, lo, f[j], kj[j]);
+      return make_double2(b.x + ((double)hi.x + (double)lo.x), b.y + ((double)hi.y + (double)lo.y));
+    } else {
+      const double* const bf = wf_bf(wf0);
+      double vr = b.x, vi = b.y;
+#pragma unroll
+      for (int j0 = 0; j0 < RK_EXTRA_STEP; j0 += 8) {
+        ST kj[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if ((use >> (j0 + j)) & 1u) kj[j] = k[(j0 + j) * n + i];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if ((use >> (j0 + j)) & 1u) {
+            vr = fma(bf[j0 + j], (double)kj[j].x, vr);
+            vi = fma(bf[j0 + j], (double)kj[j].y, vi);
+          }
+        }
+      }
+      return make_double2(vr, vi);
+    }
+  }
+};
 
-template <int DT, class GT>
-__device__ double state_norm2(const GT& g, const Ctx<DT>& X, const Ctl& c) {
+// |state|^2 of a trajectory; the state goes to ctmp[0] on the way.  The roundings are spelt
+// out, the imaginary part's square fused after a step (SEARCH: the real part's, in the
+// jump-time search): a jump's time follows the last bits of these norms, and in the mixed
+// form every later rounding of the trajectory follows the jump.
+template <bool SEARCH, int DT, class GT>
+__device__ __noinline__ double state_norm2(const GT& g, const Ctx<DT>& X, const Ctl& c) {
   double acc = 0.0;
-  for (int r = g.rank; r < X.n; r += GT::SIZE) {
-    const double2 v = state_at(X, c, r);
-    acc += v.x * v.x + v.y * v.y;
+  const StateReader<DT> at(X, c);
+  double2* const psi = X.ctmp[0];
+  const int n = X.n;
+  for (int r = g.rank; r < n; r += GT::SIZE) {
+    const double2 v = at.at(r);
+    psi[r] = v;
+    acc = __dadd_rn(acc, SEARCH ? __fma_rn(v.x, v.x, __dmul_rn(v.y, v.y))
+                                : __fma_rn(v.y, v.y, __dmul_rn(v.x, v.x)));
   }
   return g.sum(acc);
 }
@@ -802,7 +965,7 @@ __device__ __noinline__ void prep_dense_out(const GT& g, Ctx<DT>& X, Ctl& c) {
   const double dt = c.dt_int;
   ST* x10 = X.ytmp + (int64_t)(RK_STEP & 1) * X.n;
   if constexpr (DT == QG_C64) {
-    form_input_mixed(g, X, c, x10, RK_STEP, RK_STEP, dt);
+    form_input_mixed(g, X, c, x10, dt);
   } else {
     __syncwarp();
     if (lane_id() < 16)
@@ -816,27 +979,30 @@ __device__ __noinline__ void prep_dense_out(const GT& g, Ctx<DT>& X, Ctl& c) {
 
 // dense-output factors at t (Horner in tau, explicit_rk.pyx:412-430); lane i
 // evaluates factor i
-template <int DT>
-__device__ __forceinline__ void set_interp(const Ctx<DT>& X, Ctl& c, double t) {
-  const double tau = (t - c.t_prev) / c.dt_int;
-  double mine = 0.0;
-  float mh = 0.f, ml = 0.f;
-  if (lane_id() < RK_EXTRA_STEP) {
-    double acc = 0.0;
-    for (int j = DENSE_ORDER - 1; j >= 0; --j) {
-      acc += VERN7_BI[lane_id()][j];
-      acc *= tau;
+// of the warp that forms them for its block (the readers of the last ones have passed a
+// barrier since: every use of a StateReader ends in one)
+template <int DT, class GT>
+__device__ __forceinline__ void set_interp(const GT& g, const Ctx<DT>& X, Ctl& c, double t) {
+  if (g.forms_shared()) {
+    const double tau = (t - c.t_prev) / c.dt_int;
+    double mine = 0.0;
+    float mh = 0.f, ml = 0.f;
+    if (lane_id() < RK_EXTRA_STEP) {
+      double acc = 0.0;
+      for (int j = DENSE_ORDER - 1; j >= 0; --j) {
+        acc += VERN7_BI[lane_id()][j];
+        acc *= tau;
+      }
+      mine = c.dt_int * acc;
+      split_f(mine, mh, ml);
     }
-    mine = c.dt_int * acc;
-    split_f(mine, mh, ml);
+    __syncwarp();
+    if (lane_id() < RK_EXTRA_STEP) {
+      wf_bf(X.wf0)[lane_id()] = mine;
+      wf_bf4(X.wf0)[lane_id()] = make_float4(mh, mh, ml, ml);
+    }
   }
-  __syncwarp();
-  if (lane_id() < RK_EXTRA_STEP) {
-    wf_bf(X.wf)[lane_id()] = mine;
-    wf_bfh(X.wf)[lane_id()] = mh;
-    wf_bfl(X.wf)[lane_id()] = ml;
-  }
-  __syncwarp();
+  g.block_sync();
   c.out_front = 0;
   c.t = t;
 }
@@ -848,24 +1014,11 @@ __device__ int step_in_err(const GT& g, Ctx<DT>& X, Ctl& c, int nsteps_left) {
   int nsteps = 0;
   while (true) {
     const double dt = c.dt_safe;
-    double err = 0.0;
-    for (int s = 0; s < RK_STEP; ++s) {
-      const double e = stage(g, X, c, s, dt);
-      if (s == RK_STEP - 1) err = e;
-    }
+    double2 ef = make_double2(0.0, 0.0);
+    for (int s = 0; s < RK_STEP; ++s) ef = stage(g, X, c, s, dt);
+    const double err = ef.x, factor = ef.y;
     c.t_front = c.t_prev + dt;
     c.dt_int = dt;
-    // _recompute_safe_step (explicit_rk.pyx:451-467) in FP64 for both forms.  Every
-    // thread holds the same err; lane 0 of each warp takes the pow and shares it, so
-    // the FP64 pipe sees one pow per warp, not one per thread.
-    double factor;
-    if (err == 0.0) {
-      factor = 10.0;
-    } else {
-      double mine = 0.0;
-      if (lane_id() == 0) mine = fmax(0.2, fmin(10.0, 0.9 * pow(err, -1.0 / (RK_ORDER + 1))));
-      factor = shfl_d(mine, 0);
-    }
     c.dt_safe = fmax(1e-15, dt * factor);
     c.interp_ready = 0;
     c.steps += 1;
@@ -894,7 +1047,7 @@ __device__ void integrate(const GT& g, Ctx<DT>& X, Ctl& c, double t, bool step) 
   }
   if (t < c.t_front) {
     if (!c.interp_ready) prep_dense_out(g, X, c);
-    set_interp(X, c, t);
+    set_interp(g, X, c, t);
     return;
   }
   c.status = QG_NORMAL;
@@ -909,7 +1062,7 @@ __device__ void integrate(const GT& g, Ctx<DT>& X, Ctl& c, double t, bool step) 
   if (c.status < 0) return;
   if (c.t_front > t) {
     prep_dense_out(g, X, c);
-    set_interp(X, c, t);
+    set_interp(g, X, c, t);
   } else {
     c.out_front = 1;
     c.t = c.t_front;
@@ -917,79 +1070,98 @@ __device__ void integrate(const GT& g, Ctx<DT>& X, Ctl& c, double t, bool step) 
 }
 
 // ------------------------------------------------------------- outputs ------
+// This thread's part of output sum e: <op_e> for e < n_eops, else the norm or the trace.
+template <int DT>
+__device__ __noinline__ double2 output_part(const Ctx<DT>& X, const StateReader<DT>& at, int e,
+                                            bool ket, int rank, int size) {
+  const int ne = X.S->n_eops, d = X.d, n = X.n;
+  const double2* const psi = X.ctmp[0];
+  double ar = 0.0, ai = 0.0;
+  if (e < ne) {
+    const int* const rp = X.B->eop_rp + X.S->eop_rp_off + (int64_t)e * (d + 1);
+    const int* const ecol = X.B->eop_col;
+    const double* const eval = X.B->eop_val;
+    for (int r = rank; r < d; r += size) {
+      const int s = __ldg(rp + r), en = __ldg(rp + r + 1);
+      double sr = 0.0, si = 0.0;
+      for (int p = s; p < en; ++p) {
+        const int col = __ldg(ecol + p);
+        const double vr = __ldg(eval + 2 * p), vi = __ldg(eval + 2 * p + 1);
+        const double2 z = ket ? psi[col] : at.at(col + r * d);
+        sr += vr * z.x - vi * z.y;
+        si += vr * z.y + vi * z.x;
+      }
+      if (ket) {
+        const double2 pr = psi[r];
+        const double tr = pr.x * sr + pr.y * si, ti = pr.x * si - pr.y * sr;
+        sr = tr;
+        si = ti;
+      }
+      ar += sr;
+      ai += si;
+    }
+  } else if (ket) {  // the norm
+    for (int r = rank; r < n; r += size) {
+      const double2 z = psi[r];
+      ar += z.x * z.x + z.y * z.y;
+    }
+  } else {  // the trace
+    for (int r = rank; r < d; r += size) {
+      const double2 z = at.at(r + r * d);
+      ar += z.x;
+      ai += z.y;
+    }
+  }
+  return make_double2(ar, ai);
+}
+
 // expectation values of the current state into out[0..ne] (raw; host normalises).
-// A ket is interpolated once into ctmp[0] and every e_op reads it there; a density
-// matrix is read entry by entry (the e_ops touch a small part of it).
-// CTA and cluster groups gather the warp partials of up to REC_SLOTS sums behind one
-// pair of barriers (a barrier pair per sum made most of the cost of an output for
-// large items in a cluster).  Returns the host cancel flag, read once per record by
-// rank 0 and shared behind the same barriers (0 without a flag).
+// A ket is interpolated once into ctmp[0] (`ready`: the norm of this state was taken last and
+// left it there) and every e_op reads it there; a density matrix is read entry by entry (the
+// e_ops touch a small part of it).  CTA and cluster groups gather the warp partials of up to
+// REC_SLOTS sums behind one pair of barriers (a barrier pair per sum made most of the cost of
+// an output for large items in a cluster), a lane of the first warp adding each.  Returns the
+// host cancel flag, read once per record by rank 0 and shared behind the same barriers (0
+// without a flag).
 template <int DT, class GT>
 __device__ __noinline__ int record(const GT& g, const Ctx<DT>& X, const Ctl& c, double2* out,
-                                   bool ket, const volatile int32_t* cancel) {
+                                   bool ket, bool ready, const volatile int32_t* cancel) {
   const int ne = X.S->n_eops;
-  const int d = X.d;
-  const double2* psi = X.ctmp[0];
+  const StateReader<DT> at(X, c);
   if (ket) {
-    for (int r = g.rank; r < X.n; r += GT::SIZE) X.ctmp[0][r] = state_at(X, c, r);
+    if (!ready) {
+      double2* const psi = X.ctmp[0];
+      const int n = X.n;
+      for (int r = g.rank; r < n; r += GT::SIZE) psi[r] = at.at(r);
+    }
     g.sync();
   }
   int flag = 0;
-  for (int e0 = 0; e0 <= ne; e0 += REC_SLOTS) {
-    const int e1 = min(ne + 1, e0 + REC_SLOTS);
-    for (int e = e0; e < e1; ++e) {
-      double ar = 0.0, ai = 0.0;
-      if (e < ne) {
-        const int* rp = X.B->eop_rp + X.S->eop_rp_off + (int64_t)e * (d + 1);
-        for (int r = g.rank; r < d; r += GT::SIZE) {
-          const int s = __ldg(rp + r), en = __ldg(rp + r + 1);
-          double sr = 0.0, si = 0.0;
-          for (int p = s; p < en; ++p) {
-            const int col = __ldg(X.B->eop_col + p);
-            const double vr = __ldg(X.B->eop_val + 2 * p), vi = __ldg(X.B->eop_val + 2 * p + 1);
-            const double2 z = ket ? psi[col] : state_at(X, c, col + r * d);
-            sr += vr * z.x - vi * z.y;
-            si += vr * z.y + vi * z.x;
-          }
-          if (ket) {
-            const double2 pr = psi[r];
-            const double tr = pr.x * sr + pr.y * si, ti = pr.x * si - pr.y * sr;
-            sr = tr;
-            si = ti;
-          }
-          ar += sr;
-          ai += si;
-        }
-      } else if (ket) {  // the norm
-        for (int r = g.rank; r < X.n; r += GT::SIZE) {
-          const double2 z = psi[r];
-          ar += z.x * z.x + z.y * z.y;
-        }
-      } else {  // the trace
-        for (int r = g.rank; r < d; r += GT::SIZE) {
-          const double2 z = state_at(X, c, r + r * d);
-          ar += z.x;
-          ai += z.y;
-        }
+  if constexpr (GT::DEFER) {
+    for (int e0 = 0; e0 <= ne; e0 += REC_SLOTS) {
+      const int e1 = min(ne + 1, e0 + REC_SLOTS);
+      double v[2 * REC_SLOTS];
+#pragma unroll
+      for (int i = 0; i < REC_SLOTS; ++i) {
+        double2 p = make_double2(0.0, 0.0);
+        if (e0 + i < e1) p = output_part(X, at, e0 + i, ket, g.rank, GT::SIZE);
+        v[2 * i] = p.x;
+        v[2 * i + 1] = p.y;
       }
-      if constexpr (GT::DEFER) {
-        g.put2(e - e0, ar, ai);
-      } else {
-        const double2 t = g.sum2(ar, ai);
-        if (g.rank == 0) out[e] = t;
-      }
-    }
-    if constexpr (GT::DEFER) {
+      g.put_all(v);
       const bool final_chunk = e1 == ne + 1;
       if (final_chunk && cancel) g.put_flag(g.rank == 0 ? read_flag(cancel) : 0);
       g.sync();
       if (final_chunk && cancel) flag = g.take_flag();
-      if (g.rank == 0)
-        for (int e = e0; e < e1; ++e) out[e] = g.take2(e - e0);
-      if (!final_chunk) g.sync();  // rank 0 has read the partials before they are reused
+      if (g.rank < e1 - e0) out[e0 + g.rank] = g.take2(g.rank);
+      if (!final_chunk) g.sync();  // the partials are read before they are reused
     }
-  }
-  if constexpr (!GT::DEFER) {
+  } else {
+    for (int e = 0; e <= ne; ++e) {
+      const double2 p = output_part(X, at, e, ket, g.rank, GT::SIZE);
+      const double2 t = g.sum2(p.x, p.y);
+      if (g.rank == 0) out[e] = t;
+    }
     if (cancel) flag = g.bcast(g.rank == 0 ? read_flag(cancel) : 0);
   }
   g.sync();
@@ -1026,7 +1198,7 @@ __device__ double cop_apply(const GT& g, Ctx<DT>& X, int i, bool store, double t
       sr = fr;
     }
     if (store) X.ctmp[1][r] = make_double2(sr, si);
-    acc += sr * sr + si * si;
+    acc = __dadd_rn(acc, __fma_rn(sr, sr, __dmul_rn(si, si)));
   }
   const double tot = g.sum(acc);
   g.sync();
@@ -1070,7 +1242,10 @@ __device__ void run_item(const GT& g, const qg_batch& B, Ctx<DT>& X, int item) {
   double target = ket ? __dadd_rn(__dmul_rn(pcg_random(rng), 1.0 - floor_p), floor_p) : 0.0;
   int njumps = 0;
   set_initial(g, X, c, reinterpret_cast<const double2*>(B.y0) + I.y0_off, tl[0]);
-  int cancelled = record(g, X, c, out, ket, B.cancel);
+  int cancelled = record(g, X, c, out, ket, false, B.cancel);
+  // |state|^2 at c.t when `have` (taken last, with the state left in ctmp[0])
+  double norm_now = 0.0;
+  bool have = false;
   for (int o = 1; o < S->n_out && c.status >= 0; ++o) {
     const double t = tl[o];
     if (B.progress && g.rank == 0)
@@ -1085,7 +1260,7 @@ __device__ void run_item(const GT& g, const qg_batch& B, Ctx<DT>& X, int item) {
     } else {
       // MCIntegrator.integrate (mcsolve.py:286-302)
       double t_old = c.t;
-      double norm_old = state_norm2(g, X, c);
+      double norm_old = have ? norm_now : state_norm2<false>(g, X, c);
       int iters = 0;
       while (t_old < t && c.status >= 0) {
         if (++iters > MC_MAX_ITER) {
@@ -1113,12 +1288,14 @@ __device__ void run_item(const GT& g, const qg_batch& B, Ctx<DT>& X, int item) {
         integrate(g, X, c, t, true);
         if (c.status < 0) break;
         const double t_step = c.t;
-        const double nrm = state_norm2(g, X, c);
+        const double nrm = state_norm2<false>(g, X, c);
         if (nrm > target) {
           t_old = t_step;
-          norm_old = nrm;
+          norm_old = norm_now = nrm;
+          have = true;
           continue;
         }
+        have = false;
         // _find_collapse_time (mcsolve.py:321-369)
         double tp = t_old, tf = t_step, no = norm_old, nn = nrm, t_guess = tf;
         int tries = 0;
@@ -1136,7 +1313,7 @@ __device__ void run_item(const GT& g, const qg_batch& B, Ctx<DT>& X, int item) {
           if ((t_guess - tp) < B.norm_t_tol) t_guess = tp + B.norm_t_tol;
           integrate(g, X, c, t_guess, true);
           if (c.status < 0) break;
-          const double n2 = state_norm2(g, X, c);
+          const double n2 = state_norm2<true>(g, X, c);
           if (fabs(target - n2) < B.norm_tol * target) break;
           if (n2 < target) {
             tf = t_guess;
@@ -1152,7 +1329,10 @@ __device__ void run_item(const GT& g, const qg_batch& B, Ctx<DT>& X, int item) {
           break;
         }
         // _do_collapse (mcsolve.py:371-406): psi = state at t_guess
-        for (int r = g.rank; r < X.n; r += GT::SIZE) X.ctmp[0][r] = state_at(X, c, r);
+        {
+          const StateReader<DT> at(X, c);
+          for (int r = g.rank; r < X.n; r += GT::SIZE) X.ctmp[0][r] = at.at(r);
+        }
         g.sync();
         int which = 0;
         const int nc = S->n_cops;
@@ -1194,7 +1374,7 @@ __device__ void run_item(const GT& g, const qg_batch& B, Ctx<DT>& X, int item) {
       }
     }
     if (c.status < 0) break;
-    cancelled = record(g, X, c, out + (int64_t)o * ne1, ket, B.cancel);
+    cancelled = record(g, X, c, out + (int64_t)o * ne1, ket, have, B.cancel);
   }
   if (g.rank == 0) {
     int32_t* st = B.status + 4 * (int64_t)item;
@@ -1265,7 +1445,7 @@ __global__ void __launch_bounds__(WARP_BLOCK, 4) batch_warp_kernel(qg_batch B) {
   if (slot < B.n_slots) {
     Ctx<DT> X;
     bind_slot(X, B, slot);
-    X.wf = wf_s[threadIdx.x >> 5];
+    X.wf = X.wf0 = wf_s[threadIdx.x >> 5];
     if (staged) use_staged(X, B, smem_op);
     if (in_bytes > 0)
       X.ytmp = reinterpret_cast<typename elem<DT>::T*>(
@@ -1298,6 +1478,7 @@ __global__ void __launch_bounds__(BB, 65536 / (BB * 128)) batch_cta_kernel(qg_ba
   Ctx<DT> X;
   bind_slot(X, B, blockIdx.x);
   X.wf = wf_s[threadIdx.x >> 5];
+  X.wf0 = wf_s[0];
   const int64_t in_bytes = stage_smem_bytes(B.max_n, DT, 1);
   if (in_bytes > 0) X.ytmp = reinterpret_cast<typename elem<DT>::T*>(stage_smem);
   unsigned char* smem_op = stage_smem + in_bytes;
@@ -1323,7 +1504,7 @@ __global__ void __launch_bounds__(BB, 65536 / (BB * 128)) batch_cta_kernel(qg_ba
 // One cluster of CLUSTER_CTAS CTAs per item; slot = cluster index.
 template <int DT>
 __global__ void __launch_bounds__(CTA_BLOCK, 1) batch_cluster_kernel(qg_batch B) {
-  __shared__ double red[2 * (CTA_BLOCK / 32)];
+  __shared__ double red[2 * (CTA_BLOCK / 32) + 2];
   __shared__ int ibuf;
   cgrp::cluster_group cl = cgrp::this_cluster();
   const int crank = (int)cl.block_rank();
@@ -1331,10 +1512,11 @@ __global__ void __launch_bounds__(CTA_BLOCK, 1) batch_cluster_kernel(qg_batch B)
   __shared__ __align__(16) float wf_s[CTA_BLOCK / 32][WF_FLOATS];
   __shared__ double rec[REC_SLOTS * 2 * (CTA_BLOCK / 32)];
   ClusterGroup<CTA_BLOCK, CLUSTER_CTAS> g{crank * CTA_BLOCK + (int)threadIdx.x, slot, red, &ibuf,
-                                          rec};
+                                          rec, 0};
   Ctx<DT> X;
   bind_slot(X, B, slot);
   X.wf = wf_s[threadIdx.x >> 5];
+  X.wf0 = wf_s[0];
   while (true) {
     int it = 0;
     if (g.rank == 0) {

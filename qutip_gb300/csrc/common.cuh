@@ -133,7 +133,8 @@ __device__ __forceinline__ double block_sum(double v, double* smem /* [BLOCK/32]
 // of atol + rtol |y| is below 1e-13 of atol).  Used by the mixed form, whose error estimate
 // carries complex64 rounding anyway; the complex128 form keeps IEEE sqrt and division so
 // that its step sequence and jump records are the reference's.
-__device__ __forceinline__ double wrms_term(double e2, double u, double atol, double rtol) {
+// (wrms_inv2 is the factor 1 / (atol + rtol sqrt(u))^2 alone.)
+__device__ __forceinline__ double wrms_inv2(double u, double atol, double rtol) {
   double mag = 0.0;
   if (u > 1e-30) {
     const double r0 = (double)rsqrtf((float)u);
@@ -143,7 +144,10 @@ __device__ __forceinline__ double wrms_term(double e2, double u, double atol, do
   const double sc = fma(rtol, mag, atol);
   const double i0 = (double)__frcp_rn((float)sc);
   const double i1 = i0 * fma(-sc, i0, 2.0);
-  return e2 * (i1 * i1);
+  return i1 * i1;
+}
+__device__ __forceinline__ double wrms_term(double e2, double u, double atol, double rtol) {
+  return e2 * wrms_inv2(u, atol, rtol);
 }
 
 // ---------------------------------------------------- coefficient programs --
