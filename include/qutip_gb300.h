@@ -330,6 +330,11 @@ int qg_vern7_stage(const qg_csr_groups* A, const qg_rk_buffers* B, int stage, do
 int qg_vern7_range(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0, int stage1,
                    double t_prev, double dt, double atol, double rtol, unsigned int* barrier,
                    uint32_t* barrier_base, void* stream);
+/* The same by half of a Hermitian d x d state: the rows and the conditions of
+ * qg_vern7_stage_herm. */
+int qg_vern7_range_herm(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0, int stage1,
+                        double t_prev, double dt, double atol, double rtol, int64_t d,
+                        unsigned int* barrier, uint32_t* barrier_base, void* stream);
 
 /* *flag = 1 (left alone otherwise) unless the dictionary-coded superoperator A maps
  * Hermitian d x d matrices to Hermitian ones, group by group (every entry of row (r, c) has

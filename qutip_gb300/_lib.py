@@ -121,6 +121,9 @@ _SIGS = {
     "qg_vern7_range": (C.c_int, [_P(CsrGroups), _P(RkBuffers), C.c_int, C.c_int, C.c_double,
                                  C.c_double, C.c_double, C.c_double, C.c_void_p,
                                  _P(C.c_uint32), C.c_void_p]),
+    "qg_vern7_range_herm": (C.c_int, [_P(CsrGroups), _P(RkBuffers), C.c_int, C.c_int, C.c_double,
+                                      C.c_double, C.c_double, C.c_double, C.c_int64, C.c_void_p,
+                                      _P(C.c_uint32), C.c_void_p]),
     "qg_hermitian_check": (C.c_int, [_P(CsrGroups), C.c_int64, C.c_void_p, C.c_int, C.c_void_p,
                                      C.c_void_p]),
     "qg_vern7_stage_herm": (C.c_int, [_P(CsrGroups), C.c_int64, _P(RkBuffers), C.c_int,

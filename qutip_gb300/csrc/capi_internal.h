@@ -13,6 +13,8 @@ int check_launch(const char* what);
 int sm_count();
 // Validate a grouped operator (shape, layout and tables); QG_OK or an error code.
 int check_groups(const qg_csr_groups* A);
+// The same for an operator of the Hermitian half form on d x d states.
+int check_herm(const qg_csr_groups* A, int64_t d);
 }  // namespace qg
 
 // The fault flag of the fused step kernel's barrier waits, read and cleared (for

@@ -46,8 +46,13 @@ struct Drive {
   // stages [s0, s1): 0 when they went out in one launch, 1 when they do not fit one
   int range(int s0, int s1, double dt) {
     if (gen->kind != QG_GEN_CSR) return 1;
-    const int rc = qg_vern7_range(static_cast<const qg_csr_groups*>(gen->op), B, s0, s1, c->t_prev,
-                                  dt, c->atol, c->rtol, c->barrier, &c->barrier_base, stream);
+    const auto* A = static_cast<const qg_csr_groups*>(gen->op);
+    const int rc =
+        gen->hermitian_d > 0
+            ? qg_vern7_range_herm(A, B, s0, s1, c->t_prev, dt, c->atol, c->rtol, gen->hermitian_d,
+                                  c->barrier, &c->barrier_base, stream)
+            : qg_vern7_range(A, B, s0, s1, c->t_prev, dt, c->atol, c->rtol, c->barrier,
+                             &c->barrier_base, stream);
     if (rc == 0) ++c->launches;
     return rc;
   }

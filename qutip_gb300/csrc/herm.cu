@@ -293,7 +293,7 @@ static int launch_check(cudaStream_t st, const qg_csr_groups& A, int d, const vo
 
 // The layouts and shapes the half form takes: dictionary codes (split in complex128), a
 // Hilbert dimension that is a multiple of 32.
-static int check_herm(const qg_csr_groups* A, int64_t d) {
+int check_herm(const qg_csr_groups* A, int64_t d) {
   int rc = check_groups(A);
   if (rc) return rc;
   if (A->layout != (A->dtype == QG_C128 ? QG_LAYOUT_SLICED_DICT_RI : QG_LAYOUT_SLICED_DICT))

@@ -8,11 +8,20 @@
 // 21.6 us per right-hand side at 65,536 rows, whose FP64 work takes 6.4 us.  Here the
 // stages follow one another behind a grid barrier; a row keeps its operator entries (or
 // codes), its k_j and its state in shared memory and registers for the whole launch, and
-// only the stage input crosses between SMs.  Measured, whole complex128 solves: the L = 8
-// Ising chain (65,536 rows) 39.1 -> 27.9 ms (12 us a stage), the d = 125 Bose-Hubbard trimer
-// (15,625 rows, odd) 9.8 -> 6.2 ms.  An operator with more rows than the GPU has resident
-// threads at 512 a block keeps one launch a stage: there a stage is 40 us and more, and the
-// launches no longer count.
+// only the stage input crosses between SMs.
+//
+// Complex128 rows are bound by FP64 issue once the launches are gone: an FP64 instruction holds
+// its SM for 16 clocks however few lanes it has, so a row goes to fewer threads than the
+// matvec kernel's sub-warp and a coefficient that is one is not multiplied.  A Hermitian
+// density matrix (herm_d) is evaluated by half as in herm.cu, 8 warps to a unit of 32 rows x
+// 8 columns on or below the diagonal: the L = 8 Ising chain puts 8 warps on an SM that way
+// instead of 14.
+//
+// Measured, whole complex128 solves: the L = 8 Ising chain (65,536 rows) 39.1 -> 27.9 ms in
+// one launch a step, and 24.9 -> 21.5 ms by half; the d = 125 Bose-Hubbard trimer (15,625
+// rows, odd) 9.8 -> 6.2 ms.  An operator with more rows than the GPU has resident threads at
+// 512 a block keeps one launch a stage: there a stage is 40 us and more, and the launches no
+// longer count.
 //
 // The launch is cooperative (all blocks resident), and every wait at the barrier is bounded:
 // a wait that gives up sets *result to -1 and every block leaves.  A row's sum and its
@@ -21,6 +30,7 @@
 
 #include "capi_internal.h"
 #include "common.cuh"
+#include "herm.cuh"
 #include "rows.cuh"
 #include "stage.cuh"
 
@@ -33,7 +43,8 @@ constexpr int STEP_THREADS = 512;   // most threads of a block (one block per SM
 constexpr int STEP_MIN_WARPS = 4;   // fewer warps per block only spread the barrier wider
 // entries (CSR, sliced) or code words a thread keeps in shared memory; rows longer than
 // that read the rest from global memory at every stage
-constexpr int STEP_KEEP = 8;
+constexpr int STEP_KEEP = 32;
+constexpr int HERM_WARPS = 8;       // a unit of the half form: 32 rows x 8 columns
 constexpr long long STEP_WAIT_CYCLES = 16 * WAIT_CYCLES;  // the GPU may be shared meanwhile
 
 struct StepArgs {
@@ -44,6 +55,7 @@ struct StepArgs {
   double t_prev, dt;
   int s0, s1;          // stages [s0, s1)
   int keep;            // entries or code words kept per thread
+  int herm_d;          // > 0: half form of a Hermitian d x d state (HERM instantiations)
   unsigned int* bar;   // arrivals of every earlier launch and of this one
   unsigned int bar_base;
 };
@@ -52,11 +64,11 @@ __device__ unsigned int g_step_fault = 0u;
 
 // Shared memory of a block, in bytes from its start (every part 16-byte aligned).
 struct StepSmem {
-  int tval, toff, k, val, idx, rp, total;
+  int tval, toff, k, val, idx, rp, tile, total;
 };
 template <typename ST>
 __host__ __device__ inline StepSmem step_smem(const qg_csr_groups& A, int kind, int threads,
-                                              int rows, int keep) {
+                                              int rows, int keep, bool herm) {
   const int D = kind >= KIND_DICT1 ? A.lanes : 0;
   auto up = [](size_t b) { return (int)((b + 15) & ~(size_t)15); };
   StepSmem L;
@@ -68,7 +80,9 @@ __host__ __device__ inline StepSmem step_smem(const qg_csr_groups& A, int kind, 
   const int ib = kind == KIND_DICT2 ? 8 : 4;
   L.idx = L.val + up((size_t)threads * keep * vb);
   L.rp = L.idx + up((size_t)threads * keep * ib);
-  L.total = L.rp + up((size_t)rows * (kind == KIND_CSR ? A.n_groups + 1 : 2 * A.n_groups) * 4);
+  L.tile = L.rp + up((size_t)rows * (kind == KIND_CSR ? A.n_groups + 1 : 2 * A.n_groups) * 4);
+  // half form: the conjugates of a unit's k and of its stage input or y_front
+  L.total = L.tile + (herm ? (threads / 32) * 2 * HERM_PAD<double2> * 16 : 0);
   return L;
 }
 
@@ -98,7 +112,9 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int tar
   return *ok_s;
 }
 
-template <int DT, int YDT, int KIND, int LANES>
+// LANES: threads of a row.  PARTS: sums of each thread (CSR); entry p goes to lane
+// p % (LANES * PARTS) and the lanes are added pairwise, as in the matvec kernel.
+template <int DT, int YDT, int KIND, int LANES, int PARTS, bool HERM>
 __global__ void __launch_bounds__(STEP_THREADS, 1)
     vern7_range_kernel(const __grid_constant__ StepArgs a) {
   using ST = typename elem<DT>::T;
@@ -125,9 +141,27 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
   const int tid = threadIdx.x, threads = blockDim.x;
   const int rows = threads / LANES;
   const int lrow = tid / LANES, lane = tid % LANES;
-  const int row = blockIdx.x * rows + lrow;
-  const bool valid = row < n;
-  const StepSmem L = step_smem<ST>(A, KIND, threads, rows, a.keep);
+  int row = blockIdx.x * rows + lrow;
+  bool valid = row < n;
+  bool mirrored = false;
+  int mirror = 0;  // element this thread writes the conjugate of (half form)
+  if constexpr (HERM) {
+    const int d = a.herm_d, nt = d >> 5;
+    const int u = blockIdx.x * (threads / (32 * HERM_WARPS)) + (tid >> 5) / HERM_WARPS;
+    valid = u < 2 * nt * (nt + 1);
+    int tj = 0, tau = valid ? u >> 2 : 0;
+    while (tau >= nt - tj) {
+      tau -= nt - tj;
+      ++tj;
+    }
+    const int ti = tj + tau, c0 = tj * 32 + (u & 3) * HERM_WARPS;
+    row = ((c0 + ((tid >> 5) % HERM_WARPS)) * nt + ti) * 32 + (tid & 31);
+    if (!valid) row = tid & 31;
+    mirrored = valid && ti != tj;
+    const int e = tid % (32 * HERM_WARPS);
+    mirror = (c0 + e % HERM_WARPS) + (ti * 32 + e / HERM_WARPS) * d;
+  }
+  const StepSmem L = step_smem<ST>(A, KIND, threads, rows, a.keep, HERM);
   ST* tval = reinterpret_cast<ST*>(smem + L.tval);
   int* toff = reinterpret_cast<int*>(smem + L.toff);
   ST* ksm = reinterpret_cast<ST*>(smem + L.k) + lrow;  // k_j of this row at ksm[j * rows]
@@ -135,6 +169,14 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
   int* csm = reinterpret_cast<int*>(smem + L.idx) + tid;
   C4* wsm = reinterpret_cast<C4*>(smem + L.idx) + tid;
   int* rpsm = reinterpret_cast<int*>(smem + L.rp) + lrow;  // row bounds, [g * rows]
+  // half form: tiles of this thread's unit; its own place and the one it mirrors from
+  ST* tk = reinterpret_cast<ST*>(smem + L.tile);
+  YT* ty = reinterpret_cast<YT*>(smem + L.tile + (threads / 32) * HERM_PAD<double2> * 16);
+  ST* tv = reinterpret_cast<ST*>(ty);
+  constexpr int PAD = HERM_PAD<ST>, YPAD = HERM_PAD<YT>;
+  const int unit0 = (tid >> 5) / HERM_WARPS * HERM_WARPS;  // first warp (tile column) of the unit
+  const int t_own = (tid >> 5), t_from = unit0 + tid % HERM_WARPS,
+            l_from = tid % (32 * HERM_WARPS) / HERM_WARPS;
 
   // ---- once per launch: factors, coefficients, the row's operator data ----
   for (int e = tid; e < (a.s1 - a.s0) * G; e += threads) {
@@ -231,10 +273,20 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
     const unsigned int nz = nz_s[s];
     for (int j = 0; j <= s; ++j)
       if ((nz >> j) & 1u) cx_axpy(v, fac[s][j], ld_cx<R>(ksm + j * rows));
-    st_cx(ytmp + (size_t)((s + 1) & 1) * n64 + row, v);
+    ST q;
+    st_cx(&q, v);
+    ytmp[(size_t)((s + 1) & 1) * n64 + row] = q;
+    if constexpr (HERM) tv[t_own * PAD + (tid & 31)] = ST{q.x, -q.y};
+  };
+  auto mirror_input = [&](int s) {  // after a barrier that follows form_input
+    if (mirrored) ytmp[(size_t)((s + 1) & 1) * n64 + mirror] = tv[t_from * PAD + l_from];
   };
   if (a.s0 > 0) {  // the first stage's input (stages 10..15 follow an accepted step)
     if (owner) form_input(a.s0 - 1);
+    if constexpr (HERM) {
+      __syncthreads();
+      mirror_input(a.s0 - 1);
+    }
     target += gridDim.x;
     ok = grid_barrier(a.bar, target, &ok_s);
   }
@@ -250,20 +302,37 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
       int ps = rpsm[0];
       for (int g = 0; g < G; ++g) {
         const int pe = rpsm[(g + 1) * rows];
-        R ar = 0, ai = 0;
-        for (int p = ps + lane; p < pe; p += LANES, ++i) {
-          ST v;
-          int c;
-          if (i < a.keep) {
-            v = vsm[i * threads];
-            c = csm[i * threads];
-          } else {
-            v = __ldg(gval + p);
-            c = __ldg(gcol + p);
+        const int i0 = i;
+        R ar[PARTS] = {}, ai[PARTS] = {};
+        for (int p = ps + lane; p < pe; p += LANES * PARTS, i += PARTS) {
+          ST v[PARTS], xv[PARTS];
+#pragma unroll
+          for (int l = 0; l < PARTS; ++l) {
+            if (p + l * LANES >= pe) break;
+            int c;
+            if (i + l < a.keep) {
+              v[l] = vsm[(i + l) * threads];
+              c = csm[(i + l) * threads];
+            } else {
+              v[l] = __ldg(gval + p + l * LANES);
+              c = __ldg(gcol + p + l * LANES);
+            }
+            xv[l] = x[c];
           }
-          cmac_any(ar, ai, v, x[c]);
+#pragma unroll
+          for (int l = 0; l < PARTS; ++l)
+            if (p + l * LANES < pe) cmac_any(ar[l], ai[l], v[l], xv[l]);
         }
-        acc = cx_add(acc, cx_mul(coef[s][g], sub_reduce<LANES>(ar, ai)));
+        i = i0 + (pe - ps - lane + LANES - 1) / LANES;  // this thread's entries so far
+#pragma unroll
+        for (int o = PARTS / 2; o > 0; o >>= 1)
+          for (int l = 0; l < o; ++l) {
+            ar[l] += ar[l + o];
+            ai[l] += ai[l + o];
+          }
+        const cx<R> sum = sub_reduce<LANES>(ar[0], ai[0]);
+        if (sizeof(R) == 8 && ccls[s][g] == 0) acc = cx_add(acc, sum);
+        else acc = cx_add(acc, cx_mul(coef[s][g], sum));
         ps = pe;
       }
     } else if constexpr (KIND == KIND_SLICED) {
@@ -318,7 +387,9 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
     }
     if (owner) {
       st_cx(ksm + s * rows, acc);
-      kg[(size_t)s * n64] = ksm[s * rows];
+      const ST kq = ksm[s * rows];
+      kg[(size_t)s * n64] = kq;
+      if constexpr (HERM) tk[t_own * PAD + (tid & 31)] = ST{kq.x, -kq.y};
       if (s == RK_STEP - 1) {
         const unsigned int nz = nz_s[s], ne = nz_s[RK_EXTRA_STEP];
         if constexpr (MIXED) {
@@ -336,6 +407,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
           const double2 yf = make_double2(yp.x + (double)inc.re, yp.y + (double)inc.im);
           static_cast<double2*>(rk.y_front)[row] = yf;
           static_cast<float2*>(rk.y_front_s)[row] = make_float2((float)yf.x, (float)yf.y);
+          if constexpr (HERM) ty[t_own * YPAD + (tid & 31)] = make_double2(yf.x, -yf.y);
           const double er = (double)erh + (double)erl, ei = (double)eih + (double)eil;
           err_acc = wrms_term(er * er + ei * ei, yf.x * yf.x + yf.y * yf.y, rk.atol, rk.rtol);
         } else {
@@ -348,6 +420,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
           YT yq;
           st_cx(&yq, y);
           static_cast<YT*>(rk.y_front)[row] = yq;
+          if constexpr (HERM) ty[t_own * YPAD + (tid & 31)] = YT{yq.x, -yq.y};
           const cx<R> ys = ld_cx<R>(&yq);
           const double mag2 = (double)ys.re * ys.re + (double)ys.im * ys.im;
           const double sc = rk.atol + rk.rtol * sqrt(mag2);
@@ -355,6 +428,17 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
         }
       } else if (s + 1 < a.s1) {
         form_input(s);
+      }
+      if constexpr (HERM) {
+        if (mirrored) err_acc *= 2.0;  // the mirrored element has the same term
+      }
+    }
+    if constexpr (HERM) {
+      __syncthreads();
+      if (mirrored) {
+        static_cast<ST*>(rk.k)[(size_t)s * n64 + mirror] = tk[t_from * PAD + l_from];
+        if (s == RK_STEP - 1) herm_mirror_front<DT, YDT>(mirror, ty[t_from * YPAD + l_from], rk);
+        else if (s + 1 < a.s1) mirror_input(s);
       }
     }
     if (s + 1 < a.s1) {
@@ -400,24 +484,28 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
 constexpr int STEP_MAX_SMEM = 220 * 1024;
 
 // 1 when the launch does not fit (the caller then takes one launch per stage).
-template <int DT, int YDT, int KIND, int LANES>
+template <int DT, int YDT, int KIND, int LANES, int PARTS = 1, bool HERM = false>
 static int launch_range(StepArgs& a, uint32_t* bar_base, cudaStream_t st) {
   using ST = typename elem<DT>::T;
-  const int64_t warps = (a.A.n_rows * LANES + 31) / 32;
   const int64_t sms = sm_count();
+  int64_t warps = (a.A.n_rows * LANES + 31) / 32;
+  if (HERM) {
+    const int64_t nt = a.herm_d / 32;
+    warps = 2 * nt * (nt + 1) * HERM_WARPS;
+  }
   int64_t per = (warps + sms - 1) / sms;  // warps of a block, one block per SM
   if (per < STEP_MIN_WARPS) per = STEP_MIN_WARPS;
+  if (HERM) per = (per + HERM_WARPS - 1) / HERM_WARPS * HERM_WARPS;
   if (per * 32 > STEP_THREADS) return 1;
   const int threads = (int)per * 32, rows = threads / LANES;
   const int grid = (int)((warps + per - 1) / per);
-  a.keep = STEP_KEEP;
-  int smem = step_smem<ST>(a.A, KIND, threads, rows, a.keep).total;
-  if (smem > STEP_MAX_SMEM) {
-    a.keep = 2;
-    smem = step_smem<ST>(a.A, KIND, threads, rows, a.keep).total;
-    if (smem > STEP_MAX_SMEM) return 1;
+  int smem = 0;
+  for (a.keep = STEP_KEEP; a.keep >= 2; a.keep /= 2) {
+    smem = step_smem<ST>(a.A, KIND, threads, rows, a.keep, HERM).total;
+    if (smem <= STEP_MAX_SMEM) break;
   }
-  auto kern = vern7_range_kernel<DT, YDT, KIND, LANES>;
+  if (smem > STEP_MAX_SMEM) return 1;
+  auto kern = vern7_range_kernel<DT, YDT, KIND, LANES, PARTS, HERM>;
   static std::mutex mu;
   static bool opted[64] = {};
   int dev = 0;
@@ -442,25 +530,36 @@ static int launch_range(StepArgs& a, uint32_t* bar_base, cudaStream_t st) {
   return check_launch("vern7_range_kernel");
 }
 
+template <int DT, int YDT, int KIND>
+static int launch_range_dict(StepArgs& a, uint32_t* bar_base, cudaStream_t st) {
+  return a.herm_d > 0 ? launch_range<DT, YDT, KIND, 1, 1, true>(a, bar_base, st)
+                      : launch_range<DT, YDT, KIND, 1>(a, bar_base, st);
+}
+
 template <int DT, int YDT>
 static int launch_range_layout(StepArgs& a, uint32_t* bar_base, cudaStream_t st) {
   const qg_csr_groups& A = a.A;
   switch (A.layout) {
     case QG_LAYOUT_ROW_MAJOR:
+      // Four lanes as two threads of two sums each: half the FP64 instructions of the
+      // coefficients and the stage combination, where one thread of four sums leaves too few
+      // warps to hide the gathers (Bose-Hubbard, d = 125: 4 x 1 5.05 ms a solve, 2 x 2
+      // 4.48, 1 x 4 5.57).
       switch (A.lanes) {
         case 2: return launch_range<DT, YDT, KIND_CSR, 2>(a, bar_base, st);
-        case 4: return launch_range<DT, YDT, KIND_CSR, 4>(a, bar_base, st);
+        case 4: return launch_range<DT, YDT, KIND_CSR, 2, 2>(a, bar_base, st);
         case 8: return launch_range<DT, YDT, KIND_CSR, 8>(a, bar_base, st);
         default: return 1;
       }
     case QG_LAYOUT_SLICED: return launch_range<DT, YDT, KIND_SLICED, 1>(a, bar_base, st);
     case QG_LAYOUT_SLICED_DICT:
-      if (DT == QG_C128) return 1;  // complex128 dictionaries are split
-      return A.tile_nnz == 1 ? launch_range<DT, YDT, KIND_DICT1, 1>(a, bar_base, st)
-                             : launch_range<DT, YDT, KIND_DICT2, 1>(a, bar_base, st);
+      if constexpr (DT == QG_C128) return 1;  // complex128 dictionaries are split
+      return A.tile_nnz == 1 ? launch_range_dict<DT, YDT, KIND_DICT1>(a, bar_base, st)
+                             : launch_range_dict<DT, YDT, KIND_DICT2>(a, bar_base, st);
     case QG_LAYOUT_SLICED_DICT_RI:
-      return A.tile_nnz == 1 ? launch_range<DT, YDT, KIND_DICT1, 1>(a, bar_base, st)
-                             : launch_range<DT, YDT, KIND_DICT2, 1>(a, bar_base, st);
+      if constexpr (DT != QG_C128) return 1;
+      return A.tile_nnz == 1 ? launch_range_dict<DT, YDT, KIND_DICT1>(a, bar_base, st)
+                             : launch_range_dict<DT, YDT, KIND_DICT2>(a, bar_base, st);
     default: return 1;
   }
 }
@@ -476,19 +575,18 @@ int step_fault_take() {
   return (int)v;
 }
 
-extern "C" int qg_vern7_range(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0,
-                              int stage1, double t_prev, double dt, double atol, double rtol,
-                              unsigned int* barrier, uint32_t* barrier_base, void* stream) {
-  int rc = check_groups(A);
-  if (rc) return rc;
+// d > 0: the half form of a d x d state; A has been checked.
+static int vern7_range(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0, int stage1,
+                       double t_prev, double dt, double atol, double rtol, int64_t d,
+                       unsigned int* barrier, uint32_t* barrier_base, void* stream) {
   if (!barrier || !barrier_base) return set_error(QG_ERR_ARG, "null barrier word");
   if (A->n_rows != A->n_cols) return set_error(QG_ERR_ARG, "operator must be square with n rows");
   if (!((stage0 == 0 && stage1 == RK_STEP) || (stage0 == RK_STEP && stage1 == RK_EXTRA_STEP)))
     return set_error(QG_ERR_ARG, "stages must be a whole trial step or the dense-output stages");
   StepArgs a{};
   const void* x = nullptr;
-  rc = prepare_stage(B, A->dtype, A->n_rows, stage0 == 0 ? RK_STEP - 1 : stage0, dt, atol, rtol,
-                     a.rk, x);
+  const int rc = prepare_stage(B, A->dtype, A->n_rows, stage0 == 0 ? RK_STEP - 1 : stage0, dt, atol,
+                               rtol, a.rk, x);
   if (rc) return rc;
   if (B->n == 0) return 1;
   a.A = *A;
@@ -499,9 +597,27 @@ extern "C" int qg_vern7_range(const qg_csr_groups* A, const qg_rk_buffers* B, in
   a.s0 = stage0;
   a.s1 = stage1;
   a.bar = barrier;
+  a.herm_d = (int)d;
   cudaStream_t st = (cudaStream_t)stream;
   if (B->state_dtype == QG_C128 && B->stage_dtype == QG_C128)
     return launch_range_layout<QG_C128, QG_C128>(a, barrier_base, st);
   if (B->state_dtype == QG_C128) return launch_range_layout<QG_C64, QG_C128>(a, barrier_base, st);
   return launch_range_layout<QG_C64, QG_C64>(a, barrier_base, st);
+}
+
+extern "C" int qg_vern7_range(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0,
+                              int stage1, double t_prev, double dt, double atol, double rtol,
+                              unsigned int* barrier, uint32_t* barrier_base, void* stream) {
+  const int rc = check_groups(A);
+  return rc ? rc : vern7_range(A, B, stage0, stage1, t_prev, dt, atol, rtol, 0, barrier,
+                               barrier_base, stream);
+}
+
+extern "C" int qg_vern7_range_herm(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0,
+                                   int stage1, double t_prev, double dt, double atol, double rtol,
+                                   int64_t d, unsigned int* barrier, uint32_t* barrier_base,
+                                   void* stream) {
+  const int rc = check_herm(A, d);
+  return rc ? rc : vern7_range(A, B, stage0, stage1, t_prev, dt, atol, rtol, d, barrier,
+                               barrier_base, stream);
 }

@@ -681,14 +681,15 @@ class DeviceOperator:
     # -- Hermitian half form ------------------------------------------------
     def hermitian_dim(self) -> int:
         """The Hilbert dimension d when this operator can act on a Hermitian d x d state by
-        half (dictionary-coded d*d x d*d storage, d a multiple of 32, and enough rows that
-        the stages go out one by one: more than 512 per SM), else 0."""
+        half (dictionary-coded d*d x d*d storage, d a multiple of 32) and that pays: above
+        256 rows per SM, where the half form's blocks of 8 warps leave an SM fewer rows than
+        all of them spread evenly; else 0."""
         split = getattr(self, "dict_split", False)
         if self.fmt != "dict" or self.n_rows != self.n_cols or split != (self.dtype == "c128"):
             return 0
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         d = math.isqrt(self.n_rows)
-        return d if d * d == self.n_rows and d % 32 == 0 and self.n_rows > 512 * sms else 0
+        return d if d * d == self.n_rows and d % 32 == 0 and self.n_rows > 256 * sms else 0
 
     def real_coefficients(self) -> bool:
         """Whether every group's coefficient is real at every t."""
@@ -721,6 +722,17 @@ class DeviceOperator:
         if rc == 1:
             return False
         _lib.check(rc, "qg_vern7_range")
+        return True
+
+    def vern7_range_herm(self, rk, stage0: int, stage1: int, t_prev: float, dt: float,
+                         atol: float, rtol: float, barrier: int, base, stream: int) -> bool:
+        """:meth:`vern7_range` by half, for states :meth:`check_hermitian` found Hermitian."""
+        rc = _lib.load().qg_vern7_range_herm(C.byref(self.struct), C.byref(rk), stage0, stage1,
+                                             t_prev, dt, atol, rtol, math.isqrt(self.n_rows),
+                                             barrier, C.byref(base), stream)
+        if rc == 1:
+            return False
+        _lib.check(rc, "qg_vern7_range_herm")
         return True
 
     def matmat(self, t: float, X: torch.Tensor, Y: torch.Tensor, alpha=1.0, beta=0.0):

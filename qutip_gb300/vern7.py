@@ -275,9 +275,8 @@ class GpuVern7:
                 DenseLindbladOperator: _lib.QG_GEN_DENSE}.get(type(self.op))
         if kind is None:
             return None
-        half = self._hermitian and self.op.real_coefficients()
         return _lib.Generator(kind, 0, C.addressof(self.op.struct),
-                              math.isqrt(self.n) if half else 0)
+                              math.isqrt(self.n) if self._half() else 0)
 
     def _drive(self, name, gen, *args):
         """Call a driver of the library on this integrator's buffers and scalar state."""
@@ -359,16 +358,19 @@ class GpuVern7:
         return error
 
     def _stage(self):
-        """The operator's stage launch: by half when the state is a Hermitian density matrix
-        that the generator keeps Hermitian (the coefficients may have been replaced since
-        the state was set, so their part is looked at again)."""
-        if self._hermitian and self.op.real_coefficients():
-            return self.op.vern7_stage_herm
-        return self.op.vern7_stage
+        """The operator's stage launch, by half where that applies."""
+        return self.op.vern7_stage_herm if self._half() else self.op.vern7_stage
+
+    def _half(self) -> bool:
+        """Whether the state is a Hermitian density matrix that the generator keeps Hermitian
+        (the coefficients may have been replaced since the state was set, so their part is
+        looked at again)."""
+        return self._hermitian and self.op.real_coefficients()
 
     def _range(self, rk, stage0, stage1, dt, s) -> bool:
         """The stages in one launch where the operator's rows all fit the GPU at once."""
-        run = getattr(self.op, "vern7_range", None)
+        name = "vern7_range_herm" if self._half() else "vern7_range"
+        run = getattr(self.op, name, None)
         return run is not None and run(rk, stage0, stage1, self.t_prev, dt, self.atol, self.rtol,
                                        self.counter.data_ptr() + 4, self._barrier_base, s)
 

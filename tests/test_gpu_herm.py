@@ -77,6 +77,35 @@ def test_half_form_matches_the_full_stages(d, precision):
     assert torch.equal(k[:, off], k.transpose(1, 2).conj()[:, off])   # mirrored bit for bit
 
 
+@pytest.mark.parametrize("precision", ["double", "mixed", "single"])
+@pytest.mark.parametrize("d", [32, 96, 256, 352])
+def test_fused_half_form_matches_the_full_stages(d, precision):
+    """The half form inside the fused step: one block, several, one unit of 8 warps per SM and
+    two.  Bounds as above."""
+    from qutip_gb300.vern7 import GpuVern7
+    op = _operator(*_operators(d, d), "cos(1.3*t)", "c128" if precision == "double" else "c64")
+    y0 = _rho(d, d)
+    half, full = (GpuVern7(op, precision=precision, first_step=0.01) for _ in range(2))
+    op.hermitian_dim = lambda: d
+    run, calls, errors = op.vern7_range_herm, [], []
+    op.vern7_range_herm = lambda *a: calls.append(run(*a)) or calls[-1]
+    full._range = lambda *a: False
+    for ig, h in ((half, True), (full, False)):
+        ig.set_initial_value(y0, 0.2)
+        assert ig._hermitian
+        ig._hermitian = h
+        ig.t_prev = 0.2
+        errors.append([ig._compute_step(dt) for dt in (0.01, 0.03)])
+        ig.dt_int = 0.03
+        ig._prep_dense_out()
+    assert calls == [True] * 3
+    eps = 2.3e-16 if precision == "double" else 1.2e-7
+    for a, b in ((half.k, full.k), (half.y_front, full.y_front)):
+        assert float((a - b).abs().max()) <= 100 * eps * float(b.abs().max())
+    move = 0.03 * np.abs(T.E).sum() * 100 * eps * float(full.k.abs().max()) / full.atol
+    np.testing.assert_allclose(errors[0], errors[1], rtol=0, atol=move)
+
+
 @pytest.mark.parametrize("dtype", ["c128", "c64"])
 @pytest.mark.parametrize("case", ["ok", "rho", "rho_nan", "h", "c_coef"])
 def test_what_the_check_accepts(case, dtype):
