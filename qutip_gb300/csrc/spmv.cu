@@ -329,8 +329,24 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, UNR>::MIN_BLOCKS)
 // in the driven group, about 700 in the constant one), so the operator stream shrinks
 // from 12 bytes per entry (complex64 value, int32 column) to 1-2 bytes, and a stage is
 // bound by the shared-memory lookups and the L2 gathers of x instead of by HBM.
+//
+// One block of 32 warps per SM, so that an SM stages the tables and evaluates the
+// coefficients once (eight blocks did it side by side on one FP64 pipe), and the
+// evaluation runs beside the first sums, which do not need it.  At 64 registers a
+// complex64 warp has enough gathers in flight that 32 of them do as well as 48 at 40
+// registers (two blocks of 768 threads: 13.7 us at L = 9, this 11.5).  Measured, one
+// application with a driven group, 256 threads a block and the coefficients first ->
+// now: complex64 L = 8 8.4 -> 5.9 us, L = 9 13.6 -> 11.5, L = 10 34.0 -> 34.3; complex128
+// 14.2 -> 11.4, 42.5 -> 35.9 (FP64 issue alone 21), 151 -> 139.
+constexpr int DICT_BLOCK = 1024;
+
+// Barrier of `threads` threads of the block.
+__device__ __forceinline__ void named_barrier(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 template <int DT, int YDT, int EPI, int CB, bool RI>
-__global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, 4>::MIN_BLOCKS)
+__global__ void __launch_bounds__(DICT_BLOCK, 1)
     spmv_dict_kernel(qg_csr_groups A, double t, const typename elem<DT>::T* __restrict__ x,
                      AxpbyArgs ax, RkArgs rk) {
   using ST = typename elem<DT>::T;
@@ -340,44 +356,74 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, 4>::MIN_BLOCKS)
   __shared__ cx<R> coef[QG_MAX_GROUPS];
   __shared__ int ccls[QG_MAX_GROUPS];
   __shared__ int tstart[QG_MAX_GROUPS + 1];
-  __shared__ double red[SPMV_BLOCK / 32];
-  const int D = A.lanes;
+  __shared__ double red[DICT_BLOCK / 32];
+  const int D = A.lanes, G = A.n_groups;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   ST* tval = reinterpret_cast<ST*>(dict_smem);
   int* toff = reinterpret_cast<int*>(dict_smem + (size_t)D * sizeof(ST));
-  load_coefs(A, t, coef);
-  coef_classes(A, coef, ccls);
-  for (int i = threadIdx.x; i < D; i += SPMV_BLOCK) {
-    tval[i] = __ldg(static_cast<const ST*>(A.val) + i);
-    toff[i] = __ldg(A.dict_off + i);
+  // The last warp evaluates the coefficients, a few microseconds of dependent FP64 work, while
+  // the others stage the tables and form their first sums; it takes no slice of the first round.
+  const int workers = nwarps - 1;
+  const bool evaluator = warp == workers;
+  if (evaluator) {
+    if (lane < G) {
+      const cplx c = group_coef(A, lane, t);
+      coef[lane] = cx<R>{(R)c.re, (R)c.im};
+      ccls[lane] = coef_class(coef[lane]);
+    }
+    named_barrier(1, blockDim.x);
+  } else {
+    for (int i = threadIdx.x; i < D; i += workers * 32) {
+      tval[i] = __ldg(static_cast<const ST*>(A.val) + i);
+      toff[i] = __ldg(A.dict_off + i);
+    }
+    if ((int)threadIdx.x <= G) tstart[threadIdx.x] = __ldg(A.dict_start + threadIdx.x);
+    named_barrier(2, workers * 32);
   }
-  if (threadIdx.x <= (unsigned)A.n_groups) tstart[threadIdx.x] = __ldg(A.dict_start + threadIdx.x);
-  __syncthreads();
-  const int G = A.n_groups;
+  bool ready = evaluator;  // the coefficients are there
   const int n = (int)A.n_rows;
   const int S = A.n_tiles;
   const int last_col = (int)A.n_cols - 1;
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * SPMV_BLOCK + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * SPMV_BLOCK) >> 5;
   const unsigned char* __restrict__ codes = reinterpret_cast<const unsigned char*>(A.col);
   double err_acc = 0.0;
-  for (int sl = warp; sl < S; sl += nwarps) {
+  // Few slices to a warp: each block an even run of them.  Many: all blocks move through the
+  // rows together, which keeps what they gather closer in the L2.
+  const int first = (int)gridDim.x * workers, all = (int)gridDim.x * nwarps;
+  const bool runs = S <= 2 * all;
+  const int run0 = (int)((int64_t)S * blockIdx.x / gridDim.x);
+  const int s_end = runs ? (int)((int64_t)S * (blockIdx.x + 1) / gridDim.x) : S;
+  const int head = runs ? run0 + workers : first;               // end of the first round
+  const int next0 = runs ? head + warp : first + blockIdx.x * nwarps + warp;
+  int sl = evaluator ? next0 : runs ? run0 + warp : blockIdx.x * workers + warp;
+  for (; sl < s_end; sl = sl < head ? next0 : sl + (runs ? nwarps : all)) {
     const int row = sl * 32 + lane;
     cx<R> acc{0, 0};
+    int w_next = __ldg(A.tile_row + sl * G), p_next = __ldg(A.row_ptr + sl);
     for (int g = 0; g < G; ++g) {
       // exact width (uniform over the warp): whole chunks of four codes, then a tail
-      const int w = __ldg(A.tile_row + sl * G + g);
+      const int w = w_next, p0 = p_next;
+      if (g + 1 < G) {
+        w_next = __ldg(A.tile_row + sl * G + g + 1);
+        p_next = __ldg(A.row_ptr + (g + 1) * (S + 1) + sl);
+      }
       const int wq = w >> 2, wr = w & 3;
       const int t0 = tstart[g], tn = tstart[g + 1] - t0;
       const C4* __restrict__ cp =
-          reinterpret_cast<const C4*>(codes + (size_t)CB * __ldg(A.row_ptr + g * (S + 1) + sl)) +
-          lane;
+          reinterpret_cast<const C4*>(codes + (size_t)CB * p0) + lane;
       // FP64: a group whose coefficient is one accumulates into the row's sum directly
-      const bool direct = sizeof(R) == 8 && ccls[g] == 0;
+      // (the first group's sum starts from zero either way)
+      bool direct = sizeof(R) == 8 && g > 0 && ccls[g] == 0;
       R ar = direct ? acc.re : (R)0, ai = direct ? acc.im : (R)0;
+      // FP64: the next chunk of codes is on its way while the current one is looked up
+      // (complex64 keeps the registers for gathers: 34.3 against 35.1 us at L = 10)
+      constexpr bool AHEAD = sizeof(R) == 8;
+      const int wc = wq + (wr != 0);
+      C4 next{};
+      if (AHEAD && wc) next = ld_stream(cp);
 #pragma unroll 2
       for (int q = 0; q < wq; ++q) {
-        const C4 c4 = ld_stream(cp + 32 * q);
+        const C4 c4 = AHEAD ? next : ld_stream(cp + 32 * q);
+        if (AHEAD && q + 1 < wc) next = ld_stream(cp + 32 * (q + 1));
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           int k = Codes4<CB>::at(c4, u);
@@ -389,7 +435,7 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, 4>::MIN_BLOCKS)
         }
       }
       if (wr) {
-        const C4 c4 = ld_stream(cp + 32 * wq);
+        const C4 c4 = AHEAD ? next : ld_stream(cp + 32 * wq);
 #pragma unroll
         for (int u = 0; u < 3; ++u) {
           if (u < wr) {
@@ -402,6 +448,11 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, 4>::MIN_BLOCKS)
           }
         }
       }
+      if (!ready) {
+        named_barrier(1, blockDim.x);
+        ready = true;
+      }
+      if (sizeof(R) == 8 && g == 0) direct = ccls[0] == 0;
       if (direct)
         acc = cx<R>{ar, ai};
       else
@@ -409,8 +460,9 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, 4>::MIN_BLOCKS)
     }
     if (row < n) epilogue<DT, YDT, EPI>(row, acc, ax, rk, err_acc);
   }
+  if (!ready) named_barrier(1, blockDim.x);  // a warp without a slice
   if constexpr (EPI == EPI_RK) {
-    if (rk.stage == RK_STEP - 1) finish_error<SPMV_BLOCK>(rk, err_acc, red);
+    if (rk.stage == RK_STEP - 1) finish_error<DICT_BLOCK>(rk, err_acc, red);
   }
 }
 
@@ -631,13 +683,18 @@ static int launch_dict(cudaStream_t st, const qg_csr_groups& A, double t, const 
   auto kern = spmv_dict_kernel<DT, YDT, EPI, CB, RI>;
   const size_t smem = ((size_t)A.lanes * (sizeof(ST) + sizeof(int)) + 15) & ~(size_t)15;
   static OccCache cache;  // one per instantiation
-  const int per_sm = staged_occupancy(kern, SPMV_BLOCK, smem, cache);
+  const int per_sm = staged_occupancy(kern, DICT_BLOCK, smem, cache);
   if (per_sm <= 0) return set_error(QG_ERR_ARG, "dictionary does not fit in shared memory");
-  const int64_t blocks = ((int64_t)A.n_tiles * 32 + SPMV_BLOCK - 1) / SPMV_BLOCK;
-  int64_t cap = (int64_t)sm_count() * per_sm;
-  if (cap > qg_scratch_doubles()) cap = qg_scratch_doubles();
-  const int grid = (int)(blocks < 1 ? 1 : (blocks < cap ? blocks : cap));
-  kern<<<grid, SPMV_BLOCK, smem, st>>>(A, t, (const ST*)x, ax, rk);
+  int64_t grid = (int64_t)sm_count() * per_sm;
+  if (grid > A.n_tiles) grid = A.n_tiles;
+  if (grid > qg_scratch_doubles()) grid = qg_scratch_doubles();
+  if (grid < 1) grid = 1;
+  // a warp per slice of the block's run and one for the coefficients; the error reduction
+  // counts on all warps, and the tables want a few to fetch them
+  const int64_t run = (A.n_tiles + grid - 1) / grid + 1;
+  int threads = DICT_BLOCK;
+  if (EPI != EPI_RK && run < DICT_BLOCK / 32) threads = run < 8 ? 256 : (int)run * 32;
+  kern<<<(int)grid, threads, smem, st>>>(A, t, (const ST*)x, ax, rk);
   return check_launch("spmv_dict_kernel");
 }
 
