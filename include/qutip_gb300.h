@@ -251,6 +251,7 @@ typedef struct qg_generator {
   const void* op;
   int64_t hermitian_d; /* > 0: stages through qg_vern7_stage_herm (QG_GEN_CSR) */
 } qg_generator;
+#define QG_COEF_TABLE (32 * (QG_MAX_GROUPS + QG_MAX_COPS))
 typedef struct qg_vern7_ctl {
   double t, t_prev, t_front, dt_safe, dt_int;
   double atol, rtol, min_step, max_step;
@@ -265,6 +266,8 @@ typedef struct qg_vern7_ctl {
   int32_t pad_;
   unsigned int* barrier;   /* of qg_vern7_range (device) */
   double* host_result;     /* one double of pinned host memory */
+  double* coef_table;      /* QG_COEF_TABLE doubles (device) for the coefficients of a step's
+                              stages; NULL: each stage evaluates its own */
 } qg_vern7_ctl;
 
 /* ---- library ---------------------------------------------------------- */

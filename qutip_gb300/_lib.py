@@ -96,11 +96,12 @@ class Vern7Ctl(C.Structure):
         ("rhs", C.c_int64), ("launches", C.c_int64), ("status", C.c_int32),
         ("interpolate", C.c_int32), ("interp", C.c_int32), ("swaps", C.c_int32),
         ("barrier_base", C.c_uint32), ("pad_", C.c_int32), ("barrier", C.c_void_p),
-        ("host_result", C.c_void_p)]
+        ("host_result", C.c_void_p), ("coef_table", C.c_void_p)]
 
 
 QG_GEN_CSR, QG_GEN_LINDBLAD, QG_GEN_DENSE = 0, 1, 2
 QG_DEVICE_WAIT = -9
+QG_COEF_TABLE = 32 * (QG_MAX_GROUPS + QG_MAX_COPS)
 
 _P = C.POINTER
 _SIGS = {

@@ -15,6 +15,14 @@ int sm_count();
 int check_groups(const qg_csr_groups* A);
 // The same for an operator of the Hermitian half form on d x d states.
 int check_herm(const qg_csr_groups* A, int64_t d);
+// One stage with the coefficients of that stage already on the device (coefs: the operator's
+// groups, then the collapse operators, complex double each; null: the launch evaluates them).
+int stage_csr(const qg_csr_groups* A, const qg_rk_buffers* B, int stage, double t_prev, double dt,
+              double atol, double rtol, const void* coefs, void* stream);
+int stage_herm(const qg_csr_groups* A, int64_t d, const qg_rk_buffers* B, int stage, double t_prev,
+               double dt, double atol, double rtol, const void* coefs, void* stream);
+int stage_lindblad(const qg_lindblad* L, const qg_rk_buffers* B, int stage, double t_prev,
+                   double dt, double atol, double rtol, const void* coefs, void* stream);
 }  // namespace qg
 
 // The fault flag of the fused step kernel's barrier waits, read and cleared (for

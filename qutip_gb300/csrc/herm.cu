@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(HERM_BLOCK, HermBounds<DT>::MIN_BLOCKS)
   ST* tval = reinterpret_cast<ST*>(dict_smem);
   int* toff = reinterpret_cast<int*>(dict_smem + (size_t)D * sizeof(ST));
   if (threadIdx.x < G) {
-    const cplx k = group_coef(A, threadIdx.x, t);
+    const cplx k = rk.coefs ? rk.coefs[threadIdx.x] : group_coef(A, threadIdx.x, t);
     coef[threadIdx.x] = cx<CT>{(CT)k.re, (CT)k.im};
     ccls[threadIdx.x] = coef_class(coef[threadIdx.x]);
   }
@@ -327,15 +327,16 @@ extern "C" int qg_hermitian_check(const qg_csr_groups* A, int64_t d, const void*
   return set_error(QG_ERR_UNSUPPORTED, "dtype");
 }
 
-extern "C" int qg_vern7_stage_herm(const qg_csr_groups* A, int64_t d, const qg_rk_buffers* B,
-                                   int stage, double t_prev, double dt, double atol, double rtol,
-                                   void* stream) {
+int qg::stage_herm(const qg_csr_groups* A, int64_t d, const qg_rk_buffers* B, int stage,
+                   double t_prev, double dt, double atol, double rtol, const void* coefs,
+                   void* stream) {
   int rc = check_herm(A, d);
   if (rc) return rc;
   RkArgs rk;
   const void* x = nullptr;
   rc = prepare_stage(B, A->dtype, A->n_rows, stage, dt, atol, rtol, rk, x);
   if (rc) return rc;
+  rk.coefs = static_cast<const cplx*>(coefs);
   cudaStream_t st = (cudaStream_t)stream;
   const double t = t_prev + VERN7_C_HOST[stage] * dt;
   const bool one = A->tile_nnz == 1;
@@ -347,4 +348,10 @@ extern "C" int qg_vern7_stage_herm(const qg_csr_groups* A, int64_t d, const qg_r
                : launch_herm<QG_C64, QG_C128, 2>(st, *A, (int)d, t, x, rk);
   return one ? launch_herm<QG_C64, QG_C64, 1>(st, *A, (int)d, t, x, rk)
              : launch_herm<QG_C64, QG_C64, 2>(st, *A, (int)d, t, x, rk);
+}
+
+extern "C" int qg_vern7_stage_herm(const qg_csr_groups* A, int64_t d, const qg_rk_buffers* B,
+                                   int stage, double t_prev, double dt, double atol, double rtol,
+                                   void* stream) {
+  return stage_herm(A, d, B, stage, t_prev, dt, atol, rtol, nullptr, stream);
 }

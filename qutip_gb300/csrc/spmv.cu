@@ -70,9 +70,10 @@ __device__ __forceinline__ void lane_dot(const int* __restrict__ col, const VT* 
 }
 
 template <typename CT>
-__device__ __forceinline__ void load_coefs(const qg_csr_groups& A, double t, cx<CT>* coef) {
+__device__ __forceinline__ void load_coefs(const qg_csr_groups& A, double t, const cplx* table,
+                                           cx<CT>* coef) {
   if (threadIdx.x < A.n_groups) {
-    cplx c = group_coef(A, threadIdx.x, t);
+    cplx c = table ? table[threadIdx.x] : group_coef(A, threadIdx.x, t);
     coef[threadIdx.x] = cx<CT>{(CT)c.re, (CT)c.im};
   }
 }
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(SPMV_BLOCK)
   using R = typename elem<DT>::R;
   __shared__ cx<R> coef[QG_MAX_GROUPS];
   __shared__ double red[SPMV_BLOCK / 32];
-  load_coefs(A, t, coef);
+  load_coefs(A, t, rk.coefs, coef);
   __syncthreads();
 
   const int G = A.n_groups;
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(BLOCK)
   const int G = A.n_groups;
   const int nzt = A.tile_nnz;
   const size_t sb = (size_t)nzt * (sizeof(ST) + 4) + (size_t)rpt * 4;
-  load_coefs(A, t, coef);
+  load_coefs(A, t, rk.coefs, coef);
   if (threadIdx.x == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, UNR>::MIN_BLOCKS)
   using R = typename elem<DT>::R;
   __shared__ cx<R> coef[QG_MAX_GROUPS];
   __shared__ double red[SPMV_BLOCK / 32];
-  load_coefs(A, t, coef);
+  load_coefs(A, t, rk.coefs, coef);
   __syncthreads();
   const int G = A.n_groups;
   const int n = (int)A.n_rows;
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(DICT_BLOCK, 1)
   const bool evaluator = warp == workers;
   if (evaluator) {
     if (lane < G) {
-      const cplx c = group_coef(A, lane, t);
+      const cplx c = rk.coefs ? rk.coefs[lane] : group_coef(A, lane, t);
       coef[lane] = cx<R>{(R)c.re, (R)c.im};
       ccls[lane] = coef_class(coef[lane]);
     }
@@ -494,11 +495,15 @@ __global__ void __launch_bounds__(LB_BLOCK)
   __shared__ double red[LB_BLOCK / 32];
   const int G = L.n_groups, ND = L.n_diag_cops, NE = L.n_cops - L.n_diag_cops;
   if (threadIdx.x < G) {
-    const cplx k = prog_coef(L.a_coef_code, L.a_coef_start, L.a_coef_consts, threadIdx.x, t);
+    const cplx k = rk.coefs ? rk.coefs[threadIdx.x]
+                            : prog_coef(L.a_coef_code, L.a_coef_start, L.a_coef_consts,
+                                        threadIdx.x, t);
     ca[threadIdx.x] = cx<R>{(R)k.re, (R)k.im};
   }
   if (threadIdx.x < L.n_cops) {
-    const cplx f = prog_coef(L.c_coef_code, L.c_coef_start, L.c_coef_consts, threadIdx.x, t);
+    const cplx f = rk.coefs ? rk.coefs[G + threadIdx.x]
+                            : prog_coef(L.c_coef_code, L.c_coef_start, L.c_coef_consts,
+                                        threadIdx.x, t);
     wc[threadIdx.x] = (R)(f.re * f.re + f.im * f.im);
   }
   __syncthreads();
@@ -884,8 +889,8 @@ extern "C" int qg_spmv_csr(const qg_csr_groups* A, double t, const void* x, void
   return launch_any<QG_C64, QG_C64, EPI_AXPBY>(st, *A, t, x, ax, rk);
 }
 
-extern "C" int qg_vern7_stage(const qg_csr_groups* A, const qg_rk_buffers* B, int stage,
-                              double t_prev, double dt, double atol, double rtol, void* stream) {
+int qg::stage_csr(const qg_csr_groups* A, const qg_rk_buffers* B, int stage, double t_prev,
+                  double dt, double atol, double rtol, const void* coefs, void* stream) {
   int rc = check_groups(A);
   if (rc) return rc;
   if (A->n_rows != A->n_cols) return set_error(QG_ERR_ARG, "operator must be square with n rows");
@@ -894,6 +899,7 @@ extern "C" int qg_vern7_stage(const qg_csr_groups* A, const qg_rk_buffers* B, in
   rc = prepare_stage(B, A->dtype, A->n_rows, stage, dt, atol, rtol, rk, x);
   if (rc) return rc;
   if (B->n == 0) return QG_OK;
+  rk.coefs = static_cast<const cplx*>(coefs);
   AxpbyArgs ax{};
   cudaStream_t st = (cudaStream_t)stream;
   const double t = t_prev + VERN7_C_HOST[stage] * dt;
@@ -902,6 +908,11 @@ extern "C" int qg_vern7_stage(const qg_csr_groups* A, const qg_rk_buffers* B, in
   if (B->state_dtype == QG_C128)
     return launch_any<QG_C64, QG_C128, EPI_RK>(st, *A, t, x, ax, rk);
   return launch_any<QG_C64, QG_C64, EPI_RK>(st, *A, t, x, ax, rk);
+}
+
+extern "C" int qg_vern7_stage(const qg_csr_groups* A, const qg_rk_buffers* B, int stage,
+                              double t_prev, double dt, double atol, double rtol, void* stream) {
+  return stage_csr(A, B, stage, t_prev, dt, atol, rtol, nullptr, stream);
 }
 
 extern "C" int qg_lindblad_apply(const qg_lindblad* L, double t, const void* x, void* y,
@@ -917,14 +928,15 @@ extern "C" int qg_lindblad_apply(const qg_lindblad* L, double t, const void* x, 
   return launch_lindblad<QG_C64, QG_C64, EPI_AXPBY>(st, *L, t, x, ax, rk);
 }
 
-extern "C" int qg_lindblad_stage(const qg_lindblad* L, const qg_rk_buffers* B, int stage,
-                                 double t_prev, double dt, double atol, double rtol, void* stream) {
+int qg::stage_lindblad(const qg_lindblad* L, const qg_rk_buffers* B, int stage, double t_prev,
+                       double dt, double atol, double rtol, const void* coefs, void* stream) {
   int rc = check_lindblad(L);
   if (rc) return rc;
   RkArgs rk;
   const void* x = nullptr;
   rc = prepare_stage(B, L->dtype, L->d * L->d, stage, dt, atol, rtol, rk, x);
   if (rc) return rc;
+  rk.coefs = static_cast<const cplx*>(coefs);
   AxpbyArgs ax{};
   cudaStream_t st = (cudaStream_t)stream;
   const double t = t_prev + VERN7_C_HOST[stage] * dt;
@@ -933,4 +945,9 @@ extern "C" int qg_lindblad_stage(const qg_lindblad* L, const qg_rk_buffers* B, i
   if (B->state_dtype == QG_C128)
     return launch_lindblad<QG_C64, QG_C128, EPI_RK>(st, *L, t, x, ax, rk);
   return launch_lindblad<QG_C64, QG_C64, EPI_RK>(st, *L, t, x, ax, rk);
+}
+
+extern "C" int qg_lindblad_stage(const qg_lindblad* L, const qg_rk_buffers* B, int stage,
+                                 double t_prev, double dt, double atol, double rtol, void* stream) {
+  return stage_lindblad(L, B, stage, t_prev, dt, atol, rtol, nullptr, stream);
 }

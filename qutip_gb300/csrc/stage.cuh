@@ -75,6 +75,7 @@ struct RkArgs {
   // bit j set where fa_d[j] / fe_d[j] is nonzero: the factor loops test these integer
   // masks, not the factors (a floating-point compare per row would run on the FP64 pipe)
   unsigned int nz_a, nz_e;
+  const cplx* coefs;  // the stage's coefficients, evaluated before; null: by this launch
 };
 
 

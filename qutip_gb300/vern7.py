@@ -100,6 +100,7 @@ class GpuVern7:
         self._barrier_base = C.c_uint32(0)
         self.result = torch.zeros(4, dtype=torch.float64, device=dev)
         self._host = torch.zeros(4, dtype=torch.float64).pin_memory()
+        self._coefs = torch.empty(_lib.QG_COEF_TABLE, dtype=torch.float64, device=dev)
         self.y_prev, self.y_front = self._ya, self._yb
         # mixed form: complex64 copies of y_prev / y_front (stage inputs), swapped with them
         self.mixed = self.state_dt != self.stage_dt
@@ -286,7 +287,7 @@ class GpuVern7:
                           self.stats["steps"], self.stats["rejected"], self.stats["rhs"], 0,
                           self.status, int(self.interpolate), int(self._out[0] == "interp"), 0,
                           self._barrier_base.value, 0, self.counter.data_ptr() + 4,
-                          self._host.data_ptr())
+                          self._host.data_ptr(), self._coefs.data_ptr())
         rc = getattr(_lib.load(), name)(C.byref(gen), C.byref(rk), C.byref(c), *args, stream_ptr())
         _lib.LAUNCHES[0] += c.launches
         if c.swaps:

@@ -107,3 +107,28 @@ def test_failures_reach_the_caller():
     gen = _lib.Generator(7, 0, 1, 0)
     assert _lib.load().qg_vern7_integrate(gen, ig._rk(), _lib.Vern7Ctl(), 1.0, 0, None) == \
         _lib.QG_ERR_ARG
+
+
+@pytest.mark.parametrize("hermitian", [False, True])
+@pytest.mark.parametrize("n_cops", [1, 33])
+def test_coefficients_evaluated_once_per_step(hermitian, n_cops):
+    """Programs of the Hamiltonian's terms and of up to more collapse operators than a warp,
+    constant and time-dependent in turn: as when each stage evaluates its own (to rounding)."""
+    from qutip_gb300.coefficients import coefficient
+    from qutip_gb300.lindblad import LindbladOperator
+    from qutip_gb300.vern7 import GpuVern7
+    s = S.ising_chain(5)
+    f = [None, coefficient("0.5*exp(-t/3) + 0.2j*cos(t)"), coefficient("0.7*sin(2*t)")]
+    c_ops = [(0.1 * s.c_ops[i % len(s.c_ops)], f[(i + 1) % 3]) for i in range(n_cops)]
+    op = LindbladOperator.from_hamiltonian(s.h_terms, c_ops, dtype="c128")
+    op.hermitian = hermitian
+    lib, py = (GpuVern7(op) for _ in range(2))
+    py._generator = lambda: None
+    for ig in (lib, py):
+        ig.set_initial_value(torch.from_numpy(s.state0), 0.3)
+        for t in (0.35, 1.0):                          # dense output and whole steps
+            ig.integrate(t)
+        ig.check()
+    assert lib.stats == py.stats
+    # t_prev + c dt may be fused into one rounding on the host
+    assert float((lib.get_state() - py.get_state()).abs().max()) <= 1e-13
