@@ -335,10 +335,11 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, UNR>::MIN_BLOCKS)
 // coefficients once (eight blocks did it side by side on one FP64 pipe), and the
 // evaluation runs beside the first sums, which do not need it.  At 64 registers a
 // complex64 warp has enough gathers in flight that 32 of them do as well as 48 at 40
-// registers (two blocks of 768 threads: 13.7 us at L = 9, this 11.5).  Measured, one
+// registers (two blocks of 768 threads: 13.7 us at L = 9, this 11.9).  Measured, one
 // application with a driven group, 256 threads a block and the coefficients first ->
-// now: complex64 L = 8 8.4 -> 5.9 us, L = 9 13.6 -> 11.5, L = 10 34.0 -> 34.3; complex128
-// 14.2 -> 11.4, 42.5 -> 35.9 (FP64 issue alone 21), 151 -> 139.
+// now: complex64 L = 8 8.4 -> 6.1 us, L = 9 13.6 -> 11.9, L = 10 34.0 -> 34.5; complex128
+// 14.2 -> 11.6, 42.5 -> 36.4 (FP64 issue alone 21), 151 -> 140.  Constant coefficients and
+// large tables (Jaynes-Cummings N = 42 and 59, complex128): 4.6 and 4.7 us on both sides.
 constexpr int DICT_BLOCK = 1024;
 
 // Barrier of `threads` threads of the block.
@@ -362,26 +363,42 @@ __global__ void __launch_bounds__(DICT_BLOCK, 1)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   ST* tval = reinterpret_cast<ST*>(dict_smem);
   int* toff = reinterpret_cast<int*>(dict_smem + (size_t)D * sizeof(ST));
-  // The last warp evaluates the coefficients, a few microseconds of dependent FP64 work, while
-  // the others stage the tables and form their first sums; it takes no slice of the first round.
-  const int workers = nwarps - 1;
+  // Where there are programs the last warp evaluates them, a few microseconds of dependent FP64
+  // work, while the others stage the tables and form their first sums; it takes no slice of
+  // the first round.
+  const bool programs = A.coef_code && !rk.coefs;
+  const int workers = programs ? nwarps - 1 : nwarps;
   const bool evaluator = warp == workers;
+  if (evaluator ? lane < G : !programs && (int)threadIdx.x < G) {
+    const int g = evaluator ? lane : threadIdx.x;
+    const cplx c = rk.coefs ? rk.coefs[g] : group_coef(A, g, t);
+    coef[g] = cx<R>{(R)c.re, (R)c.im};
+    ccls[g] = coef_class(coef[g]);
+  }
   if (evaluator) {
-    if (lane < G) {
-      const cplx c = rk.coefs ? rk.coefs[lane] : group_coef(A, lane, t);
-      coef[lane] = cx<R>{(R)c.re, (R)c.im};
-      ccls[lane] = coef_class(coef[lane]);
-    }
     named_barrier(1, blockDim.x);
   } else {
-    for (int i = threadIdx.x; i < D; i += workers * 32) {
-      tval[i] = __ldg(static_cast<const ST*>(A.val) + i);
-      toff[i] = __ldg(A.dict_off + i);
+    const int stride = workers * 32;
+    for (int i = threadIdx.x; i < D; i += 4 * stride) {  // four entries in flight, ends included
+      ST v[4];
+      int o[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i + u * stride < D) {
+          v[u] = __ldg(static_cast<const ST*>(A.val) + i + u * stride);
+          o[u] = __ldg(A.dict_off + i + u * stride);
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i + u * stride < D) {
+          tval[i + u * stride] = v[u];
+          toff[i + u * stride] = o[u];
+        }
     }
     if ((int)threadIdx.x <= G) tstart[threadIdx.x] = __ldg(A.dict_start + threadIdx.x);
     named_barrier(2, workers * 32);
   }
-  bool ready = evaluator;  // the coefficients are there
+  bool ready = evaluator || !programs;  // the coefficients are there
   const int n = (int)A.n_rows;
   const int S = A.n_tiles;
   const int last_col = (int)A.n_cols - 1;
@@ -691,14 +708,20 @@ static int launch_dict(cudaStream_t st, const qg_csr_groups& A, double t, const 
   const int per_sm = staged_occupancy(kern, DICT_BLOCK, smem, cache);
   if (per_sm <= 0) return set_error(QG_ERR_ARG, "dictionary does not fit in shared memory");
   int64_t grid = (int64_t)sm_count() * per_sm;
-  if (grid > A.n_tiles) grid = A.n_tiles;
+  // at least four slices to a block: every block fetches the tables
+  if (grid > (A.n_tiles + 3) / 4) grid = (A.n_tiles + 3) / 4;
   if (grid > qg_scratch_doubles()) grid = qg_scratch_doubles();
   if (grid < 1) grid = 1;
-  // a warp per slice of the block's run and one for the coefficients; the error reduction
-  // counts on all warps, and the tables want a few to fetch them
+  // A warp per slice of the block's run and one for the coefficients, and enough threads that
+  // four entries each are the tables (Jaynes-Cummings N = 30, 3,190 entries: 256 threads
+  // 4.1 us, 512 3.85).  The error reduction counts on all warps.
   const int64_t run = (A.n_tiles + grid - 1) / grid + 1;
   int threads = DICT_BLOCK;
-  if (EPI != EPI_RK && run < DICT_BLOCK / 32) threads = run < 8 ? 256 : (int)run * 32;
+  if (EPI != EPI_RK && run < DICT_BLOCK / 32) {
+    threads = run < 8 ? 256 : (int)run * 32;
+    const int fetch = (A.lanes + 127) / 128 * 32;
+    if (threads < fetch) threads = fetch < DICT_BLOCK ? fetch : DICT_BLOCK;
+  }
   kern<<<(int)grid, threads, smem, st>>>(A, t, (const ST*)x, ax, rk);
   return check_launch("spmv_dict_kernel");
 }
