@@ -17,9 +17,10 @@
 // at d = 1024).  32 x 32 blocks on the diagonal are evaluated whole and not mirrored.
 //
 // Measured, whole solves of the L = 10 Ising chain (1,048,576 rows, 1646 right-hand sides):
-// complex128 279 -> 168 ms, mixed 95 -> 66 ms.  It is taken above 512 rows per SM, where the
-// stages go out one by one; smaller systems take the fused step kernel (step.cu), whose
-// stage is latency.
+// complex128 279 -> 168 ms, mixed 95 -> 66 ms (158 and 58 with the driver's loop and its
+// coefficient table).  It is taken above 512 rows per SM, where the stages go out one by
+// one; from 256 rows per SM up to there the fused step kernel (step.cu) evaluates the same
+// units.
 #include <mutex>
 
 #include "capi_internal.h"
