@@ -59,14 +59,15 @@ __global__ void __launch_bounds__(LH_BLOCK, LhBounds<DT>::MIN_BLOCKS)
   int* so = reinterpret_cast<int*>(lh_smem + (keep ? (size_t)wtot * LH_COLS * sizeof(ST) : 0));
   const int G = L.n_groups, ND = L.n_diag_cops, NE = L.n_cops - L.n_diag_cops;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const cplx* table = stage_coefs<EPI>(rk);
   if (tid < G) {
-    const cplx k = rk.coefs ? rk.coefs[tid]
-                            : prog_coef(L.a_coef_code, L.a_coef_start, L.a_coef_consts, tid, t);
+    const cplx k = table ? table[tid]
+                         : prog_coef(L.a_coef_code, L.a_coef_start, L.a_coef_consts, tid, t);
     ca[tid] = cx<R>{(R)k.re, (R)k.im};
   }
   for (int i = tid; i < L.n_cops; i += LH_BLOCK) {
-    const cplx f = rk.coefs ? rk.coefs[G + i]
-                            : prog_coef(L.c_coef_code, L.c_coef_start, L.c_coef_consts, i, t);
+    const cplx f = table ? table[G + i]
+                         : prog_coef(L.c_coef_code, L.c_coef_start, L.c_coef_consts, i, t);
     wc[i] = (R)(f.re * f.re + f.im * f.im);
   }
   const int d = (int)L.d;

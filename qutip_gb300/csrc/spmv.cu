@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(SPMV_BLOCK)
   using R = typename elem<DT>::R;
   __shared__ cx<R> coef[QG_MAX_GROUPS];
   __shared__ double red[SPMV_BLOCK / 32];
-  load_coefs(A, t, rk.coefs, coef);
+  load_coefs(A, t, stage_coefs<EPI>(rk), coef);
   __syncthreads();
 
   const int G = A.n_groups;
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(BLOCK)
   const int G = A.n_groups;
   const int nzt = A.tile_nnz;
   const size_t sb = (size_t)nzt * (sizeof(ST) + 4) + (size_t)rpt * 4;
-  load_coefs(A, t, rk.coefs, coef);
+  load_coefs(A, t, stage_coefs<EPI>(rk), coef);
   if (threadIdx.x == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, UNR>::MIN_BLOCKS)
   using R = typename elem<DT>::R;
   __shared__ cx<R> coef[QG_MAX_GROUPS];
   __shared__ double red[SPMV_BLOCK / 32];
-  load_coefs(A, t, rk.coefs, coef);
+  load_coefs(A, t, stage_coefs<EPI>(rk), coef);
   __syncthreads();
   const int G = A.n_groups;
   const int n = (int)A.n_rows;
@@ -337,9 +337,9 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SlicedBounds<DT, UNR>::MIN_BLOCKS)
 // complex64 warp has enough gathers in flight that 32 of them do as well as 48 at 40
 // registers (two blocks of 768 threads: 13.7 us at L = 9, this 11.9).  Measured, one
 // application with a driven group, 256 threads a block and the coefficients first ->
-// now: complex64 L = 8 8.4 -> 6.1 us, L = 9 13.6 -> 11.9, L = 10 34.0 -> 34.5; complex128
-// 14.2 -> 11.6, 42.5 -> 36.4 (FP64 issue alone 21), 151 -> 140.  Constant coefficients and
-// large tables (Jaynes-Cummings N = 42 and 59, complex128): 4.6 and 4.7 us on both sides.
+// now: complex64 L = 8 8.4 -> 6.1 us, L = 9 13.6 -> 11.9, L = 10 34.0 -> 35; complex128
+// 14.2 -> 11.2, 42.5 -> 35.6 (FP64 issue alone 21), 151 -> 140.  Constant coefficients and
+// large tables (Jaynes-Cummings N = 42 and 59, complex128): 4.6 and 4.8 us on both sides.
 constexpr int DICT_BLOCK = 1024;
 
 // Barrier of `threads` threads of the block.
@@ -366,12 +366,13 @@ __global__ void __launch_bounds__(DICT_BLOCK, 1)
   // Where there are programs the last warp evaluates them, a few microseconds of dependent FP64
   // work, while the others stage the tables and form their first sums; it takes no slice of
   // the first round.
-  const bool programs = A.coef_code && !rk.coefs;
+  const cplx* table = stage_coefs<EPI>(rk);
+  const bool programs = A.coef_code && !table;
   const int workers = programs ? nwarps - 1 : nwarps;
   const bool evaluator = warp == workers;
   if (evaluator ? lane < G : !programs && (int)threadIdx.x < G) {
     const int g = evaluator ? lane : threadIdx.x;
-    const cplx c = rk.coefs ? rk.coefs[g] : group_coef(A, g, t);
+    const cplx c = table ? table[g] : group_coef(A, g, t);
     coef[g] = cx<R>{(R)c.re, (R)c.im};
     ccls[g] = coef_class(coef[g]);
   }
@@ -408,8 +409,9 @@ __global__ void __launch_bounds__(DICT_BLOCK, 1)
   // rows together, which keeps what they gather closer in the L2.
   const int first = (int)gridDim.x * workers, all = (int)gridDim.x * nwarps;
   const bool runs = S <= 2 * all;
-  const int run0 = (int)((int64_t)S * blockIdx.x / gridDim.x);
-  const int s_end = runs ? (int)((int64_t)S * (blockIdx.x + 1) / gridDim.x) : S;
+  const int share = S / (int)gridDim.x, more = S % (int)gridDim.x, b = (int)blockIdx.x;
+  const int run0 = b * share + min(b, more);
+  const int s_end = runs ? run0 + share + (b < more) : S;
   const int head = runs ? run0 + workers : first;               // end of the first round
   const int next0 = runs ? head + warp : first + blockIdx.x * nwarps + warp;
   int sl = evaluator ? next0 : runs ? run0 + warp : blockIdx.x * workers + warp;
@@ -511,16 +513,17 @@ __global__ void __launch_bounds__(LB_BLOCK)
   __shared__ R wc[QG_MAX_COPS];
   __shared__ double red[LB_BLOCK / 32];
   const int G = L.n_groups, ND = L.n_diag_cops, NE = L.n_cops - L.n_diag_cops;
+  const cplx* table = stage_coefs<EPI>(rk);
   if (threadIdx.x < G) {
-    const cplx k = rk.coefs ? rk.coefs[threadIdx.x]
-                            : prog_coef(L.a_coef_code, L.a_coef_start, L.a_coef_consts,
-                                        threadIdx.x, t);
+    const cplx k = table ? table[threadIdx.x]
+                         : prog_coef(L.a_coef_code, L.a_coef_start, L.a_coef_consts,
+                                     threadIdx.x, t);
     ca[threadIdx.x] = cx<R>{(R)k.re, (R)k.im};
   }
   if (threadIdx.x < L.n_cops) {
-    const cplx f = rk.coefs ? rk.coefs[G + threadIdx.x]
-                            : prog_coef(L.c_coef_code, L.c_coef_start, L.c_coef_consts,
-                                        threadIdx.x, t);
+    const cplx f = table ? table[G + threadIdx.x]
+                         : prog_coef(L.c_coef_code, L.c_coef_start, L.c_coef_consts,
+                                     threadIdx.x, t);
     wc[threadIdx.x] = (R)(f.re * f.re + f.im * f.im);
   }
   __syncthreads();
@@ -714,7 +717,7 @@ static int launch_dict(cudaStream_t st, const qg_csr_groups& A, double t, const 
   if (grid < 1) grid = 1;
   // A warp per slice of the block's run and one for the coefficients, and enough threads that
   // four entries each are the tables (Jaynes-Cummings N = 30, 3,190 entries: 256 threads
-  // 4.1 us, 512 3.85).  The error reduction counts on all warps.
+  // 4.1 us, 512 3.85; 3.7 with 800).  The error reduction counts on all warps.
   const int64_t run = (A.n_tiles + grid - 1) / grid + 1;
   int threads = DICT_BLOCK;
   if (EPI != EPI_RK && run < DICT_BLOCK / 32) {
