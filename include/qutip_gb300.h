@@ -410,6 +410,14 @@ typedef struct qg_sde {
 /* Workspace of one trajectory, in complex128 values. */
 int64_t qg_sde_work_values(int64_t n, int32_t n_sc);
 
+/* The shape a launch of n_traj trajectories takes on a GPU of n_sms multiprocessors when
+ * every trajectory runs on one thread per entry: shape = {trajectories of a CTA, threads of
+ * a CTA, bytes of shared memory for their vectors, bytes for operators}.  Returns 1 when
+ * the states are too long or the operators too many for that kernel.  Host arithmetic
+ * only. */
+int qg_sde_row_shape(int64_t n, int32_t n_sc, int32_t open, int32_t n_traj, int32_t n_sms,
+                     int32_t* shape);
+
 /* n_steps Platen steps of dt for each of n_traj trajectories (one CTA each): states holds
  * n_traj complex128 states of length n (updated in place); dW holds the Wiener increments,
  * n_traj x n_steps x n_sc doubles (trajectory-major), as the reference's Wiener.dW draws

@@ -145,6 +145,7 @@ _SIGS = {
     "qg_dense_lindblad_stage": (C.c_int, [_P(DenseLindblad), _P(RkBuffers), C.c_int, C.c_double,
                                           C.c_double, C.c_double, C.c_double, C.c_void_p]),
     "qg_sde_work_values": (C.c_int64, [C.c_int64, C.c_int32]),
+    "qg_sde_row_shape": (C.c_int, [C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_void_p]),
     "qg_sde_platen": (C.c_int, [_P(Sde), C.c_int32, C.c_void_p, C.c_void_p, C.c_int32,
                                 C.c_double, C.c_void_p]),
     "qg_sde_euler": (C.c_int, [_P(Sde), C.c_int32, C.c_void_p, C.c_void_p, C.c_int32,

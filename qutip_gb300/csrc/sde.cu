@@ -593,41 +593,54 @@ __global__ void __launch_bounds__(NT, NT <= SDE_ROW_PAIR ? 2 : 1)
   if (on) states[(size_t)traj * n + r] = xr;
 }
 
+constexpr int SDE_ROW_SMEM = 220 * 1024;  // most dynamic shared memory of a CTA
+
+// Launch shape of the row kernel: trajectories and threads of a CTA, the bytes of its vectors
+// and of its operators in shared memory, and whether the form for two CTAs on an SM takes it.
+struct SdeRowShape {
+  int T, threads, vecs, ops;
+  bool pair;
+};
+static SdeRowShape sde_row_shape(int n, int d, int m, bool open, int n_traj, int sms) {
+  const int most = m == 1 ? SDE_ROW_THREADS<1> : SDE_ROW_THREADS<2>;
+  const int sums = (open ? 0 : m) + 2 * m * m;  // SDE_ROW_SUMS
+  const int per = 16 * (n * (2 + 2 * m) + sums * ((open ? d : n) + (open ? 1 : 2)));
+  // trajectories per CTA: enough CTAs for every SM first, then full CTAs
+  int T = (n_traj - 1) / sms + 1;
+  if (T > most / n) T = most / n;
+  // one CTA per SM at most: no second one to make room for
+  const bool pair = m == 1 && n <= SDE_ROW_PAIR && (n_traj - 1) / T + 1 > sms;
+  if (pair && T > SDE_ROW_PAIR / n) T = SDE_ROW_PAIR / n;
+  // the sums of kets of one entry and two operators outgrow the vectors: 576 bytes a trajectory
+  if (T > SDE_ROW_SMEM / per) T = SDE_ROW_SMEM / per;
+  const int vecs = T * per, room = SDE_ROW_SMEM - vecs;
+  return SdeRowShape{T, (T * n + 31) / 32 * 32, vecs,
+                     room < SDE_ROW_OP_SMEM ? room : SDE_ROW_OP_SMEM, pair};
+}
+
 template <int M, bool OPEN, int SCHEME, int NT>
 static int launch_sde_rows(const qg_sde& S, int n_traj, double2* states, const double* dW,
-                           int n_steps, double dt, int T, cudaStream_t st) {
-  const int n = (int)S.n;
-  const int threads = (T * n + 31) / 32 * 32;
-  const int cnt = OPEN ? S.d : n;
-  constexpr int K = SDE_ROW_SUMS<M, OPEN>;
-  const size_t vecs =
-      (size_t)T * 16 * ((size_t)n * (2 + 2 * M) + (size_t)K * (cnt + (OPEN ? 1 : 2)));
-  int op = 220 * 1024 - (int)vecs;
-  if (op > SDE_ROW_OP_SMEM) op = SDE_ROW_OP_SMEM;
+                           int n_steps, double dt, const SdeRowShape& sh, cudaStream_t st) {
+  const int smem = sh.vecs + sh.ops;
   auto kern = sde_row_kernel<M, OPEN, SCHEME, NT>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)(vecs + op)) != cudaSuccess)
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return set_error(QG_ERR_CUDA, "stochastic kernel: shared memory opt-in failed");
-  kern<<<(n_traj + T - 1) / T, threads, vecs + op, st>>>(S, n_traj, states, dW, n_steps, dt, T, op);
+  kern<<<(n_traj - 1) / sh.T + 1, sh.threads, smem, st>>>(S, n_traj, states, dW, n_steps, dt, sh.T,
+                                                         sh.ops);
   return check_launch("sde_row_kernel");
 }
 
 template <bool OPEN, int SCHEME>
 static int launch_sde_rows_shape(const qg_sde& S, int n_traj, double2* states, const double* dW,
                                  int n_steps, double dt, cudaStream_t st) {
-  const int n = (int)S.n, most = S.n_sc == 1 ? SDE_ROW_THREADS<1> : SDE_ROW_THREADS<2>;
-  // trajectories per CTA: enough CTAs for every SM first, then full CTAs
-  int T = (n_traj + sm_count() - 1) / sm_count();
-  if (T > most / n) T = most / n;
+  const SdeRowShape sh = sde_row_shape((int)S.n, S.d, S.n_sc, OPEN, n_traj, sm_count());
   if (S.n_sc == 2)
     return launch_sde_rows<2, OPEN, SCHEME, SDE_ROW_THREADS<2>>(S, n_traj, states, dW, n_steps, dt,
-                                                                T, st);
-  // one CTA per SM at most: no second one to make room for
-  if (n > SDE_ROW_PAIR || (n_traj + T - 1) / T <= sm_count())
+                                                                sh, st);
+  if (!sh.pair)
     return launch_sde_rows<1, OPEN, SCHEME, SDE_ROW_THREADS<1>>(S, n_traj, states, dW, n_steps, dt,
-                                                                T, st);
-  if (T > SDE_ROW_PAIR / n) T = SDE_ROW_PAIR / n;
-  return launch_sde_rows<1, OPEN, SCHEME, SDE_ROW_PAIR>(S, n_traj, states, dW, n_steps, dt, T, st);
+                                                                sh, st);
+  return launch_sde_rows<1, OPEN, SCHEME, SDE_ROW_PAIR>(S, n_traj, states, dW, n_steps, dt, sh, st);
 }
 
 static int check_sde(const qg_sde* S) {
@@ -679,6 +692,20 @@ using namespace qg;
 
 extern "C" int64_t qg_sde_work_values(int64_t n, int32_t n_sc) {
   return (5 + 5 * (int64_t)n_sc) * n;
+}
+
+extern "C" int qg_sde_row_shape(int64_t n, int32_t n_sc, int32_t open, int32_t n_traj,
+                                int32_t n_sms, int32_t* shape) {
+  if (!shape) return set_error(QG_ERR_ARG, "null shape");
+  if (n < 1 || n_sc < 1 || n_traj < 1 || n_sms < 1) return set_error(QG_ERR_ARG, "bad launch");
+  if (n_sc > SDE_ROW_MAX_M || n > (n_sc == 1 ? SDE_ROW_THREADS<1> : SDE_ROW_THREADS<2>)) return 1;
+  int d = (int)n;
+  if (open)
+    for (d = 1; (int64_t)d * d < n;) ++d;
+  const SdeRowShape s = sde_row_shape((int)n, d, n_sc, open != 0, n_traj, n_sms);
+  const int32_t v[4] = {s.T, s.threads, s.vecs, s.ops};
+  for (int i = 0; i < 4; ++i) shape[i] = v[i];
+  return QG_OK;
 }
 
 extern "C" int qg_sde_platen(const qg_sde* S, int32_t n_traj, void* states, const double* dW,
