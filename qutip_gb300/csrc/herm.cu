@@ -255,9 +255,10 @@ __global__ void __launch_bounds__(HERM_BLOCK, HermBounds<DT>::MIN_BLOCKS)
 
 static int herm_occupancy(const void* kern, size_t smem) {
   // one launch shape per (device, kernel, table size): asked for at every launch, as the
-  // tables' size differs between operators (a host query of about a microsecond)
-  if (smem > 32 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem) != cudaSuccess)
+  // tables' size differs between operators (a host query of about a microsecond).  Any size is
+  // opted in: the 48 KB default counts the 9 to 17 KB of static shared memory too.
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+      cudaSuccess)
     return -1;
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, HERM_BLOCK, smem) !=
