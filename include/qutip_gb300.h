@@ -263,9 +263,12 @@ typedef struct qg_vern7_ctl {
   int32_t interp; /* 1: the state at t is the dense output of the current step */
   int32_t swaps;  /* toggled when y_prev and y_front changed places */
   uint32_t barrier_base;   /* of qg_vern7_range */
-  int32_t pad_;
+  int32_t wait_mcycles;    /* most millions of SM clocks waited at a barrier of qg_vern7_range;
+                              0: the library's limit */
   unsigned int* barrier;   /* of qg_vern7_range (device) */
-  double* host_result;     /* one double of pinned host memory */
+  double* host_result;     /* two doubles of pinned host memory: the error norm, and a word, zero
+                              before the first call, that turns negative when a wait of a
+                              dense-output launch gives up */
   double* coef_table;      /* QG_COEF_TABLE doubles (device) for the coefficients of a step's
                               stages; NULL: each stage evaluates its own */
 } qg_vern7_ctl;
@@ -328,8 +331,8 @@ int qg_vern7_stage(const qg_csr_groups* A, const qg_rk_buffers* B, int stage, do
  * or 32, a complex128 dictionary that is not split): the caller then launches the stages
  * one by one.  barrier: one word of device memory, zero before the first launch and owned
  * by the caller's stream order; barrier_base: host word, zero at first, advanced by each
- * call.  A bounded wait that gave up leaves *B->result = -1 and sets qg_device_fault(); zero both
- * words before the next call. */
+ * call.  A bounded wait that gave up leaves *B->result = -1 and NaN in the launch's
+ * stages, and sets qg_device_fault(); zero both words before the next call. */
 int qg_vern7_range(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0, int stage1,
                    double t_prev, double dt, double atol, double rtol, unsigned int* barrier,
                    uint32_t* barrier_base, void* stream);
@@ -437,14 +440,19 @@ int qg_device_fault(void);
 /* Explicit_RungeKutta.integrate (explicit_rk.pyx:278-331) from c->t to t: trial steps until
  * t is reached, then the dense output when it was passed; step != 0: one step at most.  The
  * buffers' y_prev / y_front pointers change places as steps are accepted (c->swaps).  Failures
- * of the integration are in c->status; waits for the error norm of each trial step. */
+ * of the integration are in c->status; waits for the error norm of each trial step.  A wait
+ * in a launch that gave up is QG_ERR_CUDA with c->status = QG_DEVICE_WAIT: of a trial step in the
+ * same call, of the dense output in the next one (c->host_result[1], and NaN in the state
+ * meanwhile).  Zero the barrier's words after it. */
 int qg_vern7_integrate(const qg_generator* gen, qg_rk_buffers* B, qg_vern7_ctl* c, double t,
                        int step, void* stream);
 
 /* The outputs of a master equation: integrate to each of n_times (host memory) and record
  * the expectation values as qg_expect_dm does, one row of 2 (G + 1) doubles (device) per time,
  * the times inside one step together (qg_expect_dm_times; ops group-major).  Stops at the
- * first time the integration fails (c->status < 0). */
+ * first time the integration fails (c->status < 0).  Does not wait for the last outputs: once
+ * out has been read, c->host_result[1] < 0 tells that a wait of the last dense output gave
+ * up (what it should have given is NaN). */
 int qg_vern7_run_dm(const qg_generator* gen, qg_rk_buffers* B, qg_vern7_ctl* c,
                     const double* tlist, int n_times, const qg_csr_groups* ops, int64_t d,
                     double* out, void* stream);

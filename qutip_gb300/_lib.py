@@ -95,7 +95,7 @@ class Vern7Ctl(C.Structure):
         ("max_numsteps", C.c_int64), ("steps", C.c_int64), ("rejected", C.c_int64),
         ("rhs", C.c_int64), ("launches", C.c_int64), ("status", C.c_int32),
         ("interpolate", C.c_int32), ("interp", C.c_int32), ("swaps", C.c_int32),
-        ("barrier_base", C.c_uint32), ("pad_", C.c_int32), ("barrier", C.c_void_p),
+        ("barrier_base", C.c_uint32), ("wait_mcycles", C.c_int32), ("barrier", C.c_void_p),
         ("host_result", C.c_void_p), ("coef_table", C.c_void_p)]
 
 

@@ -23,6 +23,11 @@ int stage_herm(const qg_csr_groups* A, int64_t d, const qg_rk_buffers* B, int st
                double dt, double atol, double rtol, const void* coefs, void* stream);
 int stage_lindblad(const qg_lindblad* L, const qg_rk_buffers* B, int stage, double t_prev,
                    double dt, double atol, double rtol, const void* coefs, void* stream);
+// qg_vern7_range (d = 0) or qg_vern7_range_herm, with the limit of a wait in millions of SM
+// clocks (0: the default).
+int range_csr(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0, int stage1,
+              double t_prev, double dt, double atol, double rtol, int64_t d, int32_t wait_mcycles,
+              unsigned int* barrier, uint32_t* barrier_base, void* stream);
 }  // namespace qg
 
 // The fault flag of the fused step kernel's barrier waits, read and cleared (for

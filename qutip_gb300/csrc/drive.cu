@@ -3,10 +3,13 @@
 // stage launches of this library.  A step of a small system is tens of microseconds on the
 // GPU; the same loop in the host language above spent 65 us a step between the launches, on
 // building arguments, reading the error norm back and asking for the outputs.  The error
-// norm goes straight to a word of pinned host memory that the loop watches.  Measured, whole
+// norm goes straight to a word of pinned host memory that the loop watches; a second word
+// tells of a dense-output launch that gave up, which the loop does not wait for.  Measured, whole
 // solves: Jaynes-Cummings N = 10 5.4 -> 2.8 ms, Bose-Hubbard d = 125 6.2 -> 4.8, Ising L = 8
 // 27.4 -> 24.9, L = 10 mixed 66 -> 61 (matrix form 98 -> 92), dense d = 128 7.9 -> 7.3.
 #include <math.h>
+
+#include <atomic>
 
 #include "capi_internal.h"
 #include "common.cuh"
@@ -102,12 +105,9 @@ struct Drive {
   int range(int s0, int s1, double dt) {
     if (gen->kind != QG_GEN_CSR) return 1;
     const auto* A = static_cast<const qg_csr_groups*>(gen->op);
-    const int rc =
-        gen->hermitian_d > 0
-            ? qg_vern7_range_herm(A, B, s0, s1, c->t_prev, dt, c->atol, c->rtol, gen->hermitian_d,
-                                  c->barrier, &c->barrier_base, stream)
-            : qg_vern7_range(A, B, s0, s1, c->t_prev, dt, c->atol, c->rtol, c->barrier,
-                             &c->barrier_base, stream);
+    const int rc = range_csr(A, B, s0, s1, c->t_prev, dt, c->atol, c->rtol,
+                             gen->hermitian_d > 0 ? gen->hermitian_d : 0, c->wait_mcycles,
+                             c->barrier, &c->barrier_base, stream);
     if (rc == 0) ++c->launches;
     return rc;
   }
@@ -132,18 +132,33 @@ struct Drive {
       return check_launch("vern7 trial step");
     err = *word;
     if (err == NOT_YET) return set_error(QG_ERR_CUDA, "the step's error norm did not arrive");
-    if (err < 0.0) {
-      c->status = QG_DEVICE_WAIT;
-      return set_error(QG_ERR_CUDA,
-                       "a device wait of the fused step kernel gave up; the GPU may be unhealthy");
-    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    if (err < 0.0 || dense_gave_up()) return gave_up();
     return QG_OK;
+  }
+
+  // The waits of a dense-output launch: known once the launch is over, so looked at after the
+  // next trial step's wait, and by the caller after its own.
+  bool dense_gave_up() const {
+    return const_cast<volatile double*>(c->host_result)[1] < 0.0;
+  }
+
+  int gave_up() {
+    // every block leaves within the same limit, and may still write the words until then
+    cudaStreamSynchronize((cudaStream_t)stream);
+    c->host_result[1] = 0.0;
+    c->status = QG_DEVICE_WAIT;
+    return set_error(QG_ERR_CUDA,
+                     "a device wait of the fused step kernel gave up; the GPU may be unhealthy");
   }
 
   // _prep_dense_out (explicit_rk.pyx:399-410)
   int dense_out() {
     const double dt = c->dt_int;
+    double* const device_result = B->result;
+    B->result = c->host_result + 1;  // written when a wait gives up
     int rc = range(RK_STEP, RK_EXTRA_STEP, dt);
+    B->result = device_result;
     if (rc == 1) {
       qg_state_view v = {};
       const bool mixed = B->state_dtype != B->stage_dtype;

@@ -24,7 +24,8 @@
 // longer count.
 //
 // The launch is cooperative (all blocks resident), and every wait at the barrier is bounded:
-// a wait that gives up sets *result to -1 and every block leaves.  A row's sum and its
+// a wait that gives up sets *result to -1, every block leaves, and the launch's stages hold NaN
+// in its rows: what is read from them before the host sees the word is no value.  A row's sum and its
 // stage combination are formed by the operations of the per-stage kernels in their order.
 #include <mutex>
 
@@ -58,6 +59,7 @@ struct StepArgs {
   int herm_d;          // > 0: half form of a Hermitian d x d state (HERM instantiations)
   unsigned int* bar;   // arrivals of every earlier launch and of this one
   unsigned int bar_base;
+  long long wait;      // most SM clocks at a barrier
 };
 
 __device__ unsigned int g_step_fault = 0u;
@@ -89,7 +91,7 @@ __host__ __device__ inline StepSmem step_smem(const qg_csr_groups& A, int kind, 
 // Grid barrier: block arrivals counted in one word that only grows; this launch's n-th
 // barrier completes at base + n * blocks.  False when the bounded wait gave up.
 __device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int target,
-                                             bool* ok_s) {
+                                             long long wait, bool* ok_s) {
   if (gridDim.x == 1) {
     __syncthreads();
     return true;
@@ -104,7 +106,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int tar
     do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
       ok = (int)(v - target) >= 0;
-    } while (!ok && clock64() - t0 < STEP_WAIT_CYCLES);
+    } while (!ok && clock64() - t0 < wait);
     __threadfence();
     *ok_s = ok;
   }
@@ -288,7 +290,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
       mirror_input(a.s0 - 1);
     }
     target += gridDim.x;
-    ok = grid_barrier(a.bar, target, &ok_s);
+    ok = grid_barrier(a.bar, target, a.wait, &ok_s);
   }
 
   // ---- stages ----
@@ -443,10 +445,17 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
     }
     if (s + 1 < a.s1) {
       target += gridDim.x;
-      ok = grid_barrier(a.bar, target, &ok_s);
+      ok = grid_barrier(a.bar, target, a.wait, &ok_s);
     }
   }
   if (!ok) {
+    const R none = (R)__longlong_as_double(0x7ff8000000000000LL);
+    for (int s = a.s0; s < a.s1; ++s) {
+      if (owner) kg[(size_t)s * n64] = ST{none, none};
+      if constexpr (HERM) {
+        if (mirrored) static_cast<ST*>(rk.k)[(size_t)s * n64 + mirror] = ST{none, none};
+      }
+    }
     if (tid == 0) {
       atomicOr(&g_step_fault, 1u);
       if (rk.result) *rk.result = -1.0;
@@ -578,7 +587,8 @@ int step_fault_take() {
 // d > 0: the half form of a d x d state; A has been checked.
 static int vern7_range(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0, int stage1,
                        double t_prev, double dt, double atol, double rtol, int64_t d,
-                       unsigned int* barrier, uint32_t* barrier_base, void* stream) {
+                       int32_t wait_mcycles, unsigned int* barrier, uint32_t* barrier_base,
+                       void* stream) {
   if (!barrier || !barrier_base) return set_error(QG_ERR_ARG, "null barrier word");
   if (A->n_rows != A->n_cols) return set_error(QG_ERR_ARG, "operator must be square with n rows");
   if (!((stage0 == 0 && stage1 == RK_STEP) || (stage0 == RK_STEP && stage1 == RK_EXTRA_STEP)))
@@ -598,6 +608,7 @@ static int vern7_range(const qg_csr_groups* A, const qg_rk_buffers* B, int stage
   a.s1 = stage1;
   a.bar = barrier;
   a.herm_d = (int)d;
+  a.wait = wait_mcycles > 0 ? 1000000LL * wait_mcycles : STEP_WAIT_CYCLES;
   cudaStream_t st = (cudaStream_t)stream;
   if (B->state_dtype == QG_C128 && B->stage_dtype == QG_C128)
     return launch_range_layout<QG_C128, QG_C128>(a, barrier_base, st);
@@ -605,19 +616,27 @@ static int vern7_range(const qg_csr_groups* A, const qg_rk_buffers* B, int stage
   return launch_range_layout<QG_C64, QG_C64>(a, barrier_base, st);
 }
 
+int qg::range_csr(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0, int stage1,
+                  double t_prev, double dt, double atol, double rtol, int64_t d,
+                  int32_t wait_mcycles, unsigned int* barrier, uint32_t* barrier_base,
+                  void* stream) {
+  const int rc = d > 0 ? check_herm(A, d) : check_groups(A);
+  return rc ? rc : vern7_range(A, B, stage0, stage1, t_prev, dt, atol, rtol, d, wait_mcycles,
+                               barrier, barrier_base, stream);
+}
+
 extern "C" int qg_vern7_range(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0,
                               int stage1, double t_prev, double dt, double atol, double rtol,
                               unsigned int* barrier, uint32_t* barrier_base, void* stream) {
-  const int rc = check_groups(A);
-  return rc ? rc : vern7_range(A, B, stage0, stage1, t_prev, dt, atol, rtol, 0, barrier,
-                               barrier_base, stream);
+  return range_csr(A, B, stage0, stage1, t_prev, dt, atol, rtol, 0, 0, barrier, barrier_base,
+                   stream);
 }
 
 extern "C" int qg_vern7_range_herm(const qg_csr_groups* A, const qg_rk_buffers* B, int stage0,
                                    int stage1, double t_prev, double dt, double atol, double rtol,
                                    int64_t d, unsigned int* barrier, uint32_t* barrier_base,
                                    void* stream) {
-  const int rc = check_herm(A, d);
-  return rc ? rc : vern7_range(A, B, stage0, stage1, t_prev, dt, atol, rtol, d, barrier,
-                               barrier_base, stream);
+  const int rc = check_herm(A, d);  // d <= 0 among what it refuses
+  return rc ? rc : range_csr(A, B, stage0, stage1, t_prev, dt, atol, rtol, d, 0, barrier,
+                             barrier_base, stream);
 }

@@ -160,6 +160,7 @@ def _evolve(ig: GpuVern7, tlist, ex: ExpectOps, d: int, store_states, store_fina
         i += 1
     final = ig.get_state().clone() if store_final else None
     r = raw.cpu().numpy()
+    ig.check()                           # of the last dense output, which is over by now
     vals = r[:, 0:2 * G:2] + 1j * r[:, 1:2 * G:2]
     norm = r[:, 2 * G] + 1j * r[:, 2 * G + 1]
     if G and normalize:

@@ -37,6 +37,7 @@ from .operator import DeviceOperator, qg_dtype, stream_ptr, torch_dtype
 
 AT_FRONT, INTERPOLATED, NORMAL = 2, 1, 0
 TOO_MUCH_WORK, DT_UNDERFLOW, OUTSIDE_RANGE, NOT_INITIATED = -1, -2, -3, -4
+DEVICE_WAIT = _lib.QG_DEVICE_WAIT
 STATUS_MESSAGES = {
     AT_FRONT: "Internal state at the desired time.",
     INTERPOLATED: "Internal state past the desired time and interpolation to step done.",
@@ -46,6 +47,7 @@ STATUS_MESSAGES = {
     DT_UNDERFLOW: "Step size becomes too small. Try increasing tolerance.",
     OUTSIDE_RANGE: "Step outside available range.",
     NOT_INITIATED: "Not initialized.",
+    DEVICE_WAIT: ("a device wait of the fused step kernel gave up; the GPU may be unhealthy"),
 }
 PRECISIONS = {"double": ("c128", "c128"), "mixed": ("c128", "c64"), "single": ("c64", "c64")}
 
@@ -99,7 +101,10 @@ class GpuVern7:
         self.counter = torch.zeros(4, dtype=torch.int32, device=dev)
         self._barrier_base = C.c_uint32(0)
         self.result = torch.zeros(4, dtype=torch.float64, device=dev)
+        # word 0: the error norm; word 1: negative when a dense-output launch gave up
         self._host = torch.zeros(4, dtype=torch.float64).pin_memory()
+        self._words = self._host.numpy()
+        self._wait_mcycles = 0           # limit of a wait; 0: the library's
         self._coefs = torch.empty(_lib.QG_COEF_TABLE, dtype=torch.float64, device=dev)
         self.y_prev, self.y_front = self._ya, self._yb
         # mixed form: complex64 copies of y_prev / y_front (stage inputs), swapped with them
@@ -228,6 +233,7 @@ class GpuVern7:
         if not self._set:
             self.status = NOT_INITIATED
             return
+        self._check_waits()
         gen = self._generator()
         if gen is not None:
             self._drive("qg_vern7_integrate", gen, t, int(step))
@@ -286,7 +292,8 @@ class GpuVern7:
                           self.rtol, self.min_step, self.max_step, self.max_numsteps,
                           self.stats["steps"], self.stats["rejected"], self.stats["rhs"], 0,
                           self.status, int(self.interpolate), int(self._out[0] == "interp"), 0,
-                          self._barrier_base.value, 0, self.counter.data_ptr() + 4,
+                          self._barrier_base.value, self._wait_mcycles,
+                          self.counter.data_ptr() + 4,
                           self._host.data_ptr(), self._coefs.data_ptr())
         rc = getattr(_lib.load(), name)(C.byref(gen), C.byref(rk), C.byref(c), *args, stream_ptr())
         _lib.LAUNCHES[0] += c.launches
@@ -296,10 +303,8 @@ class GpuVern7:
         self.dt_safe, self.dt_int, self.status = c.dt_safe, c.dt_int, c.status
         self.stats.update(steps=c.steps, rejected=c.rejected, rhs=c.rhs)
         self._barrier_base.value = c.barrier_base
-        if rc != _lib.QG_OK and c.status == _lib.QG_DEVICE_WAIT:
-            self.counter.zero_()
-            self._barrier_base.value = 0
-            raise IntegratorError(_lib.load().qg_last_error().decode())
+        if rc != _lib.QG_OK and c.status == DEVICE_WAIT:
+            self._wait_gave_up()
         _lib.check(rc, name)
         if c.status >= 0:
             if c.interp:
@@ -309,10 +314,12 @@ class GpuVern7:
 
     def run_dm(self, tlist, ops, d: int, out: torch.Tensor) -> bool:
         """Integrate to each of ``tlist`` and record ``ops``' expectation values, one row of
-        ``out`` per time, up to the first failure; False when the loops here must do it."""
+        ``out`` per time, up to the first failure; False when the loops here must do it.
+        :meth:`check` after ``out`` was read tells whether all of it is valid."""
         gen = self._generator()
         if gen is None or not self._set:
             return False
+        self._check_waits()
         tl = np.ascontiguousarray(tlist, dtype=np.float64)
         self._drive("qg_vern7_run_dm", gen, tl.ctypes.data, len(tl), C.byref(ops.struct), d,
                     out.data_ptr())
@@ -352,11 +359,22 @@ class GpuVern7:
         self.t_front = self.t_prev + dt
         error = self._read_result()
         if fused and error < 0:
-            self.counter.zero_()
-            self._barrier_base.value = 0
-            raise IntegratorError("a device wait of the fused step kernel gave up; the GPU may "
-                                  "be unhealthy")
+            self._wait_gave_up()
         return error
+
+    def _check_waits(self):
+        """Raise when a wait of an earlier dense-output launch gave up (its stages hold NaN)."""
+        if self._words[1] < 0:
+            self._wait_gave_up()
+
+    def _wait_gave_up(self):
+        torch.cuda.current_stream().synchronize()   # every block has left and written its word
+        self.counter.zero_()
+        self._barrier_base.value = 0
+        self._words[1] = 0.0
+        self.status = DEVICE_WAIT
+        self._set = False                           # no step to go on from
+        raise IntegratorError(STATUS_MESSAGES[DEVICE_WAIT])
 
     def _stage(self):
         """The operator's stage launch, by half where that applies."""
@@ -379,6 +397,7 @@ class GpuVern7:
         # explicit_rk.pyx:399-410
         dt = self.dt_int
         rk = self._rk()
+        rk.result = self._host.data_ptr() + 8       # written when a wait gives up
         s = stream_ptr()
         if not self._range(rk, T.RK_STEP, T.RK_EXTRA_STEP, dt, s):
             self._combine(self._stage_base(),
@@ -429,9 +448,10 @@ class GpuVern7:
 
     # -- outputs ------------------------------------------------------------
     def successful(self) -> bool:
-        return self.status >= 0
+        return self.status >= 0 and self._words[1] >= 0
 
     def check(self):
+        self._check_waits()
         if not self.successful():
             raise IntegratorError(STATUS_MESSAGES[self.status])
 
