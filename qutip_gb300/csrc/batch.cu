@@ -1535,16 +1535,6 @@ static bool warp_mode(int64_t max_n, int group) {
   return group == QG_GROUP_WARP || (group == QG_GROUP_AUTO && max_n <= WARP_MAX_N);
 }
 
-// Opt a kernel into `bytes` of dynamic shared memory.  The 48 KB default limit counts the
-// kernel's static shared memory too (the per-warp factor slices: up to 5.6 KB), so any
-// dynamic size is opted in: 45.7 KB of staged vectors plus the slices had 0 blocks per SM.
-template <typename K>
-static bool allow_smem(K kernel, int64_t bytes) {
-  if (bytes <= 0) return true;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) ==
-         cudaSuccess;
-}
-
 static bool valid_group(int group) {
   return group == QG_GROUP_AUTO || group == QG_GROUP_WARP || group == QG_GROUP_CTA ||
          group == QG_GROUP_CLUSTER || group == QG_GROUP_CTA128;
@@ -1710,7 +1700,7 @@ static int group_slots(int64_t max_n, int dtype, int group, int64_t smem) {
   }
   if (smem > MAX_DYN_SMEM) return set_error(QG_ERR_ARG, "staged data exceed shared memory");
   const Shape sh = shape_of(max_n, dtype, group);
-  if (!allow_smem(sh.kernel, smem)) return set_error(QG_ERR_CUDA, "shared-memory opt-in failed");
+  if (!allow_smem((const void*)sh.kernel, (size_t)smem)) return set_error(QG_ERR_CUDA, "shared-memory opt-in failed");
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sh.kernel, sh.block, smem);
   if (e != cudaSuccess || per_sm <= 0) {
     char msg[200];
@@ -1779,7 +1769,7 @@ extern "C" int qg_batch_vern7(const qg_batch* B, void* stream) {
   }
   const Shape sh = shape_of(B->max_n, B->dtype, B->group);
   const int64_t smem = launch_smem(*B);
-  if (!allow_smem(sh.kernel, smem)) return set_error(QG_ERR_CUDA, "shared-memory opt-in failed");
+  if (!allow_smem((const void*)sh.kernel, (size_t)smem)) return set_error(QG_ERR_CUDA, "shared-memory opt-in failed");
   const int grid = (B->n_slots + sh.groups_per_cta - 1) / sh.groups_per_cta;
   sh.kernel<<<grid, sh.block, smem, st>>>(*B);
   return check_launch("batch_vern7 (warp or CTA groups)");

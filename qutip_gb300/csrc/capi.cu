@@ -2,6 +2,9 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <map>
+#include <utility>
+
 #include "capi_internal.h"
 #include "common.cuh"
 
@@ -32,6 +35,38 @@ int sm_count() {
     cache[dev] = v;
   }
   return cache[dev];
+}
+
+bool allow_smem(const void* kernel, size_t bytes) {
+  if (bytes == 0) return true;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, size_t> allowed;
+  std::lock_guard<std::mutex> lock(mu);
+  size_t& most = allowed[{dev, kernel}];
+  if (bytes <= most) return true;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
+      cudaSuccess) {
+    cudaGetLastError();  // reported by the caller, not by the next launch
+    return false;
+  }
+  most = bytes;
+  return true;
+}
+
+int launch_occupancy(const void* kernel, int block, size_t smem, OccCache& c) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= OCC_MAX_DEVICES) return -1;
+  std::lock_guard<std::mutex> lock(c.mu);
+  if (c.occ[dev] > 0 && c.smem[dev] == smem) return c.occ[dev];
+  if (!allow_smem(kernel, smem)) return -1;
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem) != cudaSuccess)
+    return -1;
+  c.smem[dev] = smem;
+  c.occ[dev] = per_sm;
+  return per_sm;
 }
 
 }  // namespace qg

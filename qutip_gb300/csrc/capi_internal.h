@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <mutex>
+
 #include "qutip_gb300.h"
 
 namespace qg {
@@ -11,6 +13,21 @@ int set_error(int code, const char* msg);
 int check_launch(const char* what);
 // Multiprocessor count of the current device (cached per device).
 int sm_count();
+// Opt a kernel into `bytes` of dynamic shared memory on the current device.  Any size is opted
+// in: the 48 KB default counts a kernel's static shared memory too (17 KB of tiles or 5.6 KB of
+// factor slices had launches of 32 to 47 KB refused).  The limit only grows: host threads
+// with launches of different sizes would otherwise lower it between one another's call and
+// launch.
+bool allow_smem(const void* kernel, size_t bytes);
+// The same, and the resident blocks per SM (<= 0 on failure).  The caller keeps one cache
+// per kernel instantiation, an entry per device, shared by host threads under its mutex.
+constexpr int OCC_MAX_DEVICES = 64;
+struct OccCache {
+  std::mutex mu;
+  int occ[OCC_MAX_DEVICES] = {};
+  size_t smem[OCC_MAX_DEVICES] = {};
+};
+int launch_occupancy(const void* kernel, int block, size_t smem, OccCache& c);
 // Validate a grouped operator (shape, layout and tables); QG_OK or an error code.
 int check_groups(const qg_csr_groups* A);
 // The same for an operator of the Hermitian half form on d x d states.

@@ -253,27 +253,14 @@ __global__ void __launch_bounds__(HERM_BLOCK, HermBounds<DT>::MIN_BLOCKS)
   if (last) finish_error<HERM_BLOCK>(rk, err_acc, red);
 }
 
-static int herm_occupancy(const void* kern, size_t smem) {
-  // one launch shape per (device, kernel, table size): asked for at every launch, as the
-  // tables' size differs between operators (a host query of about a microsecond).  Any size is
-  // opted in: the 48 KB default counts the 9 to 17 KB of static shared memory too.
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return -1;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, HERM_BLOCK, smem) !=
-      cudaSuccess)
-    return -1;
-  return per_sm;
-}
-
 template <int DT, int YDT, int CB>
 static int launch_herm(cudaStream_t st, const qg_csr_groups& A, int d, double t, const void* x,
                        const RkArgs& rk) {
   using ST = typename elem<DT>::T;
   auto kern = vern7_herm_kernel<DT, YDT, CB, DT == QG_C128>;
   const size_t smem = ((size_t)A.lanes * (sizeof(ST) + sizeof(int)) + 15) & ~(size_t)15;
-  const int per_sm = herm_occupancy((const void*)kern, smem);
+  static OccCache cache;  // one per instantiation
+  const int per_sm = launch_occupancy((const void*)kern, HERM_BLOCK, smem, cache);
   if (per_sm <= 0) return set_error(QG_ERR_ARG, "dictionary does not fit in shared memory");
   const int64_t nt = d / 32;
   int64_t grid = (int64_t)sm_count() * per_sm;

@@ -623,7 +623,7 @@ static int launch_sde_rows(const qg_sde& S, int n_traj, double2* states, const d
                            int n_steps, double dt, const SdeRowShape& sh, cudaStream_t st) {
   const int smem = sh.vecs + sh.ops;
   auto kern = sde_row_kernel<M, OPEN, SCHEME, NT>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+  if (!allow_smem((const void*)kern, (size_t)smem))
     return set_error(QG_ERR_CUDA, "stochastic kernel: shared memory opt-in failed");
   kern<<<(n_traj - 1) / sh.T + 1, sh.threads, smem, st>>>(S, n_traj, states, dW, n_steps, dt, sh.T,
                                                          sh.ops);

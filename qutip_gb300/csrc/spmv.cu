@@ -655,33 +655,6 @@ __global__ void __launch_bounds__(LB_BLOCK)
 }
 
 // ------------------------------------------------------------------ launch --
-// Opt `kernel` into `smem` bytes of dynamic shared memory and return its
-// resident blocks per SM.  The caller keeps one cache per kernel instantiation; it
-// holds one entry per device (the attribute is set with that device current) and is
-// shared by host threads under its mutex.
-constexpr int OCC_MAX_DEVICES = 64;
-struct OccCache {
-  std::mutex mu;
-  int occ[OCC_MAX_DEVICES] = {};
-  size_t smem[OCC_MAX_DEVICES] = {};
-};
-template <typename K>
-static int staged_occupancy(K kernel, int block, size_t smem, OccCache& c) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= OCC_MAX_DEVICES) return -1;
-  std::lock_guard<std::mutex> lock(c.mu);
-  if (c.occ[dev] > 0 && c.smem[dev] == smem) return c.occ[dev];
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return -1;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem) != cudaSuccess)
-    return -1;
-  c.smem[dev] = smem;
-  c.occ[dev] = per_sm;
-  return per_sm;
-}
-
 template <int DT, int YDT, int EPI, int LANES>
 static int launch_staged(cudaStream_t st, const qg_csr_groups& A, double t, const void* x,
                          const AxpbyArgs& ax, const RkArgs& rk) {
@@ -692,7 +665,7 @@ static int launch_staged(cudaStream_t st, const qg_csr_groups& A, double t, cons
   const size_t smem = 2 * sb;
   auto kern = spmv_staged_kernel<DT, YDT, LANES, EPI, BLOCK>;
   static OccCache cache;  // one per instantiation of this function (and so of kern)
-  const int per_sm = staged_occupancy(kern, BLOCK, smem, cache);
+  const int per_sm = launch_occupancy((const void*)kern, BLOCK, smem, cache);
   if (per_sm <= 0) return set_error(QG_ERR_ARG, "staged tile does not fit in shared memory");
   int64_t grid = (int64_t)sm_count() * per_sm;
   if (grid > A.n_tiles) grid = A.n_tiles;
@@ -708,7 +681,7 @@ static int launch_dict(cudaStream_t st, const qg_csr_groups& A, double t, const 
   auto kern = spmv_dict_kernel<DT, YDT, EPI, CB, RI>;
   const size_t smem = ((size_t)A.lanes * (sizeof(ST) + sizeof(int)) + 15) & ~(size_t)15;
   static OccCache cache;  // one per instantiation
-  const int per_sm = staged_occupancy(kern, DICT_BLOCK, smem, cache);
+  const int per_sm = launch_occupancy((const void*)kern, DICT_BLOCK, smem, cache);
   if (per_sm <= 0) return set_error(QG_ERR_ARG, "dictionary does not fit in shared memory");
   int64_t grid = (int64_t)sm_count() * per_sm;
   // at least four slices to a block: every block fetches the tables
@@ -749,7 +722,7 @@ static int launch_any(cudaStream_t st, const qg_csr_groups& A, double t, const v
     // per fused stage on the L=10 Liouvillian, so only the 4-entry variant is built.)
     auto kern = spmv_sliced_kernel<DT, YDT, EPI, 4>;
     static OccCache cache;  // one per instantiation
-    const int per_sm = staged_occupancy(kern, SPMV_BLOCK, 0, cache);
+    const int per_sm = launch_occupancy((const void*)kern, SPMV_BLOCK, 0, cache);
     if (per_sm <= 0) return set_error(QG_ERR_CUDA, "occupancy query failed");
     int64_t warps_needed = A.n_tiles;
     int64_t blocks = (warps_needed * 32 + SPMV_BLOCK - 1) / SPMV_BLOCK;
@@ -800,7 +773,7 @@ static int launch_lindblad(cudaStream_t st, const qg_lindblad& L, double t, cons
   if (L.hermitian) return launch_lindblad_herm<DT, YDT, EPI>(st, L, t, x, ax, rk);
   auto kern = lindblad_kernel<DT, YDT, EPI>;
   static OccCache cache;  // one per instantiation
-  const int per_sm = staged_occupancy(kern, LB_BLOCK, 0, cache);
+  const int per_sm = launch_occupancy((const void*)kern, LB_BLOCK, 0, cache);
   if (per_sm <= 0) return set_error(QG_ERR_CUDA, "occupancy query failed");
   const int64_t n = L.d * L.d;
   const int64_t blocks = (n + LB_BLOCK - 1) / LB_BLOCK;
