@@ -271,6 +271,12 @@ typedef struct qg_vern7_ctl {
                               dense-output launch gives up */
   double* coef_table;      /* QG_COEF_TABLE doubles (device) for the coefficients of a step's
                               stages; NULL: each stage evaluates its own */
+  double slice;    /* seconds after which a call returns between steps or outputs, with paused
+                      set, so that the caller can look at its signals; 0: never.  The same
+                      call with the same arguments goes on from there. */
+  int64_t left;    /* steps left to the paused integration */
+  int32_t paused;  /* 1: inside an integration, 2: between outputs; 0 for a new call */
+  int32_t n_done;  /* outputs recorded (qg_vern7_run_dm) */
 } qg_vern7_ctl;
 
 /* ---- library ---------------------------------------------------------- */

@@ -96,7 +96,8 @@ class Vern7Ctl(C.Structure):
         ("rhs", C.c_int64), ("launches", C.c_int64), ("status", C.c_int32),
         ("interpolate", C.c_int32), ("interp", C.c_int32), ("swaps", C.c_int32),
         ("barrier_base", C.c_uint32), ("wait_mcycles", C.c_int32), ("barrier", C.c_void_p),
-        ("host_result", C.c_void_p), ("coef_table", C.c_void_p)]
+        ("host_result", C.c_void_p), ("coef_table", C.c_void_p), ("slice", C.c_double),
+        ("left", C.c_int64), ("paused", C.c_int32), ("n_done", C.c_int32)]
 
 
 QG_GEN_CSR, QG_GEN_LINDBLAD, QG_GEN_DENSE = 0, 1, 2

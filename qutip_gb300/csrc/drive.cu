@@ -10,6 +10,7 @@
 #include <math.h>
 
 #include <atomic>
+#include <chrono>
 
 #include "capi_internal.h"
 #include "common.cuh"
@@ -55,6 +56,15 @@ struct Drive {
   qg_rk_buffers* B;
   qg_vern7_ctl* c;
   void* stream;
+
+  using Clock = std::chrono::steady_clock;
+  const Clock::time_point start = Clock::now();
+  // Whether the call has run for its slice of time: a caller that waits for signals (an
+  // interrupt) gets them between calls.
+  bool late() const {
+    return c->slice > 0.0 &&
+           std::chrono::duration<double>(Clock::now() - start).count() >= c->slice;
+  }
 
   int n_coefs = 0;  // coefficients of a stage in the table; 0: no table
 
@@ -236,24 +246,29 @@ struct Drive {
 
   // integrate (explicit_rk.pyx:278-331)
   int integrate(double t, int step) {
-    if (t == c->t) return QG_OK;
-    if (t < c->t_prev) {
-      c->status = QG_OUTSIDE_RANGE;
-      return QG_OK;
-    }
-    if (c->interpolate && t < c->t_front) {
-      if (c->status != QG_INTERPOLATED) {
-        const int rc = dense_out();
-        if (rc != QG_OK) return rc;
-        c->status = QG_INTERPOLATED;
+    int64_t left = c->left;
+    if (c->paused == 1) {
+      c->paused = 0;  // goes on in the loop below
+    } else {
+      if (t == c->t) return QG_OK;
+      if (t < c->t_prev) {
+        c->status = QG_OUTSIDE_RANGE;
+        return QG_OK;
       }
-      c->interp = 1;
-      c->t = t;
-      return QG_OK;
+      if (c->interpolate && t < c->t_front) {
+        if (c->status != QG_INTERPOLATED) {
+          const int rc = dense_out();
+          if (rc != QG_OK) return rc;
+          c->status = QG_INTERPOLATED;
+        }
+        c->interp = 1;
+        c->t = t;
+        return QG_OK;
+      }
+      left = c->max_numsteps;
+      c->status = QG_NORMAL;
+      if (step && c->t < c->t_front && t > c->t_front) t = c->t_front;
     }
-    int64_t left = c->max_numsteps;
-    c->status = QG_NORMAL;
-    if (step && c->t < c->t_front && t > c->t_front) t = c->t_front;
     while (c->t_front < t && c->status >= 0) {
       swap();
       c->t_prev = c->t_front;
@@ -262,6 +277,11 @@ struct Drive {
       if (rc != QG_OK) return rc;
       left -= n;
       if (step) break;
+      if (c->t_front < t && c->status >= 0 && late()) {
+        c->left = left;
+        c->paused = 1;
+        return QG_OK;
+      }
     }
     if (c->status < 0) return QG_OK;
     if (c->t_front > t) {
@@ -313,16 +333,23 @@ extern "C" int qg_vern7_run_dm(const qg_generator* gen, qg_rk_buffers* B, qg_ver
   v.base_dtype = B->state_dtype;
   v.k_dtype = B->stage_dtype;
   v.k = B->k;
-  for (int i = 0; i < n_times;) {
+  int i = c->paused ? c->n_done : 0;
+  if (c->paused == 2) c->paused = 0;
+  while (i < n_times) {
     rc = dr.integrate(tlist[i], 0);
-    if (rc != QG_OK || c->status < 0) return rc;
+    c->n_done = i;
+    if (rc != QG_OK || c->status < 0 || c->paused) return rc;
     ++c->launches;
     if (c->status != QG_INTERPOLATED) {
       // the state at the end of a step, or the time asked for again
       v.base = B->y_front;
       rc = qg_expect_dm(ops, d, &v, out + i * row, stream);
       if (rc != QG_OK) return rc;
-      ++i;
+      c->n_done = ++i;
+      if (i < n_times && dr.late()) {
+        c->paused = 2;
+        return QG_OK;
+      }
       continue;
     }
     // every following output time inside this step is read from its dense output
@@ -338,7 +365,11 @@ extern "C" int qg_vern7_run_dm(const qg_generator* gen, qg_rk_buffers* B, qg_ver
                             stream);
     if (rc != QG_OK) return rc;
     c->t = tlist[i + m - 1];
-    i += m;
+    c->n_done = i += m;
+    if (i < n_times && dr.late()) {
+      c->paused = 2;
+      return QG_OK;
+    }
   }
   return QG_OK;
 }

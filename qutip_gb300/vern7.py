@@ -105,6 +105,7 @@ class GpuVern7:
         self._host = torch.zeros(4, dtype=torch.float64).pin_memory()
         self._words = self._host.numpy()
         self._wait_mcycles = 0           # limit of a wait; 0: the library's
+        self._slice = 0.05               # seconds between looks at the interpreter's signals
         self._coefs = torch.empty(_lib.QG_COEF_TABLE, dtype=torch.float64, device=dev)
         self.y_prev, self.y_front = self._ya, self._yb
         # mixed form: complex64 copies of y_prev / y_front (stage inputs), swapped with them
@@ -295,14 +296,15 @@ class GpuVern7:
                           self._barrier_base.value, self._wait_mcycles,
                           self.counter.data_ptr() + 4,
                           self._host.data_ptr(), self._coefs.data_ptr())
-        rc = getattr(_lib.load(), name)(C.byref(gen), C.byref(rk), C.byref(c), *args, stream_ptr())
-        _lib.LAUNCHES[0] += c.launches
-        if c.swaps:
-            self._swap()
-        self.t, self.t_prev, self.t_front = c.t, c.t_prev, c.t_front
-        self.dt_safe, self.dt_int, self.status = c.dt_safe, c.dt_int, c.status
-        self.stats.update(steps=c.steps, rejected=c.rejected, rhs=c.rhs)
-        self._barrier_base.value = c.barrier_base
+        c.slice = self._slice
+        run = getattr(_lib.load(), name)
+        while True:                   # an interrupt is raised between the calls
+            try:
+                rc = run(C.byref(gen), C.byref(rk), C.byref(c), *args, stream_ptr())
+            finally:
+                self._take(c)
+            if not c.paused:
+                break
         if rc != _lib.QG_OK and c.status == DEVICE_WAIT:
             self._wait_gave_up()
         _lib.check(rc, name)
@@ -311,6 +313,17 @@ class GpuVern7:
                 self._set_interp(self.t)
             else:
                 self._out = ("front", None)
+
+    def _take(self, c):
+        """The scalar state after a call of the library's driver."""
+        _lib.LAUNCHES[0] += c.launches
+        if c.swaps:
+            self._swap()
+        c.launches = c.swaps = 0
+        self.t, self.t_prev, self.t_front = c.t, c.t_prev, c.t_front
+        self.dt_safe, self.dt_int, self.status = c.dt_safe, c.dt_int, c.status
+        self.stats.update(steps=c.steps, rejected=c.rejected, rhs=c.rhs)
+        self._barrier_base.value = c.barrier_base
 
     def run_dm(self, tlist, ops, d: int, out: torch.Tensor) -> bool:
         """Integrate to each of ``tlist`` and record ``ops``' expectation values, one row of
