@@ -276,12 +276,14 @@ class GpuVern7:
     # -- the same loop in the library ---------------------------------------
     def _generator(self):
         """The operator as the library's driver takes it (``qg_vern7_integrate``); None for
-        an operator that is not one of the library's own, which the loops here then drive."""
+        an operator that is not one of the library's own or whose ``vern7_stage`` was replaced,
+        which the loops here then drive."""
         from .dense import DenseLindbladOperator
         from .lindblad import LindbladOperator
+        cls = type(self.op)
         kind = {DeviceOperator: _lib.QG_GEN_CSR, LindbladOperator: _lib.QG_GEN_LINDBLAD,
-                DenseLindbladOperator: _lib.QG_GEN_DENSE}.get(type(self.op))
-        if kind is None:
+                DenseLindbladOperator: _lib.QG_GEN_DENSE}.get(cls)
+        if kind is None or not self._stages_of(cls):
             return None
         return _lib.Generator(kind, 0, C.addressof(self.op.struct),
                               math.isqrt(self.n) if self._half() else 0)
@@ -393,18 +395,25 @@ class GpuVern7:
         """The operator's stage launch, by half where that applies."""
         return self.op.vern7_stage_herm if self._half() else self.op.vern7_stage
 
+    def _stages_of(self, cls) -> bool:
+        """Whether the operator's stages are those of ``cls``: a subclass or an object with a
+        ``vern7_stage`` of its own gets every stage through it."""
+        return getattr(self.op.vern7_stage, "__func__", None) is cls.vern7_stage
+
     def _half(self) -> bool:
         """Whether the state is a Hermitian density matrix that the generator keeps Hermitian
         (the coefficients may have been replaced since the state was set, so their part is
         looked at again)."""
-        return self._hermitian and self.op.real_coefficients()
+        return (self._hermitian and self.op.real_coefficients()
+                and self._stages_of(DeviceOperator))
 
     def _range(self, rk, stage0, stage1, dt, s) -> bool:
         """The stages in one launch where the operator's rows all fit the GPU at once."""
-        name = "vern7_range_herm" if self._half() else "vern7_range"
-        run = getattr(self.op, name, None)
-        return run is not None and run(rk, stage0, stage1, self.t_prev, dt, self.atol, self.rtol,
-                                       self.counter.data_ptr() + 4, self._barrier_base, s)
+        if not self._stages_of(DeviceOperator):
+            return False
+        run = self.op.vern7_range_herm if self._half() else self.op.vern7_range
+        return run(rk, stage0, stage1, self.t_prev, dt, self.atol, self.rtol,
+                   self.counter.data_ptr() + 4, self._barrier_base, s)
 
     def _prep_dense_out(self):
         # explicit_rk.pyx:399-410
