@@ -76,7 +76,8 @@ class GpuVern7:
         self.op = op
         self.precision = precision
         self.atol, self.rtol = float(atol), float(rtol)
-        self.max_numsteps = int(nsteps)
+        # 64 bits in the library: what no integration counts to is as good as any larger limit
+        self.max_numsteps = max(min(int(nsteps), 2**63 - 1), -2**63)
         self.first_step = float(first_step)
         self.min_step = float(min_step) or 1e-15       # explicit_rk.pyx:133
         self.max_step = float(max_step)
