@@ -55,7 +55,7 @@ __device__ __forceinline__ double max_part(float2 v) {
 // row (r, c) without its conjugate at the mirrored place of row (c, r)), or rho is not
 // Hermitian.  Entries are compared to the rounding of their row's largest value (the sums
 // of a Liouvillian's terms round differently at mirrored places), rho element by element;
-// a NaN or an infinity counts as not Hermitian.
+// a NaN or an infinity, in either, counts as not Hermitian.
 template <int DT, int XDT, int CB, bool RI>
 __global__ void __launch_bounds__(HERM_BLOCK)
     hermitian_check_kernel(qg_csr_groups A, int d, const typename elem<XDT>::T* x, int* flag) {
@@ -74,7 +74,8 @@ __global__ void __launch_bounds__(HERM_BLOCK)
     {
       const auto p = x[row], q = x[mrow];
       const double tol = relx * max_part(p);
-      ok = fabs((double)p.x - (double)q.x) <= tol && fabs((double)p.y + (double)q.y) <= tol;
+      ok = isfinite(tol) && fabs((double)p.x - (double)q.x) <= tol &&
+           fabs((double)p.y + (double)q.y) <= tol;
     }
     for (int g = 0; g < A.n_groups && ok; ++g) {
       const int t0 = __ldg(A.dict_start + g), tn = __ldg(A.dict_start + g + 1) - t0;
@@ -83,7 +84,11 @@ __global__ void __launch_bounds__(HERM_BLOCK)
       double top = 0.0;
       for (int j = 0; j < w; ++j) {
         const int k = code_at<CB>(A, codes, g, row, j);
-        if (k > 0 && k < tn) top = fmax(top, max_part(tval[t0 + k]));
+        if (k <= 0 || k >= tn) continue;
+        const ST v = tval[t0 + k];
+        top = fmax(top, max_part(v));
+        // a NaN beside a zero does not show in the maximum, an infinity leaves no tolerance
+        if (!isfinite(v.x) || !isfinite(v.y)) ok = false;
       }
       const double tol = rel * top;
       for (int j = 0; j < w && ok; ++j) {
