@@ -115,6 +115,10 @@ typedef struct qg_csr_groups {
   const double* coef_consts; /* complex constants as (re, im) pairs */
   const int32_t* dict_off;   /* dictionary layouts: column - row of each table entry */
   const int32_t* dict_start; /* dictionary layouts: [n_groups+1] table bounds */
+  int32_t row_words; /* most stored entries of a row over all groups (sliced: of a slice's
+                        width; dictionary layouts: words of four codes); 0: unknown.  A launch
+                        that keeps rows in shared memory reserves for this many. */
+  int32_t pad_;
 } qg_csr_groups;
 
 /* Dia matrix in the reference's layout (qutip/core/data/dia.pxd:17-38):

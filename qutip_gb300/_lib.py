@@ -33,7 +33,7 @@ class CsrGroups(C.Structure):
                 ("col", C.c_void_p), ("val", C.c_void_p), ("tile_row", C.c_void_p),
                 ("coef_code", C.c_void_p), ("coef_start", C.c_void_p),
                 ("coef_consts", C.c_void_p), ("dict_off", C.c_void_p),
-                ("dict_start", C.c_void_p)]
+                ("dict_start", C.c_void_p), ("row_words", C.c_int32), ("pad_", C.c_int32)]
 
 
 class Lindblad(C.Structure):

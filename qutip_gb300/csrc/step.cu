@@ -42,9 +42,17 @@ enum Kind { KIND_CSR = 0, KIND_SLICED = 1, KIND_DICT1 = 2, KIND_DICT2 = 3 };
 
 constexpr int STEP_THREADS = 512;   // most threads of a block (one block per SM)
 constexpr int STEP_MIN_WARPS = 4;   // fewer warps per block only spread the barrier wider
-// entries (CSR, sliced) or code words a thread keeps in shared memory; rows longer than
+// most entries (CSR, sliced) or code words a thread keeps in shared memory; rows longer than
 // that read the rest from global memory at every stage
 constexpr int STEP_KEEP = 32;
+// A thread's share of the longest row, where that is known: the launch waits until all its
+// blocks fit beside whatever else the GPU runs, so it takes no more than it uses (the
+// four-entry rows of a Jaynes-Cummings system: 27 KB a block where 32 entries take 98).
+static int step_keep(const qg_csr_groups& A, int kind, int lanes) {
+  if (A.row_words <= 0) return STEP_KEEP;
+  const int most = kind == KIND_CSR ? (A.row_words + A.n_groups * (lanes - 1)) / lanes : A.row_words;
+  return most < STEP_KEEP ? most : STEP_KEEP;
+}
 constexpr int HERM_WARPS = 8;       // a unit of the half form: 32 rows x 8 columns
 constexpr long long STEP_WAIT_CYCLES = 16 * WAIT_CYCLES;  // the GPU may be shared meanwhile
 
@@ -508,11 +516,10 @@ static int launch_range(StepArgs& a, uint32_t* bar_base, cudaStream_t st) {
   if (per * 32 > STEP_THREADS) return 1;
   const int threads = (int)per * 32, rows = threads / LANES;
   const int grid = (int)((warps + per - 1) / per);
-  int smem = 0;
-  for (a.keep = STEP_KEEP; a.keep >= 2; a.keep /= 2) {
-    smem = step_smem<ST>(a.A, KIND, threads, rows, a.keep, HERM).total;
-    if (smem <= STEP_MAX_SMEM) break;
-  }
+  a.keep = step_keep(a.A, KIND, LANES);
+  auto bytes = [&] { return step_smem<ST>(a.A, KIND, threads, rows, a.keep, HERM).total; };
+  int smem = bytes();
+  for (; smem > STEP_MAX_SMEM && a.keep > 2; smem = bytes()) a.keep = a.keep > 4 ? a.keep / 2 : 2;
   if (smem > STEP_MAX_SMEM) return 1;
   auto kern = vern7_range_kernel<DT, YDT, KIND, LANES, PARTS, HERM>;
   static std::mutex mu;

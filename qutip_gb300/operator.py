@@ -292,6 +292,12 @@ def row_tiles(row_start, tile_nnz, max_rows):
     return np.asarray(out, dtype=np.int32)
 
 
+def _longest(parts, n_groups: int) -> int:
+    """Most of a row or slice: ``parts`` holds its ``n_groups`` groups side by side (numpy, or a
+    device tensor, whose answer is read back)."""
+    return int(parts.reshape(-1, n_groups).sum(1).max()) if len(parts) else 0
+
+
 class DeviceOperator:
     """``A(t) = sum_g c_g(t) A_g`` resident on the GPU.
 
@@ -350,6 +356,7 @@ class DeviceOperator:
             rp, widths, codes, cb, t_off, t_val, t_start, total = lay
             self.stored = total
             self.code_bytes = cb
+            self.row_words = _longest((widths + 3) // 4, G)
             self.slice_width = torch.from_numpy(widths).to(self.device)
             self.row_ptr = torch.from_numpy(rp.astype(np.int32)).to(self.device)
             self.col = torch.from_numpy(codes if cb == 1 else codes.view(np.int16)).to(self.device)
@@ -361,10 +368,12 @@ class DeviceOperator:
         if fmt == "sliced":
             rp, widths, col, val, total = sliced_layout(mats, self.n_cols)
             self.stored = total
+            self.row_words = _longest(widths, G)
             self.slice_width = torch.from_numpy(widths).to(self.device)
         else:
             rp, col, val = row_major_layout(mats)
             self.stored = len(col)
+            self.row_words = _longest(np.diff(rp), G)
             self.slice_width = None
         if self.stored >= 2**31 - 16 or self.n_rows * G >= 2**31 - 16:
             raise ValueError("operators beyond 2^31 stored entries need 64-bit indices")
@@ -436,6 +445,7 @@ class DeviceOperator:
             self.fmt = "dict"
             self.stored = total
             self.code_bytes = cb
+            self.row_words = _longest((widths + 3) // 4, len(groups))
             self.slice_width = widths
             self.row_ptr, self.col, self.val = rp, codes, t_val.to(_TORCH[dtype])
             self.dict_off, self.dict_start = t_off, t_start
@@ -447,6 +457,7 @@ class DeviceOperator:
         if total >= 2**31 - 16 or n * len(groups) >= 2**31 - 16:
             raise ValueError("operators beyond 2^31 stored entries need 64-bit indices")
         self.stored = total
+        self.row_words = _longest(widths, len(groups))
         self.slice_width = widths
         self.row_ptr = torch.zeros(rp.numel() + P, dtype=torch.int32, device=self.device)
         self.row_ptr[:rp.numel()] = rp.to(torch.int32)
@@ -506,7 +517,7 @@ class DeviceOperator:
             self.n_rows, self.n_cols, G, _QG[dtype], layout, 4, 0, 0,
             _ptr(self.row_ptr), _ptr(self.col), _ptr(self.val), None, _ptr(self.coef_code),
             _ptr(self.coef_start), _ptr(self.coef_consts), _ptr(self.dict_off),
-            _ptr(self.dict_start))
+            _ptr(self.dict_start), self.row_words, 0)
         self.set_launch(self.default_launch())
 
     def _choose_format(self, mats) -> str:
