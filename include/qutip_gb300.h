@@ -407,7 +407,9 @@ typedef struct qg_sde {
   int32_t open;     /* 0: SSE (ket), 1: SME (vec(rho), column-stacked) */
   int32_t n_sc;     /* stochastic operators (1..QG_MAX_COPS) */
   int32_t d;        /* Hilbert-space dimension */
-  int32_t reserved; /* 0 */
+  int32_t op_bytes; /* shared memory that holds every operator, each with its rows padded to
+                       its longest: sum of longest * n * 20 rounded up to 16; 0: unknown.  A
+                       launch that keeps operators there reserves no more. */
   const int32_t* l_rp;
   const int32_t* l_col;
   const void* l_val;
@@ -425,11 +427,11 @@ int64_t qg_sde_work_values(int64_t n, int32_t n_sc);
 
 /* The shape a launch of n_traj trajectories takes on a GPU of n_sms multiprocessors when
  * every trajectory runs on one thread per entry: shape = {trajectories of a CTA, threads of
- * a CTA, bytes of shared memory for their vectors, bytes for operators}.  Returns 1 when
- * the states are too long or the operators too many for that kernel.  Host arithmetic
- * only. */
+ * a CTA, bytes of shared memory for their vectors, bytes for operators (op_bytes as in
+ * qg_sde)}.  Returns 1 when the states are too long or the operators too many for that
+ * kernel.  Host arithmetic only. */
 int qg_sde_row_shape(int64_t n, int32_t n_sc, int32_t open, int32_t n_traj, int32_t n_sms,
-                     int32_t* shape);
+                     int32_t op_bytes, int32_t* shape);
 
 /* n_steps Platen steps of dt for each of n_traj trajectories (one CTA each): states holds
  * n_traj complex128 states of length n (updated in place); dW holds the Wiener increments,

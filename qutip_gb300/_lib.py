@@ -51,7 +51,7 @@ class Lindblad(C.Structure):
 
 class Sde(C.Structure):
     _fields_ = [("n", C.c_int64), ("open", C.c_int32), ("n_sc", C.c_int32), ("d", C.c_int32),
-                ("reserved", C.c_int32), ("l_rp", C.c_void_p), ("l_col", C.c_void_p),
+                ("op_bytes", C.c_int32), ("l_rp", C.c_void_p), ("l_col", C.c_void_p),
                 ("l_val", C.c_void_p), ("c_rp", C.c_void_p), ("c_col", C.c_void_p),
                 ("c_val", C.c_void_p), ("m_rp", C.c_void_p), ("m_col", C.c_void_p),
                 ("m_val", C.c_void_p), ("work", C.c_void_p)]
@@ -146,7 +146,8 @@ _SIGS = {
     "qg_dense_lindblad_stage": (C.c_int, [_P(DenseLindblad), _P(RkBuffers), C.c_int, C.c_double,
                                           C.c_double, C.c_double, C.c_double, C.c_void_p]),
     "qg_sde_work_values": (C.c_int64, [C.c_int64, C.c_int32]),
-    "qg_sde_row_shape": (C.c_int, [C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_void_p]),
+    "qg_sde_row_shape": (C.c_int, [C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
+                                   C.c_void_p]),
     "qg_sde_platen": (C.c_int, [_P(Sde), C.c_int32, C.c_void_p, C.c_void_p, C.c_int32,
                                 C.c_double, C.c_void_p]),
     "qg_sde_euler": (C.c_int, [_P(Sde), C.c_int32, C.c_void_p, C.c_void_p, C.c_int32,

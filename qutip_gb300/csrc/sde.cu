@@ -317,6 +317,10 @@ __global__ void __launch_bounds__(32 * SDE_WARPS) sde_warp_kernel(
 // Measured, 100 steps: 256 master-equation trajectories of 400 entries 5.63 -> 2.90
 // ms (29 us a step); 1000 kets of 40 entries 4.67 -> 1.58 ms.  Longer states and more
 // operators keep the kernels above: their vectors outgrow shared memory and registers.
+// A launch reserves what its operators need; a block still waits for an SM with that room (and
+// registers for up to 640 threads) to spare, so beside a batch that holds every SM in part a
+// launch of kets with a CTA each ran at once (0.35 ms for 0.23 alone), one of 400-entry states
+// or of seven kets a CTA at the batch's end, where the kernels above found room.
 // Most threads of a CTA: 96 registers for one operator, 128 for two.  CTAs of up to
 // SDE_ROW_PAIR threads with one operator are compiled for two on an SM (72 registers): one
 // alone leaves the FP64 pipe idle behind its barriers.
@@ -601,7 +605,8 @@ struct SdeRowShape {
   int T, threads, vecs, ops;
   bool pair;
 };
-static SdeRowShape sde_row_shape(int n, int d, int m, bool open, int n_traj, int sms) {
+static SdeRowShape sde_row_shape(int n, int d, int m, bool open, int n_traj, int sms,
+                                 int op_bytes) {
   const int most = m == 1 ? SDE_ROW_THREADS<1> : SDE_ROW_THREADS<2>;
   const int sums = (open ? 0 : m) + 2 * m * m;  // SDE_ROW_SUMS
   const int per = 16 * (n * (2 + 2 * m) + sums * ((open ? d : n) + (open ? 1 : 2)));
@@ -614,8 +619,11 @@ static SdeRowShape sde_row_shape(int n, int d, int m, bool open, int n_traj, int
   // the sums of kets of one entry and two operators outgrow the vectors: 576 bytes a trajectory
   if (T > SDE_ROW_SMEM / per) T = SDE_ROW_SMEM / per;
   const int vecs = T * per, room = SDE_ROW_SMEM - vecs;
-  return SdeRowShape{T, (T * n + 31) / 32 * 32, vecs,
-                     room < SDE_ROW_OP_SMEM ? room : SDE_ROW_OP_SMEM, pair};
+  // what the operators need where that is known: blocks find room beside other work and one
+  // another
+  int ops = room < SDE_ROW_OP_SMEM ? room : SDE_ROW_OP_SMEM;
+  if (op_bytes > 0 && op_bytes < ops) ops = op_bytes;
+  return SdeRowShape{T, (T * n + 31) / 32 * 32, vecs, ops, pair};
 }
 
 template <int M, bool OPEN, int SCHEME, int NT>
@@ -633,7 +641,8 @@ static int launch_sde_rows(const qg_sde& S, int n_traj, double2* states, const d
 template <bool OPEN, int SCHEME>
 static int launch_sde_rows_shape(const qg_sde& S, int n_traj, double2* states, const double* dW,
                                  int n_steps, double dt, cudaStream_t st) {
-  const SdeRowShape sh = sde_row_shape((int)S.n, S.d, S.n_sc, OPEN, n_traj, sm_count());
+  const SdeRowShape sh = sde_row_shape((int)S.n, S.d, S.n_sc, OPEN, n_traj, sm_count(),
+                                       S.op_bytes);
   if (S.n_sc == 2)
     return launch_sde_rows<2, OPEN, SCHEME, SDE_ROW_THREADS<2>>(S, n_traj, states, dW, n_steps, dt,
                                                                 sh, st);
@@ -695,14 +704,14 @@ extern "C" int64_t qg_sde_work_values(int64_t n, int32_t n_sc) {
 }
 
 extern "C" int qg_sde_row_shape(int64_t n, int32_t n_sc, int32_t open, int32_t n_traj,
-                                int32_t n_sms, int32_t* shape) {
+                                int32_t n_sms, int32_t op_bytes, int32_t* shape) {
   if (!shape) return set_error(QG_ERR_ARG, "null shape");
   if (n < 1 || n_sc < 1 || n_traj < 1 || n_sms < 1) return set_error(QG_ERR_ARG, "bad launch");
   if (n_sc > SDE_ROW_MAX_M || n > (n_sc == 1 ? SDE_ROW_THREADS<1> : SDE_ROW_THREADS<2>)) return 1;
   int d = (int)n;
   if (open)
     for (d = 1; (int64_t)d * d < n;) ++d;
-  const SdeRowShape s = sde_row_shape((int)n, d, n_sc, open != 0, n_traj, n_sms);
+  const SdeRowShape s = sde_row_shape((int)n, d, n_sc, open != 0, n_traj, n_sms, op_bytes);
   const int32_t v[4] = {s.T, s.threads, s.vecs, s.ops};
   for (int i = 0; i < 4; ++i) shape[i] = v[i];
   return QG_OK;

@@ -43,6 +43,12 @@ def _csr_blocks(mats, device):
             torch.from_numpy(m.data.astype(np.complex128)).to(device))
 
 
+def _padded_bytes(mat) -> int:
+    """Bytes of a matrix with its rows padded to the longest, as the row kernel keeps it."""
+    rows = np.diff(sp.csr_matrix(mat, dtype=np.complex128).indptr)
+    return (int(rows.max(initial=0)) * len(rows) * 20 + 15) // 16 * 16
+
+
 class SdeOperator:
     """Drift and diffusion operators of a stochastic system (ssystem.pyx:119-250).
 
@@ -70,7 +76,9 @@ class SdeOperator:
         self._work = None
         self._n_work = 0
         st = _lib.Sde()
-        st.n, st.open, st.n_sc, st.d, st.reserved = self.n, int(self.open), self.n_sc, self.d, 0
+        st.n, st.open, st.n_sc, st.d = self.n, int(self.open), self.n_sc, self.d
+        st.op_bytes = min(sum(_padded_bytes(a) for a in [L, *C_ops, *([] if open else M_ops)]),
+                          2**31 - 1)
         st.l_rp, st.l_col, st.l_val = (t.data_ptr() for t in self.L)
         st.c_rp, st.c_col, st.c_val = (t.data_ptr() for t in self.C)
         if self.M is not None:

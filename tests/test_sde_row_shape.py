@@ -22,7 +22,7 @@ def test_vectors_and_operators_fit(open_, n_sc, sms):
     for n in lengths:
         d = math.isqrt(n) if open_ else n
         for n_traj in (1, sms, 3 * sms + 1, 100 * sms, 392 * sms, 600 * sms, 2**31 - 1):
-            rc = lib.qg_sde_row_shape(n, n_sc, int(open_), n_traj, sms, shape.ctypes.data)
+            rc = lib.qg_sde_row_shape(n, n_sc, int(open_), n_traj, sms, 0, shape.ctypes.data)
             assert rc == (1 if n > (640 if n_sc == 1 else 512) else 0)
             if rc:
                 continue
@@ -34,10 +34,15 @@ def test_vectors_and_operators_fit(open_, n_sc, sms):
             need = 16 * T * ((2 + 2 * n_sc) * n + sums * (d + (1 if open_ else 2)))
             assert T >= 1 and vecs >= need and ops >= 0 and vecs + ops <= LIMIT, (n, n_traj)
             assert T * n <= threads <= (640 if n_sc == 1 else 512) and threads % 32 == 0
+            most = ops
+            for known in (16, 4096, 71 * 1024, 73 * 1024, 2**31 - 1):
+                assert lib.qg_sde_row_shape(n, n_sc, int(open_), n_traj, sms, known,
+                                            shape.ctypes.data) == 0
+                assert list(shape) == [T, threads, vecs, min(most, known)]
     assert taken > 100
-    assert lib.qg_sde_row_shape(4, 3, 0, 1, sms, shape.ctypes.data) == 1
-    assert lib.qg_sde_row_shape(0, 1, 0, 1, sms, shape.ctypes.data) == _lib.QG_ERR_ARG
-    assert lib.qg_sde_row_shape(4, 1, 0, 1, sms, None) == _lib.QG_ERR_ARG
+    assert lib.qg_sde_row_shape(4, 3, 0, 1, sms, 0, shape.ctypes.data) == 1
+    assert lib.qg_sde_row_shape(0, 1, 0, 1, sms, 0, shape.ctypes.data) == _lib.QG_ERR_ARG
+    assert lib.qg_sde_row_shape(4, 1, 0, 1, sms, 0, None) == _lib.QG_ERR_ARG
 
 
 @pytest.mark.gpu
