@@ -147,7 +147,8 @@ def _evolve(ig: GpuVern7, tlist, ex: ExpectOps, d: int, store_states, store_fina
         ig.integrate(float(tlist[i]))
         ig.check()
         if kind == "me" and G and not store_states and ig.status == INTERPOLATED:
-            # every following output time inside this step is read from its dense output
+            # an operator that run_dm leaves to the loop here: every following output time
+            # inside this step is read from its dense output
             j = i + 1
             while j < nt and ig.t_prev <= tlist[j] < ig.t_front:
                 j += 1

@@ -21,7 +21,9 @@ state ``y``, the stage combinations and the error control in FP64) and
 step-size recurrences run on the host in IEEE double; the only per-step
 device-to-host transfer is the 8-byte error norm.  For the library's own operators that
 host loop is the library's (``qg_vern7_integrate``); the methods below are the same loop for
-any other operator with ``matvec`` and ``vern7_stage``.
+subclasses of them, for objects with a ``vern7_stage`` of their own and for any other operator
+with ``matvec`` and ``vern7_stage``.  The package itself has none of these: there the loop below
+is what the tests hold the library's against.
 """
 from __future__ import annotations
 
