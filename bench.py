@@ -336,6 +336,12 @@ def run_reference(args, dist):
     if dist.rank != 0:
         return
     cores = os.cpu_count() or 1
+    try:
+        host_qutip()
+    except ImportError as exc:
+        print(json.dumps({"impl": "reference", "unavailable":
+                          f"the reference QuTiP is not installed on this machine ({exc})"}))
+        return
     r = reference_solve(args.steps, args.warmup)
     times = r["times"]
     K = len(times)
@@ -1017,6 +1023,129 @@ def operator_upload_bytes(rhs, rho0) -> int:
     return b + 16 * n * n
 
 
+class QutipHost:
+    """The headline workload as a QuTiP user calls it: ``qutip.mesolve`` with this library's
+    integrator."""
+    call = ("qutip.mesolve(H, rho0, tlist, c_ops, e_ops, options={'method': 'gpu_vern7'}) from host "
+            "Qobjs")
+
+    def __init__(self, tlist):
+        self.qt, rw = host_qutip()
+        from qutip_gb300 import qutip_plugin
+        self.plugin = qutip_plugin                   # registers gpu_vern7, GpuDense
+        self.H, self.c_ops, self.rho0, self.e_ops = rw.ising_qobjs(N_SITES)
+        self.tlist = tlist
+        self.rho_dev = self.rho0.to("gpu")
+        self.n_eops = len(self.e_ops)
+
+    def solver(self, precision):
+        return self.qt.MESolver(self.H, self.c_ops, options=mesolve_opts(precision))
+
+    def op(self, solver):
+        return solver._integrator._op
+
+    def solve(self, solver, n_out=None):
+        return solver.run(self.rho_dev, self.tlist[:n_out], e_ops=self.e_ops)
+
+    def counts(self, solver):
+        """Steps and right-hand sides of the solver's solves so far."""
+        st = solver._integrator._ode.stats
+        return st["steps"], st["rhs"]
+
+    def whole_call(self):
+        return self.qt.mesolve(self.H, self.rho0, self.tlist, self.c_ops, e_ops=self.e_ops,
+                               options=mesolve_opts("double"))
+
+    def upload_bytes(self, solver):
+        return operator_upload_bytes(solver.rhs, self.rho0)
+
+    def breakdown(self):
+        import torch
+        t0 = time.perf_counter()
+        ref_solver = self.qt.MESolver(self.H, self.c_ops, options={"method": "vern7"})
+        liou_s = time.perf_counter() - t0
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        self.plugin.IntegratorGpuVern7(ref_solver, mesolve_opts("double"))
+        torch.cuda.synchronize()
+        return {"qutip_liouvillian_host": liou_s, "device_build": time.perf_counter() - t0}
+
+    def state0(self):
+        return self.rho0.full().reshape(-1, order="F")
+
+
+class LibraryHost:
+    """The same workload where QuTiP is not installed: the library's own ``mesolve`` on the same
+    matrices."""
+    call = ("qutip_gb300.solver.mesolve(H, rho0, tlist, c_ops, e_ops) from host matrices (QuTiP is "
+            "not installed on this machine)")
+
+    def __init__(self, tlist):
+        from qutip_gb300 import systems as S
+        from qutip_gb300.solver import ExpectOps
+        self.sys = S.ising_chain(N_SITES, build_terms=False)
+        self.tlist = tlist
+        self.ex = ExpectOps(self.sys.e_ops)
+        self.n_eops = len(self.sys.e_ops)
+        self._counts = {}
+
+    def _terms(self):
+        from qutip_gb300.solver import liouvillian_terms
+        return liouvillian_terms([list(t) if t[1] is not None else t[0] for t in self.sys.h_terms],
+                                 self.sys.c_ops)
+
+    def solver(self, precision):
+        from qutip_gb300.operator import DeviceOperator
+        return precision, DeviceOperator(self._terms(), dtype="c128" if precision == "double" else "c64")
+
+    def op(self, solver):
+        return solver[1]
+
+    def solve(self, solver, n_out=None):
+        from qutip_gb300.solver import solve_system
+        res = solve_system(self.sys, self.tlist[:n_out], {"precision": solver[0]}, op=solver[1],
+                           ex=self.ex)
+        steps, rhs = self._counts.get(id(solver[1]), (0, 0))
+        self._counts[id(solver[1])] = (steps + res.stats["steps"], rhs + res.stats["rhs"])
+        return res
+
+    def counts(self, solver):
+        return self._counts.get(id(solver[1]), (0, 0))
+
+    def whole_call(self):
+        from qutip_gb300.solver import mesolve
+        d = self.sys.dim
+        return mesolve([list(t) if t[1] is not None else t[0] for t in self.sys.h_terms],
+                       self.sys.state0.reshape(d, d, order="F"), self.tlist, self.sys.c_ops,
+                       self.sys.e_ops)
+
+    def upload_bytes(self, solver):
+        return sum(t.numel() * t.element_size() for t in solver[1].device_arrays()) + \
+            16 * self.sys.dim**2
+
+    def breakdown(self):
+        import torch
+        from qutip_gb300.operator import DeviceOperator
+        t0 = time.perf_counter()
+        terms = self._terms()
+        liou_s = time.perf_counter() - t0
+        t0 = time.perf_counter()
+        DeviceOperator(terms, dtype="c128")
+        torch.cuda.synchronize()
+        return {"liouvillian_host": liou_s, "device_build": time.perf_counter() - t0}
+
+    def state0(self):
+        return self.sys.state0
+
+
+def headline_host(tlist):
+    try:
+        return QutipHost(tlist)
+    except ImportError as exc:
+        log(f"QuTiP is not installed ({exc}): the library's own mesolve")
+        return LibraryHost(tlist)
+
+
 def run_ours(args, dist):
     import torch
     from qutip_gb300 import _lib
@@ -1025,22 +1154,18 @@ def run_ours(args, dist):
 
     dist.init()
     hbm_peak, peak_src = hbm_peak_gbs()
-    qt, RW = host_qutip()
-    from qutip_gb300 import qutip_plugin  # noqa: F401  (registers gpu_vern7, GpuDense)
-    H, c_ops, rho0, e_ops = RW.ising_qobjs(N_SITES)
     tlist = np.linspace(0.0, T_END, N_OUT)
+    host = headline_host(tlist)
     want = np.load(GOLDEN)["expect"]             # the reference's FP64 result
 
-    log("building the complex128 solver (QuTiP's Liouvillian, device operator)")
+    log("building the complex128 solver (Liouvillian, device operator)")
     t0 = time.perf_counter()
-    solver = qt.MESolver(H, c_ops, options=mesolve_opts("double"))
+    solver = host.solver("double")
     build_s = time.perf_counter() - t0
-    ig = solver._integrator
-    op = ig._op
-    rho_dev = rho0.to("gpu")
+    op = host.op(solver)
 
     def solve(s=solver):
-        return s.run(rho_dev, tlist, e_ops=e_ops)
+        return host.solve(s)
 
     log(f"warm-up ({op.launch_desc()})")
     for _ in range(args.warmup):
@@ -1049,8 +1174,7 @@ def run_ours(args, dist):
     clocks = ClockSampler(dist.local)
     clocks.start()
     n0 = _lib.LAUNCHES[0]
-    rhs0 = ig._ode.stats["rhs"]
-    steps0 = ig._ode.stats["steps"]
+    steps0, rhs0 = host.counts(solver)
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     e0.record()
     for _ in range(args.steps):
@@ -1059,8 +1183,9 @@ def run_ours(args, dist):
     dist.barrier()
     ms = e0.elapsed_time(e1)
     launches = _lib.LAUNCHES[0] - n0
-    rhs_full = (ig._ode.stats["rhs"] - rhs0) // args.steps
-    steps_full = (ig._ode.stats["steps"] - steps0) // args.steps
+    steps1, rhs1 = host.counts(solver)
+    rhs_full = (rhs1 - rhs0) // args.steps
+    steps_full = (steps1 - steps0) // args.steps
     clk = clocks.stop()
     ms_max = dist.max(ms)
     value = args.steps * dist.world / (ms_max / 1000.0)
@@ -1072,26 +1197,18 @@ def run_ours(args, dist):
     dist.barrier()
     t0 = time.perf_counter()
     for _ in range(n_e2e):
-        r_e2e = qt.mesolve(H, rho0, tlist, c_ops, e_ops=e_ops, options=mesolve_opts("double"))
+        r_e2e = host.whole_call()
     dist.barrier()
     e2e = n_e2e * dist.world / dist.max(time.perf_counter() - t0)
     rel_e2e, _, within_e2e = rel_err(r_e2e.expect, want)
-    h2d = operator_upload_bytes(solver.rhs, rho0)
-    d2h = N_OUT * (32 * len(e_ops) + 16) + 8 * steps_full
-    # where the end-to-end time goes: QuTiP's host Liouvillian, the device build
-    t0 = time.perf_counter()
-    ref_solver = qt.MESolver(H, c_ops, options={"method": "vern7"})
-    liou_s = time.perf_counter() - t0
-    torch.cuda.synchronize()
-    t0 = time.perf_counter()
-    qutip_plugin.IntegratorGpuVern7(ref_solver, mesolve_opts("double"))
-    torch.cuda.synchronize()
-    dev_build_s = time.perf_counter() - t0
-    del ref_solver
-    log(f"e2e {e2e:.3f} solves/s (Liouvillian {liou_s:.2f} s, device build {dev_build_s:.2f} s)")
+    h2d = host.upload_bytes(solver)
+    d2h = N_OUT * (32 * host.n_eops + 16) + 8 * steps_full
+    # where the end-to-end time goes: the host Liouvillian, the device build
+    breakdown = host.breakdown()
+    log(f"e2e {e2e:.3f} solves/s (" + ", ".join(f"{k} {v:.2f} s" for k, v in breakdown.items()) + ")")
 
     # the mixed form through the same API
-    solver_m = qt.MESolver(H, c_ops, options=mesolve_opts("mixed"))
+    solver_m = host.solver("mixed")
     solve(solver_m)
     nm = max(2, args.steps // 2)
     torch.cuda.synchronize()
@@ -1101,10 +1218,10 @@ def run_ours(args, dist):
     torch.cuda.synchronize()
     mixed_v = nm / (time.perf_counter() - t0)
     rel_m, abs_m, within_m = rel_err(res_m.expect, want)
-    op64 = solver_m._integrator._op
+    op64 = host.op(solver_m)
 
     log("roofline measurements")
-    state0 = rho0.full().reshape(-1, order="F")
+    state0 = host.state0()
     fmas = []
     stage_ms, stage_b, stage_gbs = measure_stage_roofline(op, state0, "double", fmas=fmas)
     fp64_tflops = 2 * fmas[0] / (stage_ms * 1e-3) / 1e12
@@ -1125,12 +1242,10 @@ def run_ours(args, dist):
         "config": CONFIG,
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h),
-                "call": "qutip.mesolve(H, rho0, tlist, c_ops, e_ops, options={'method': "
-                        "'gpu_vern7'}) from host Qobjs",
+                "call": host.call,
                 "reps": n_e2e, "rel_err_vs_reference_fp64": rel_e2e,
                 "within_reference_tolerance": within_e2e,
-                "breakdown_s": {"qutip_liouvillian_host": liou_s, "device_build": dev_build_s,
-                                "solve": 1.0 / value}},
+                "breakdown_s": {**breakdown, "solve": 1.0 / value}},
         "gpu_launches": int(launches),
         "solver_stats": {"steps": int(steps_full), "rhs": int(rhs_full),
                          "build_s": build_s, "launch": op.launch_desc()},
@@ -1178,7 +1293,10 @@ def run_ours(args, dist):
         out["dense_bucket"] = run_dense(args)
     if dist.rank == 0 and "sde" in sections:
         log("stochastic solvers")
-        out["sde"] = run_sde(args)
+        try:
+            out["sde"] = run_sde(args)
+        except ImportError as exc:
+            out["sde"] = {"unavailable": f"runs through QuTiP's own API ({exc})"}
     if dist.rank == 0 and "matrix" in sections:
         log("matrix form")
         sysm = S.ising_chain(N_SITES, build_terms=False)
@@ -1191,9 +1309,9 @@ def run_ours(args, dist):
         log("CPU baseline")
         try:
             k = max(1, min(args.cpu_sample, N_OUT - 1))
-            ig._ode.stats["rhs"] = 0
-            solver.run(rho_dev, tlist[:k + 1], e_ops=e_ops)
-            rhs_sample = int(ig._ode.stats["rhs"])
+            before = host.counts(solver)[1]
+            host.solve(solver, k + 1)
+            rhs_sample = int(host.counts(solver)[1] - before)
             out["cpu_baseline"] = cpu_baseline(k, rhs_sample, int(rhs_full))
         except Exception as exc:  # noqa: BLE001
             out["cpu_baseline"] = {"value": None, "error": repr(exc)[:300]}
