@@ -71,7 +71,7 @@ struct RkArgs {
   double* result;
   double fa_d[16], fe_d[16];
   float fa_f[16], fe_f[16];
-  float fe_l[16];  // fe_d - fe_f: the error weights as float pairs (mixed form)
+  float fa_l[16], fe_l[16];  // fa_d - fa_f, fe_d - fe_f: the weights as float pairs
   // bit j set where fa_d[j] / fe_d[j] is nonzero: the factor loops test these integer
   // masks, not the factors (a floating-point compare per row would run on the FP64 pipe)
   unsigned int nz_a, nz_e;
@@ -260,6 +260,7 @@ static inline int prepare_stage(const qg_rk_buffers* B, int op_dtype, int64_t n_
     rk.fe_d[j] = e;
     rk.fa_f[j] = (float)a;
     rk.fe_f[j] = (float)e;
+    rk.fa_l[j] = (float)(a - (double)rk.fa_f[j]);
     rk.fe_l[j] = (float)(e - (double)rk.fe_f[j]);
     if (a != 0.0) rk.nz_a |= 1u << j;
     if (e != 0.0) rk.nz_e |= 1u << j;

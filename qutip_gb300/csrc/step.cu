@@ -36,6 +36,7 @@
 // in its rows: what is read from them before the host sees the word is no value.  A row's sum and its
 // stage combination are formed by the operations of the per-stage kernels in their order.
 #include <mutex>
+#include <type_traits>
 
 #include "capi_internal.h"
 #include "common.cuh"
@@ -142,11 +143,14 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
   constexpr bool RI = DT == QG_C128;
   constexpr bool DICT = KIND >= KIND_DICT1;
   constexpr int CB = KIND == KIND_DICT2 ? 2 : 1;
+  using Sum = typename std::conditional<HERM, HermSum<R>, PlainSum<R>>::type;
   using C4 = typename Codes4<CB>::T;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ cx<R> coef[RK_EXTRA_STEP][QG_MAX_GROUPS];
   __shared__ int ccls[RK_EXTRA_STEP][QG_MAX_GROUPS];
   __shared__ R fac[RK_EXTRA_STEP][RK_EXTRA_STEP];  // dt a of the combination after stage s
+  constexpr bool FF = HERM && sizeof(R) == 4;      // their low parts, for HermSum
+  __shared__ float fac_l[FF ? RK_EXTRA_STEP : 1][RK_EXTRA_STEP];
   __shared__ R fe_s[RK_STEP];
   __shared__ float fel_s[RK_STEP];
   __shared__ unsigned int nz_s[RK_EXTRA_STEP + 1];
@@ -209,6 +213,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
     if (s == RK_STEP - 1 && a.s0 == 0) v = j < RK_STEP ? a.dt * VERN7_B[j] : 0.0;
     else if (s + 1 < RK_EXTRA_STEP && j <= s) v = a.dt * VERN7_A[s + 1][j];
     fac[s][j] = (R)v;
+    if constexpr (FF) fac_l[s][j] = (float)(v - (double)(float)v);
     const double w = s == 0 && j < RK_STEP ? a.dt * VERN7_E[j] : 0.0;
     if (s == 0 && j < RK_STEP) {
       fe_s[j] = (R)w;
@@ -286,13 +291,14 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
   unsigned int target = a.bar_base;
   bool ok = true;
   // out = base + sum_{j <= s} (dt a_{s+1,j}) k_j, in the reference's order
+  auto low = [&](int s, int j) { return FF ? fac_l[FF ? s : 0][j] : 0.f; };
   auto form_input = [&](int s) {
-    cx<R> v = base;
+    Sum v{base};
     const unsigned int nz = nz_s[s];
     for (int j = 0; j <= s; ++j)
-      if ((nz >> j) & 1u) cx_axpy(v, fac[s][j], ld_cx<R>(ksm + j * rows));
+      if ((nz >> j) & 1u) v.add(fac[s][j], low(s, j), ld_cx<R>(ksm + j * rows));
     ST q;
-    st_cx(&q, v);
+    st_cx(&q, v.value());
     ytmp[(size_t)((s + 1) & 1) * n64 + row] = q;
     if constexpr (HERM) tv[t_own * PAD + (tid & 31)] = ST{q.x, -q.y};
   };
@@ -411,32 +417,34 @@ __global__ void __launch_bounds__(STEP_THREADS, 1)
       if (s == RK_STEP - 1) {
         const unsigned int nz = nz_s[s], ne = nz_s[RK_EXTRA_STEP];
         if constexpr (MIXED) {
-          cx<R> inc{0, 0};
+          Sum inc{cx<R>{0, 0}};
           float erh = 0.f, erl = 0.f, eih = 0.f, eil = 0.f;
           for (int j = 0; j < RK_STEP; ++j) {
             const cx<R> kj = ld_cx<R>(ksm + j * rows);
-            if ((nz >> j) & 1u) cx_axpy(inc, fac[s][j], kj);
+            if ((nz >> j) & 1u) inc.add(fac[s][j], low(s, j), kj);
             if ((ne >> j) & 1u) {  // the error estimate in float-float
               ff_acc(erh, erl, fe_s[j], fel_s[j], (float)kj.re);
               ff_acc(eih, eil, fe_s[j], fel_s[j], (float)kj.im);
             }
           }
           const double2 yp = static_cast<const double2*>(rk.y_prev)[row];
-          const double2 yf = make_double2(yp.x + (double)inc.re, yp.y + (double)inc.im);
+          const double2 dy = inc.wide();
+          const double2 yf = make_double2(yp.x + dy.x, yp.y + dy.y);
           static_cast<double2*>(rk.y_front)[row] = yf;
           static_cast<float2*>(rk.y_front_s)[row] = make_float2((float)yf.x, (float)yf.y);
           if constexpr (HERM) ty[t_own * YPAD + (tid & 31)] = make_double2(yf.x, -yf.y);
           const double er = (double)erh + (double)erl, ei = (double)eih + (double)eil;
           err_acc = wrms_term(er * er + ei * ei, yf.x * yf.x + yf.y * yf.y, rk.atol, rk.rtol);
         } else {
-          cx<R> y = base, e{0, 0};
+          Sum y{base};
+          cx<R> e{0, 0};
           for (int j = 0; j < RK_STEP; ++j) {
             const cx<R> kj = ld_cx<R>(ksm + j * rows);
-            if ((nz >> j) & 1u) cx_axpy(y, fac[s][j], kj);
+            if ((nz >> j) & 1u) y.add(fac[s][j], low(s, j), kj);
             if ((ne >> j) & 1u) cx_axpy(e, fe_s[j], kj);
           }
           YT yq;
-          st_cx(&yq, y);
+          st_cx(&yq, y.value());
           static_cast<YT*>(rk.y_front)[row] = yq;
           if constexpr (HERM) ty[t_own * YPAD + (tid & 31)] = YT{yq.x, -yq.y};
           const cx<R> ys = ld_cx<R>(&yq);
