@@ -337,12 +337,11 @@ def run_reference(args, dist):
         return
     cores = os.cpu_count() or 1
     try:
-        host_qutip()
+        r = reference_solve(args.steps, args.warmup)
     except ImportError as exc:
         print(json.dumps({"impl": "reference", "unavailable":
                           f"the reference QuTiP is not installed on this machine ({exc})"}))
         return
-    r = reference_solve(args.steps, args.warmup)
     times = r["times"]
     K = len(times)
     total = float(sum(times))
