@@ -972,7 +972,8 @@ def run_matrix_form(args, sysm, tlist, ex, want, hbm_peak):
            "rel_err_vs_reference_fp64": rel, "max_abs_err_vs_reference_fp64": absmax,
            "within_reference_tolerance": within,
            "hermitian_branch": bool(lop.hermitian),
-           "stage_kernel": {"kernel": "lindblad_kernel<C64,C128,RK>", "ms": ms,
+           "stage_kernel": {"kernel": "lindblad_herm_kernel<C64,C128,RK>" if lop.hermitian else
+                            "lindblad_kernel<C64,C128,RK>", "ms": ms,
                             "algorithmic_bytes": int(b), "gbs": gbs, "frac_hbm": gbs / hbm_peak,
                             "bound": "instruction issue (operators L1-resident, state "
                                      "L2-resident; HBM carries only the stage vectors)"},
@@ -1253,7 +1254,8 @@ def run_ours(args, dist):
                      "traffic_source": f"{TRAFFIC_PROFILE} (ncu dram__bytes_read.sum + "
                                        "dram__bytes_write.sum per launch)",
                      "kernel": (f"spmv_dict_kernel<C128,C128,RK,{op.code_bytes}> (fused Vern7 "
-                                "stage, complex128, dictionary-coded operator)"
+                                "stage, complex128, dictionary-coded operator, full form; the "
+                                "Hermitian state of the solve takes vern7_herm_kernel)"
                                 if op.fmt == "dict" else
                                 "spmv_sliced_kernel<C128,C128,RK> (fused Vern7 stage)"),
                      "bytes_per_launch": stage_b, "ms_per_launch": stage_ms,
@@ -1272,7 +1274,8 @@ def run_ours(args, dist):
         "mixed": {"value": mixed_v, "unit": UNIT, "dtype": "c64 stages / f64 state and step control",
                   "rel_err_vs_reference_fp64": rel_m, "max_abs_err": abs_m,
                   "within_reference_tolerance": within_m, "bound_rel": 1e-6,
-                  "stage_kernel": {"kernel": f"spmv_dict_kernel<C64,C128,RK,{op64.code_bytes}>"
+                  "stage_kernel": {"kernel": f"spmv_dict_kernel<C64,C128,RK,{op64.code_bytes}> "
+                                             "(full form)"
                                    if op64.fmt == "dict" else op64.launch_desc(),
                                    "ms": st64_ms, "bytes": st64_b, "gbs": st64_gbs,
                                    "frac_hbm": st64_gbs / hbm_peak}},

@@ -541,7 +541,7 @@ __device__ void matvec_to_k(const GT& g, Ctx<DT>& X, Ctl& c, double t,
 // to the compiler and loaded together before the row's matvec, and the pair sums run on
 // packed components.  Measured, clocks per stage of a trajectory's CTA (512 rows, two CTAs per
 // SM) 15.5k -> 7.5k, of a 3600-row item's 71k -> 35k; with the shared sums and step control
-// above, 608 Bose-Hubbard trajectories 47 -> 33 ms and 96 Jaynes-Cummings requests 39 -> 25 ms
+// above, 608 Bose-Hubbard trajectories 45 -> 32 ms and 96 Jaynes-Cummings requests 40 -> 27 ms
 // per call (13 to 17 ms of either are host work).
 template <int DT, int S>
 __device__ __noinline__ double stage_rows(const Ctx<DT>& X, int rank, int size, int cur) {

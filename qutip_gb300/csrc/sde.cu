@@ -3,11 +3,13 @@
 // of qutip/solver/sode/ssystem.pyx:119-250.  A group of threads integrates one trajectory
 // through n_steps fixed steps with the Wiener increments the host drew (the reference's own
 // generator stream), so a launch covers a whole output interval of one or many
-// trajectories.  A state of up to 64 entries is integrated by one warp (4 trajectories
-// per CTA; syncs are __syncwarp), a larger one by a CTA of 256 threads.  Every vector
-// operation follows the reference's order of operations
+// trajectories.  States of up to 640 entries with one stochastic operator (512 with two) take
+// a thread per entry (sde_row_kernel, below).  With more operators a state of up to 64 entries
+// is integrated by one warp (4 trajectories per CTA; syncs are __syncwarp), and a larger one by a
+// CTA of 256 threads; there every vector operation follows the reference's order of operations
 // (`_data.add(a, b, s)` is a + s b element by element, the complex scalars formed the way
-// the reference forms them); CSR rows are summed in column order.
+// the reference forms them), where the row kernel contracts to fused multiply-adds.  CSR rows
+// are summed in column order in both.
 #include "capi_internal.h"
 #include "common.cuh"
 

@@ -891,9 +891,9 @@ class IntegratorGpuVern7(Integrator):
         only): ``"auto"`` sends small systems with dense operators in the mixed form to
         the dense bucket, ``True`` forces it, ``False`` keeps the sparse kernel;
         hermitian_branch (matrix form only): with a Hermitian rho0, ``"auto"`` evaluates
-        half the elements where that is faster (at least two 32 x 32 tiles per SM),
-        ``True`` always, ``False``
-        never."""
+        half the elements where that is faster (two 32 x 32 blocks on or below the diagonal
+        per SM in the mixed form, two for five SMs in complex128), ``True`` always,
+        ``False`` never."""
         return self._options
 
     @options.setter
