@@ -843,14 +843,19 @@ class IntegratorGpuVern7(Integrator):
         except IntegratorError as exc:
             raise IntegratorException(str(exc)) from None
 
-    def integrate(self, t, copy=True):
-        self._ode.integrate(t, step=False)
+    def _advance(self, t, step):
+        try:
+            self._ode.integrate(t, step=step)
+        except IntegratorError as exc:              # a device wait that gave up
+            raise IntegratorException(str(exc)) from None
         self._check()
+
+    def integrate(self, t, copy=True):
+        self._advance(t, False)
         return self.get_state(copy)
 
     def mcstep(self, t, copy=True):
-        self._ode.integrate(t, step=True)
-        self._check()
+        self._advance(t, True)
         return self.get_state(copy)
 
     def reset(self, hard=False):

@@ -176,6 +176,8 @@ class GpuVern7:
         y0 = torch.as_tensor(y0)
         if y0.numel() != self.n:
             raise ValueError(f"state of size {y0.numel()} for a generator of size {self.n}")
+        if self._words[1] < 0:                      # of the state before: nothing to it any more
+            self._reset_waits()
         self.y_prev.copy_(y0.reshape(-1).to(self.y_prev.device, self.y_prev.dtype))
         self.y_front.copy_(self.y_prev)
         if self.mixed:
@@ -385,11 +387,14 @@ class GpuVern7:
         if self._words[1] < 0:
             self._wait_gave_up()
 
-    def _wait_gave_up(self):
+    def _reset_waits(self):
         torch.cuda.current_stream().synchronize()   # every block has left and written its word
         self.counter.zero_()
         self._barrier_base.value = 0
         self._words[1] = 0.0
+
+    def _wait_gave_up(self):
+        self._reset_waits()
         self.status = DEVICE_WAIT
         self._set = False                           # no step to go on from
         raise IntegratorError(STATUS_MESSAGES[DEVICE_WAIT])

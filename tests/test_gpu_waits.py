@@ -94,6 +94,25 @@ def test_a_dense_output_that_gives_up(form, precision):
         assert bool(torch.isfinite(torch.view_as_real(ig.get_state())).all())
 
 
+def test_a_new_state_after_a_give_up():
+    """Set while the last state's dense output is known to have given up: a fresh start."""
+    s, ig = _integrator("csr", "double")
+    ig.integrate(100.0, step=True)
+    _no_arrivals(ig)
+    ig.integrate(0.5 * (ig.t_prev + ig.t_front))
+    torch.cuda.synchronize()
+    assert not ig.successful()
+    ig._wait_mcycles = 0
+    again = _integrator("csr", "double")[1]
+    for g in (ig, again):
+        g.set_initial_value(torch.from_numpy(s.state0), 0.0)
+        g.integrate(1.0)
+        g.check()
+    assert torch.equal(ig.get_state(), again.get_state())
+    from qutip_gb300 import _lib
+    assert _lib.load().qg_device_fault() != 0        # read and cleared
+
+
 @pytest.mark.parametrize("in_library", [False, True])
 def test_a_give_up_seen_by_the_next_call(in_library):
     """A dense output that gave up ends the next call, before its trial step or, where it
