@@ -21,6 +21,10 @@ mcsolve, the matrix-free form and the L = 12 chain.
 reference QuTiP (compiled from its sources into oracle/_ref) on the host cores,
 split into ``--steps`` chunks of output times; nothing is extrapolated.
 
+Where QuTiP is not installed, the reference arm prints its ``unavailable`` line, and the other arm
+solves the same workload through the library's own ``mesolve`` (``e2e``: from host matrices); the
+sections that run through QuTiP's API say so.
+
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 """
 from __future__ import annotations
