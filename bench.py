@@ -22,7 +22,7 @@ reference QuTiP (compiled from its sources into oracle/_ref) on the host cores,
 split into ``--steps`` chunks of output times; nothing is extrapolated.
 
 Where QuTiP is not installed, the reference arm prints its ``unavailable`` line, and the other arm
-solves the same workload through the library's own ``mesolve`` (``e2e``: from host matrices); the
+solves the same workload through the library's own calls (``e2e``: from host matrices); the
 sections that run through QuTiP's API say so.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
@@ -1079,10 +1079,11 @@ class QutipHost:
 
 
 class LibraryHost:
-    """The same workload where QuTiP is not installed: the library's own ``mesolve`` on the same
-    matrices."""
-    call = ("qutip_gb300.solver.mesolve(H, rho0, tlist, c_ops, e_ops) from host matrices (QuTiP is "
-            "not installed on this machine)")
+    """The same workload where QuTiP is not installed: the library's own solve of the same
+    matrices, the generator laid out on the device as the plugin does."""
+    call = ("qutip_gb300: liouvillian_terms(H, c_ops), DeviceOperator.from_device_groups, "
+            "solve_system(rho0, tlist, e_ops) from host matrices (QuTiP is not installed on this "
+            "machine)")
 
     def __init__(self, tlist):
         from qutip_gb300 import systems as S
@@ -1098,9 +1099,14 @@ class LibraryHost:
         return liouvillian_terms([list(t) if t[1] is not None else t[0] for t in self.sys.h_terms],
                                  self.sys.c_ops)
 
-    def solver(self, precision):
+    def _device_op(self, terms, precision):
         from qutip_gb300.operator import DeviceOperator
-        return precision, DeviceOperator(self._terms(), dtype="c128" if precision == "double" else "c64")
+        from qutip_gb300.superop import device_term_groups
+        return DeviceOperator.from_device_groups(device_term_groups(terms),
+                                                 "c128" if precision == "double" else "c64")
+
+    def solver(self, precision):
+        return precision, self._device_op(self._terms(), precision)
 
     def op(self, solver):
         return solver[1]
@@ -1117,24 +1123,21 @@ class LibraryHost:
         return self._counts.get(id(solver[1]), (0, 0))
 
     def whole_call(self):
-        from qutip_gb300.solver import mesolve
-        d = self.sys.dim
-        return mesolve([list(t) if t[1] is not None else t[0] for t in self.sys.h_terms],
-                       self.sys.state0.reshape(d, d, order="F"), self.tlist, self.sys.c_ops,
-                       self.sys.e_ops)
+        from qutip_gb300.solver import ExpectOps, solve_system
+        return solve_system(self.sys, self.tlist, op=self._device_op(self._terms(), "double"),
+                            ex=ExpectOps(self.sys.e_ops))
 
     def upload_bytes(self, solver):
-        return sum(t.numel() * t.element_size() for t in solver[1].device_arrays()) + \
+        return sum(m.data.nbytes + m.indices.nbytes + m.indptr.nbytes for m, _ in self._terms()) + \
             16 * self.sys.dim**2
 
     def breakdown(self):
         import torch
-        from qutip_gb300.operator import DeviceOperator
         t0 = time.perf_counter()
         terms = self._terms()
         liou_s = time.perf_counter() - t0
         t0 = time.perf_counter()
-        DeviceOperator(terms, dtype="c128")
+        self._device_op(terms, "double")
         torch.cuda.synchronize()
         return {"liouvillian_host": liou_s, "device_build": time.perf_counter() - t0}
 
@@ -1146,7 +1149,7 @@ def headline_host(tlist):
     try:
         return QutipHost(tlist)
     except ImportError as exc:
-        log(f"QuTiP is not installed ({exc}): the library's own mesolve")
+        log(f"QuTiP is not installed ({exc}): the library's own calls")
         return LibraryHost(tlist)
 
 
