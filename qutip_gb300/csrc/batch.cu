@@ -1700,7 +1700,8 @@ static int group_slots(int64_t max_n, int dtype, int group, int64_t smem) {
   }
   if (smem > MAX_DYN_SMEM) return set_error(QG_ERR_ARG, "staged data exceed shared memory");
   const Shape sh = shape_of(max_n, dtype, group);
-  if (!allow_smem((const void*)sh.kernel, (size_t)smem)) return set_error(QG_ERR_CUDA, "shared-memory opt-in failed");
+  if (!allow_smem((const void*)sh.kernel, (size_t)smem))
+    return set_error(QG_ERR_CUDA, "shared-memory opt-in failed");
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sh.kernel, sh.block, smem);
   if (e != cudaSuccess || per_sm <= 0) {
     char msg[200];
@@ -1769,7 +1770,8 @@ extern "C" int qg_batch_vern7(const qg_batch* B, void* stream) {
   }
   const Shape sh = shape_of(B->max_n, B->dtype, B->group);
   const int64_t smem = launch_smem(*B);
-  if (!allow_smem((const void*)sh.kernel, (size_t)smem)) return set_error(QG_ERR_CUDA, "shared-memory opt-in failed");
+  if (!allow_smem((const void*)sh.kernel, (size_t)smem))
+    return set_error(QG_ERR_CUDA, "shared-memory opt-in failed");
   const int grid = (B->n_slots + sh.groups_per_cta - 1) / sh.groups_per_cta;
   sh.kernel<<<grid, sh.block, smem, st>>>(*B);
   return check_launch("batch_vern7 (warp or CTA groups)");

@@ -28,13 +28,14 @@
 // block per SM with 100 KB of batch on each: the N = 10 Jaynes-Cummings solve runs beside it
 // (4.3 ms, 2.5 alone), at 30 or 170 KB (the SM keeps its split between L1 and shared memory
 // while a block runs) it waits for the batch's end, as does the L = 6 Ising solve, whose
-// stages one by one ran beside it.  A CSR operator that should not wait takes a launch shape without
-// this kernel (sub-warps of 16).
+// stages one by one ran beside it.  A CSR operator that should not wait takes a launch shape
+// without this kernel (sub-warps of 16).
 //
 // The launch is cooperative (all blocks resident), and every wait at the barrier is bounded:
 // a wait that gives up sets *result to -1, every block leaves, and the launch's stages hold NaN
-// in its rows: what is read from them before the host sees the word is no value.  A row's sum and its
-// stage combination are formed by the operations of the per-stage kernels in their order.
+// in its rows: what is read from them before the host sees the word is no value.  A row's sum
+// and its stage combination are formed by the operations of the per-stage kernels in their
+// order.
 #include <mutex>
 #include <type_traits>
 

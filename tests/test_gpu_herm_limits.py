@@ -48,8 +48,8 @@ def _rho(d, seed):
 # static shared memory and tables together pass the 48 KB default at 1,599 entries of 20 bytes
 # (complex128) and 3,355 of 12 bytes (complex64)
 @pytest.mark.parametrize("precision,entries", [
-    ("double", 64), ("double", 1597), ("double", 1598), ("double", 1599), ("double", 1638), ("double", 1639),
-    ("double", 4096), ("mixed", 2730), ("mixed", 2731), ("mixed", 3355), ("mixed", 4096)])
+    ("double", 64), ("double", 1597), ("double", 1598), ("double", 1599), ("double", 1638),
+    ("double", 1639), ("double", 4096), ("mixed", 2730), ("mixed", 2731), ("mixed", 3355), ("mixed", 4096)])
 def test_every_size_of_the_tables_is_taken(precision, entries):
     """A trial step and the dense-output stages by half against the full form: rows of at most
     12 entries of magnitude one at most, summed in another order: 100 eps of the largest k."""
